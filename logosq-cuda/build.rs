@@ -14,6 +14,7 @@ const SOURCES: &[&str] = &[
     "variational.cu",
     "profile.cu",
     "batch.cu",
+    "adjoint.cu",
     "tc.cu",
     "learned.cu",
     "noise.cu",

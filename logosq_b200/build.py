@@ -24,6 +24,7 @@ SOURCES = [
     "variational.cu",
     "profile.cu",
     "batch.cu",
+    "adjoint.cu",
     "tc.cu",
     "learned.cu",
     "noise.cu",

@@ -288,7 +288,7 @@ static int choose_lanes(const int rpos[4], int T, int *lane) {
     // Thread-index bits go to the tile positions outside R.  The first three
     // should be positions whose swizzle images (p mod 3 for p < 6) differ, so
     // that 8 consecutive threads touch 8 distinct 16-byte bank groups.
-    bool inR[kMaxT] = {false};
+    bool inR[kMaxT + 1] = {false};
     for (int k = 0; k < 4; ++k) inR[rpos[k]] = true;
     std::vector<int> free;
     for (int p = 0; p < T; ++p)
@@ -310,16 +310,16 @@ static int choose_lanes(const int rpos[4], int T, int *lane) {
     return (int)order.size();
 }
 
-static void pad_rpos(std::vector<int> &R, int T) {
-    // Fill up to four register bits, preferring positions that keep one of
+static void pad_rpos(std::vector<int> &R, int T, int count = 4) {
+    // Fill up to `count` register bits, preferring positions that keep one of
     // each pair (r, r+3), r < 3, outside R (see choose_lanes).
     auto conflicts = [&](int p) {
         if (p >= 6) return false;
         const int partner = p < 3 ? p + 3 : p - 3;
         return std::find(R.begin(), R.end(), partner) != R.end();
     };
-    for (int pass = 0; pass < 2 && (int)R.size() < 4; ++pass) {
-        for (int p = T - 1; p >= 0 && (int)R.size() < 4; --p) {
+    for (int pass = 0; pass < 2 && (int)R.size() < count; ++pass) {
+        for (int p = T - 1; p >= 0 && (int)R.size() < count; --p) {
             if (std::find(R.begin(), R.end(), p) != R.end()) continue;
             if (pass == 0 && conflicts(p)) continue;
             R.push_back(p);
@@ -717,7 +717,7 @@ static void fold_pairs(std::vector<GateOp> &gops, std::vector<int> &orig, int T)
     }
 }
 
-std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T) {
+std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T, int maxr) {
     const int m = T - 4;
     std::vector<PlanStep> steps;
     const int G = (int)gops.size();
@@ -728,7 +728,7 @@ std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T
     for (int i = 0; i < G; ++i) {
         bits[i] = op_bits(gops[i]);
         rbits[i] = reg_bits(gops[i]);
-        fusable[i] = !gops[i].renorm && popc(rbits[i]) <= 4;
+        fusable[i] = !gops[i].renorm && popc(rbits[i]) <= maxr;
     }
     int remaining = G, first = 0;
     while (remaining > 0) {
@@ -797,7 +797,7 @@ std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T
             uint64_t R = 0, blk = 0;
             for (int k = 0; k < P; ++k) {
                 if (sched[k]) continue;
-                if ((gall[k] & blk) == 0 && popc(R | lreg[k]) <= 4) {
+                if ((gall[k] & blk) == 0 && popc(R | lreg[k]) <= maxr) {
                     R |= lreg[k];
                     rd.ops.push_back(k);
                     sched[k] = 1;
@@ -809,8 +809,8 @@ std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T
             std::vector<int> Rv;
             for (int p = 0; p < T; ++p)
                 if (R >> p & 1) Rv.push_back(p);
-            pad_rpos(Rv, T);
-            for (int k = 0; k < 4; ++k) rd.rpos[k] = Rv[k];
+            pad_rpos(Rv, T, maxr);
+            for (int k = 0; k < 4; ++k) rd.rpos[k] = k < maxr ? Rv[k] : T;
             st.pass.rounds.push_back(rd);
         }
         steps.push_back(st);
@@ -825,7 +825,8 @@ void fill_round(FusedRound &fr, const int rpos[4], int T, int h) {
             if (e >> k & 1) off |= 1 << rpos[k];
         fr.eoff[e] = swz(off) << 4;
     }
-    for (int k = 0; k < 4; ++k) fr.gpos[k] = 1ull << global_pos(rpos[k], h);
+    // (position T is the selector of a second state: it is no index bit)
+    for (int k = 0; k < 4; ++k) fr.gpos[k] = rpos[k] < T ? 1ull << global_pos(rpos[k], h) : 0ull;
     fr.nlane = choose_lanes(rpos, T, fr.lane);
 }
 

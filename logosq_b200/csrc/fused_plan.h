@@ -25,8 +25,10 @@ struct PlanStep {  // either a fused pass or a standalone gate
     PlannedPass pass;
 };
 
-// Window [0,4) U [h, h+T-4); returns passes and standalone gates in order.
-std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T);
+// Window [0,4) U [h, h+T-4); returns passes and standalone gates in order.  With
+// maxr = 3 a round picks three tile bits and its fourth register bit is tile
+// position T, the selector of a second state in the same tile (adjoint.cu).
+std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T, int maxr = 4);
 // Round record (element offsets, register bit masks, thread lanes).
 void fill_round(FusedRound &fr, const int rpos[4], int T, int h);
 // Append the register op of gate g in a round with register positions rpos.

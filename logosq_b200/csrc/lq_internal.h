@@ -50,6 +50,9 @@ struct Phases4 {  // up to 4 complex phases
 // Reduction scratch sizes (per state handle).
 constexpr int kRedBlocks = 148 * 8;   // partial slots of a two-stage reduction
 constexpr int kMaxTermsPerPass = 32;  // Pauli terms accumulated per sweep
+// Terms of one X mask in a Pauli sweep: they sit in its dynamic shared memory (24
+// bytes each, 48 KB per block without an opt-in); larger groups are refused.
+constexpr int kMaxGroupTerms = 2000;
 
 // Flag word written by kernels that wait (bounded) on a barrier.
 constexpr unsigned kFlagTimeout = 1u;

@@ -2,10 +2,14 @@
 // ParameterShift::compute_gradient (src/optimization/gradient.rs:44-78) and
 // FiniteDifference::compute_gradient (src/optimization/gradient.rs:96-125).
 //
-// This is the plain per-circuit path: every energy is one Circuit::execute from
-// |0...0> (fused passes) followed by one Pauli-sum reduction, exactly as the
-// reference re-simulates each shifted circuit.  The batched engine (batch.cu)
-// runs the same 2P+1 circuits of many instances in one persistent launch.
+// An energy is one Circuit::execute from |0...0> (fused passes) followed by one
+// Pauli-sum reduction.  A parameter-shift gradient is one reverse sweep over the
+// circuit where that gives the same values (adjoint.cu); otherwise every shifted
+// circuit is simulated, as the reference does.
+#include <cmath>
+#include <map>
+
+#include "adjoint.h"
 #include "lq_internal.h"
 
 namespace lq {
@@ -34,6 +38,44 @@ static int energy_at(lq_state *work, const lq_gate *ops, int nops, const double 
     return expectation_impl(work, terms, nterms, yconv, e, nullptr);
 }
 
+// Whether the observable is one that every energy of the gradient would accept
+// (otherwise the shifted circuits report the error).
+static bool plain_terms(const lq_pauli_term *terms, int nterms, int n) {
+    const uint64_t lim = (1ull << n) - 1;
+    std::map<uint64_t, int> per_mask;
+    for (int t = 0; t < nterms; ++t) {
+        if ((terms[t].xmask & ~lim) || (terms[t].zmask & ~lim)) return false;
+        if (terms[t].ny != __builtin_popcountll(terms[t].xmask & terms[t].zmask)) return false;
+        if (++per_mask[terms[t].xmask] > kMaxGroupTerms) return false;
+    }
+    return true;
+}
+
+// The gradient by a reverse sweep; *done stays false where the shifted circuits
+// have to run (adj_plan declines, or its second state cannot be allocated).
+static int sweep_gradient(lq_state *work, const lq_gate *ops, int nops, const double *theta,
+                          int nparams, const lq_pauli_term *terms, int nterms, int yconv,
+                          double shift, double *grad, bool *done) {
+    *done = false;
+    if (nparams == 0 || work->dtype != LQ_C128 || !std::isfinite(shift)) return LQ_OK;
+    for (int i = 0; i < nparams; ++i)
+        if (!std::isfinite(theta[i])) return LQ_OK;
+    if (!plain_terms(terms, nterms, work->n)) return LQ_OK;
+    const auto plan = adj_plan({AdjSpec{work->n, ops, nops, nparams, terms, nterms, yconv}}, 11,
+                               (size_t)-1);
+    if (!plan) return LQ_OK;
+    const int rc = adj_upload(*plan, work, work->stream);
+    if (rc == LQ_ERR_OOM) return LQ_OK;
+    LQ_TRY(rc);
+    std::vector<double> up(theta, theta + nparams), out(nparams + 1);
+    up.push_back(shift);
+    LQ_TRY(adj_enqueue(*plan, work->stream, up.data(), out.data()));
+    LQ_CUDA_TRY(cudaStreamSynchronize(work->stream));
+    std::copy(out.begin() + 1, out.end(), grad);
+    *done = true;
+    return LQ_OK;
+}
+
 }  // namespace lq
 
 using namespace lq;
@@ -53,6 +95,10 @@ int lq_parameter_shift(lq_state *work, const lq_gate *ops, int nops, const doubl
                        double shift, double *grad) {
     LQ_TRY(check_variational(work, ops, nops, theta, nparams, terms, nterms, y_convention));
     if (nparams > 0 && !grad) return set_error(LQ_ERR_INVALID_ARG, "null gradient output");
+    bool done;
+    LQ_TRY(sweep_gradient(work, ops, nops, theta, nparams, terms, nterms, y_convention, shift,
+                          grad, &done));
+    if (done) return LQ_OK;
     std::vector<double> p(theta, theta + nparams);
     for (int i = 0; i < nparams; ++i) {
         double ep, em;
