@@ -18,13 +18,22 @@
 // non-unitary matrix, a gate that fits no window) keeps the shifted circuits.
 //
 // Rounds.  (psi, lambda) is one state with a selector bit above the tile: a tile
-// holds 2^T amplitudes of each, and a register round picks three tile bits plus
-// the selector (tile position T), so the ping-pong routines of fused_round.cuh
-// apply a gate to both halves and a thread holds the matching amplitudes of both
-// for the inner products.  All rotations of a run on one qubit share one 2x2 and one
-// set of sums (S_x, S_y, S_z) = Im <lambda| (X, Y, Z) |psi> taken just before the
-// run is undone; a parameter's derivative is the combination of the three with its
-// axis turned by the run's later gates, computed with the 2x2s on the device.
+// holds 2^T amplitudes of each in shared memory, and a register round gives every
+// thread the 16 amplitudes that differ in three tile bits and the selector (going
+// forward: in four tile bits of psi alone).  A round undoes one run of single-qubit
+// gates on each of its bits, straight-line code in place.  All rotations of a run
+// share one 2x2 and one set of sums (S_x, S_y, S_z) = Im <lambda| (X, Y, Z) |psi> taken just
+// before the run is undone; a parameter's derivative is the combination of the three
+// with its axis turned by the run's later gates, computed with the 2x2s on the device.
+//
+// Gates that permute basis states linearly (CNOT, X, SWAP) move no data: the tile
+// keeps a map logical index -> shared-memory place, linear over XOR, and such a gate
+// only changes the map's vectors, which the planner knows (a control outside the
+// window adds a vector where that bit of the tile's index is 1).  Rounds address
+// through the map and the store writes logical order back.  The first form of this
+// kernel ran each gate as an op of the ping-pong rounds (fused_round.cuh): of its
+// 2570 instructions per warp and round 690 were FP64, the rest register moves at the
+// op switch's joins, selects of the CNOTs and the op dispatch.
 //
 // States of up to 2^12 amplitudes: one CTA does everything in shared memory
 // (k_adj_small).  Larger ones: one launch per pass over the tiles of all circuits
@@ -42,11 +51,60 @@ constexpr int kAdjSmallMax = 12;   // largest state kept in one CTA's shared mem
 constexpr int kAdjMinN = 5;        // smaller circuits are planned as 5 qubits (upper bits 0)
 constexpr int kAdjSmallThreads = 256;
 constexpr int kAdjThreads = 128;
-constexpr int kRoundSlots = 8;     // gradient runs of one round
-constexpr int kHChunk = 1024;      // amplitudes of one block of k_adj_h
+constexpr int kRoundSlots = 3;     // gradient runs of one round
+constexpr int kHChunk = 2048;      // amplitudes of one block of k_adj_h
+constexpr int kHStage = 12288;     // bytes of a Pauli sum that its blocks keep in shared memory
+constexpr int kStageBytes = 4096;  // program bytes of one chunk (two are staged)
 
-enum AdjCode { AC_M1 = 0, AC_M1C = 4, AC_X = 8, AC_XC = 12, AC_DIAG = 16, AC_SWAP = 17,
-               AC_M2 = 23, AC_GM1 = 64 };
+enum RoundType {
+    RT_RUN = 0,   // nrun runs of single-qubit gates, on register bits 0 .. nrun-1
+    RT_DIAG = 1,  // diagonal gates
+    RT_CTRL = 2,  // controlled 2x2 or X on register bit 0
+    RT_M2 = 3     // 4x4 on register bits 0 (high) and 1
+};
+
+constexpr int kMaxCst = 8;  // outside bits that a pass's map may depend on
+
+struct AdjRound {
+    int32_t type, nrun;
+    int32_t data;           // offset of its coefficients (doubles) in the program's data
+    int32_t ndiag;
+    uint32_t reg[4];        // byte offsets of the register bits (swizzled tile)
+    uint32_t base;          // byte offset of logical index 0
+    int32_t nlane;
+    int32_t slots;          // the pass's first gradient slot of this round << 8 | mask of runs
+                            // that have one
+    int32_t ncst;
+    uint32_t lane[12];      // byte offset << 4 | tile position of the thread-index bits
+    uint32_t cst_vec[kMaxCst];
+    int32_t cst_bit[kMaxCst];
+    uint64_t gpos[4];       // index masks of the register bits
+};
+static_assert(sizeof(AdjRound) % 16 == 0, "rounds are staged in 16-byte pieces");
+
+struct AdjMap {  // logical tile index -> byte offset in the swizzled tile
+    uint32_t vec[kMaxT];
+    uint32_t base;
+    int32_t ncst;
+    uint32_t cst_vec[kMaxCst];
+    int32_t cst_bit[kMaxCst];
+};
+
+struct AdjDiagOp {  // amplitude *= ph[pattern] where the index bits fix are all 1
+    uint64_t fix;
+    int32_t pb0, pb1, npat, pad;
+    double pad2;
+    double ph[8];
+};
+static_assert(sizeof(AdjDiagOp) == 12 * sizeof(double), "whole 16-byte pieces");
+
+struct AdjCtrlOp {
+    uint64_t gmask;      // index bits outside the registers that must be 1
+    int32_t cm, is_x;    // register bits that must be 1
+    double pad[2];
+    double m[8];
+};
+static_assert(sizeof(AdjCtrlOp) == 12 * sizeof(double), "whole 16-byte pieces");
 
 enum AtomKind { AT_CONST = 0, AT_RX = 1, AT_RY = 2, AT_RZ = 3 };
 
@@ -63,33 +121,51 @@ struct AdjRun {
     int32_t ntiles, pad;
 };
 
+// Consecutive rounds whose program (round records and data, each contiguous) is
+// staged into shared memory together.
+struct AdjChunk {
+    int32_t round_begin, nrounds;
+    int32_t data_begin, ndata;
+};
+
 struct AdjInst {
     int32_t n, T;
-    int32_t f_round, f_nrounds;  // small circuits: rounds forward and back
-    int32_t b_round, b_nrounds;
+    int32_t f_chunk, f_nchunks;  // small circuits: chunks forward and back
+    int32_t b_chunk, b_nchunks;
     int32_t group_begin, ngroups;
     int64_t off;                 // first amplitude in the wave's buffers (large circuits)
     int64_t epart;               // energy partials
     int32_t neparts, pad;
     int64_t part;                // small circuits: partial sums
+    int32_t map;                 // small circuits: layout of the final state
+    int32_t term_begin, nterms, pad2;
 };
 
 struct AdjPass {
     int32_t inst, h;
-    int32_t round_begin, nrounds;
+    int32_t chunk_begin, nchunks;
     int32_t tile_begin, ntiles;  // its blocks in the launch
     int64_t part;                // partial sums of its gradient runs
+    int32_t map, pad;            // layout after its last round
 };
 
 struct AdjGroup {  // Pauli terms sharing an X mask
-    uint64_t x;
+    uint32_t x;
     int32_t term_begin, nterms;
+    uint32_t vx;       // small circuits: x through the final state's layout
+    int32_t odd;       // some term has an odd number of Y (an imaginary element)
+    int32_t flat;      // no term has a Z bit among bits 8-10
 };
+static_assert(sizeof(AdjGroup) == 24, "staged in 8-byte pieces");
 
 struct AdjTerm {  // matrix element (-1)^popcount(i & z) (ca - i cb) between i and i ^ x
-    uint64_t z;
     double ca, cb;
+    uint32_t z;       // (circuits of at most 32 qubits)
+    uint8_t p;        // bits 8-10 of z: terms without X are sorted by it
+    uint8_t flips;    // bit k: parity of k & p, the sign between i and i + 256 k
+    uint16_t pad;
 };
+static_assert(sizeof(AdjTerm) == 24, "staged in 8-byte pieces");
 
 // ---------------------------------------------------------------------------
 // Device: coefficients of every run from the parameters
@@ -178,6 +254,19 @@ __global__ void __launch_bounds__(128)
 // ---------------------------------------------------------------------------
 // Device: register rounds
 // ---------------------------------------------------------------------------
+template <int K>
+__device__ __forceinline__ void m1_inplace(double2 (&v)[16], const double *__restrict__ c) {
+    const double2 m00 = *(const double2 *)c, m01 = *(const double2 *)(c + 2);
+    const double2 m10 = *(const double2 *)(c + 4), m11 = *(const double2 *)(c + 6);
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        if (e & (1 << K)) continue;
+        const double2 x0 = v[e], x1 = v[e | (1 << K)];
+        v[e] = cmad2(m00, x0, m01, x1);
+        v[e | (1 << K)] = cmad2(m10, x0, m11, x1);
+    }
+}
+
 // Sums of one gradient run over this thread's amplitudes: register elements 0-7 are
 // psi, 8-15 lambda.
 template <int K>
@@ -188,9 +277,9 @@ __device__ __forceinline__ void grad3(const double2 (&s)[16], double &sx, double
         if (e & (1 << K)) continue;
         const double2 a = s[e], b = s[e | (1 << K)];
         const double2 p = s[8 | e], q = s[8 | e | (1 << K)];
-        sz += fma(p.x, a.y, -(p.y * a.x)) - fma(q.x, b.y, -(q.y * b.x));
-        sx += fma(p.x, b.y, -(p.y * b.x)) + fma(q.x, a.y, -(q.y * a.x));
-        sy += fma(q.x, a.x, q.y * a.y) - fma(p.x, b.x, p.y * b.y);
+        sz = fma(p.x, a.y, fma(-p.y, a.x, fma(-q.x, b.y, fma(q.y, b.x, sz))));
+        sx = fma(p.x, b.y, fma(-p.y, b.x, fma(q.x, a.y, fma(-q.y, a.x, sx))));
+        sy = fma(q.x, a.x, fma(q.y, a.y, fma(-p.x, b.x, fma(-p.y, b.y, sy))));
     }
 }
 
@@ -218,116 +307,138 @@ __device__ __forceinline__ void grad_emit(const GradOut &go, int nwarps, int slo
     }
 }
 
-template <bool BWD, int NWARPS>
-__device__ __forceinline__ void adj_apply(const double2 (&s)[16], double2 (&d)[16],
-                                          const PassOp &op, const double *__restrict__ c,
-                                          uint64_t gbase, const uint64_t *__restrict__ gp,
-                                          const GradOut &go) {
-    int code = (gbase & op.gmask) == op.gmask ? op.code : -1;
-    if (BWD && code >= AC_GM1) {
-        code -= AC_GM1;
-        double sx, sy, sz;
-        if (code == 0) grad3<0>(s, sx, sy, sz);
-        else if (code == 1) grad3<1>(s, sx, sy, sz);
-        else grad3<2>(s, sx, sy, sz);
-        grad_emit(go, NWARPS, op.bits, sx, sy, sz);
-    }
-    switch (code) {
-    case AC_M1 + 0: pp_m1<0>(s, d, c, 0); break;
-    case AC_M1 + 1: pp_m1<1>(s, d, c, 0); break;
-    case AC_M1 + 2: pp_m1<2>(s, d, c, 0); break;
-    case AC_M1 + 3: if constexpr (!BWD) pp_m1<3>(s, d, c, 0); break;
-    case AC_M1C + 0: pp_m1<0>(s, d, c, op.cm); break;
-    case AC_M1C + 1: pp_m1<1>(s, d, c, op.cm); break;
-    case AC_M1C + 2: pp_m1<2>(s, d, c, op.cm); break;
-    case AC_M1C + 3: if constexpr (!BWD) pp_m1<3>(s, d, c, op.cm); break;
-    case AC_X + 0: pp_x<0>(s, d, 0); break;
-    case AC_X + 1: pp_x<1>(s, d, 0); break;
-    case AC_X + 2: pp_x<2>(s, d, 0); break;
-    case AC_X + 3: if constexpr (!BWD) pp_x<3>(s, d, 0); break;
-    case AC_XC + 0: pp_x<0>(s, d, op.cm); break;
-    case AC_XC + 1: pp_x<1>(s, d, op.cm); break;
-    case AC_XC + 2: pp_x<2>(s, d, op.cm); break;
-    case AC_XC + 3: if constexpr (!BWD) pp_x<3>(s, d, op.cm); break;
-    case AC_DIAG: pp_diag(s, d, op, c, gbase, gp); break;
-    case AC_SWAP + 0: pp_swap<0, 1>(s, d); break;
-    case AC_SWAP + 1: pp_swap<0, 2>(s, d); break;
-    case AC_SWAP + 2: if constexpr (!BWD) pp_swap<0, 3>(s, d); break;
-    case AC_SWAP + 3: pp_swap<1, 2>(s, d); break;
-    case AC_SWAP + 4: if constexpr (!BWD) pp_swap<1, 3>(s, d); break;
-    case AC_SWAP + 5: if constexpr (!BWD) pp_swap<2, 3>(s, d); break;
-    case AC_M2 + 0: pp_m2<0, 1, false>(s, d, c); break;
-    case AC_M2 + 1: pp_m2<0, 2, false>(s, d, c); break;
-    case AC_M2 + 2: if constexpr (!BWD) pp_m2<0, 3, false>(s, d, c); break;
-    case AC_M2 + 3: pp_m2<1, 2, false>(s, d, c); break;
-    case AC_M2 + 4: if constexpr (!BWD) pp_m2<1, 3, false>(s, d, c); break;
-    case AC_M2 + 5: if constexpr (!BWD) pp_m2<2, 3, false>(s, d, c); break;
-    default:
-#pragma unroll
-        for (int e = 0; e < 16; ++e) d[e] = s[e];
-        break;
-    }
-}
-
 // One round for register set `v` (of 2^(T-4) forward, 2^(T-3) back) of the tile.
-template <bool BWD, int NWARPS>
-__device__ __forceinline__ void adj_round(uint32_t tile_a, const FusedRound &rd,
-                                          const PassOp *__restrict__ ops,
-                                          const double *__restrict__ coef, uint64_t tile_base,
+template <bool BWD, int NW>
+__device__ __forceinline__ void adj_round(uint32_t tile_a, const AdjRound &rd,
+                                          const double *__restrict__ data, uint64_t tile_base,
                                           int h, int v, const GradOut &go) {
+    uint32_t sb = rd.base;
     int tbase = 0;
-    for (int j = 0; j < rd.nlane; ++j) tbase |= ((v >> j) & 1) << rd.lane[j];
-    const uint32_t sb = (uint32_t)swz(tbase) << 4;
-    const uint64_t gbase = tile_base | (uint64_t)(tbase & 15) | ((uint64_t)(tbase >> 4) << h);
-    const uint32_t E0 = (uint32_t)rd.eoff[1], E1 = (uint32_t)rd.eoff[2];
-    const uint32_t E2 = (uint32_t)rd.eoff[4], E3 = (uint32_t)rd.eoff[8];
+    for (int j = 0; j < rd.nlane; ++j) {
+        const uint32_t on = 0u - ((uint32_t)(v >> j) & 1u), w = rd.lane[j];
+        sb ^= (w >> 4) & on;
+        tbase |= (int)((1u << (w & 15u)) & on);
+    }
+    for (int j = 0; j < rd.ncst; ++j)
+        sb ^= rd.cst_vec[j] & (0u - (uint32_t)((tile_base >> rd.cst_bit[j]) & 1ull));
+    const uint32_t E0 = rd.reg[0], E1 = rd.reg[1], E2 = rd.reg[2], E3 = rd.reg[3];
     auto addr_of = [&](int e) {
         const uint32_t x = ((e & 1) ? E0 : 0u) ^ ((e & 2) ? E1 : 0u) ^ ((e & 4) ? E2 : 0u) ^
                            ((e & 8) ? E3 : 0u);
         return tile_a + (sb ^ x);
     };
-    double2 a[16], b[16];
-#pragma unroll
-    for (int e = 0; e < 16; ++e)
-        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
-                     : "=d"(a[e].x), "=d"(a[e].y)
-                     : "r"(addr_of(e)));
-    const int o1 = rd.op_end;
-    int o = rd.op_begin;
-    for (; o + 1 < o1; o += 2) {
-        const PassOp p0 = ops[o];
-        const PassOp p1 = ops[o + 1];
-        adj_apply<BWD, NWARPS>(a, b, p0, coef + p0.coef, gbase, rd.gpos, go);
-        adj_apply<BWD, NWARPS>(b, a, p1, coef + p1.coef, gbase, rd.gpos, go);
-    }
-    const bool odd = o < o1;
-    if (odd) {
-        const PassOp p0 = ops[o];
-        adj_apply<BWD, NWARPS>(a, b, p0, coef + p0.coef, gbase, rd.gpos, go);
-    }
-    if (odd) {
+    double2 a[16];
+    auto load = [&]() {
 #pragma unroll
         for (int e = 0; e < 16; ++e)
-            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr_of(e)), "d"(b[e].x),
-                         "d"(b[e].y)
+            asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
+                         : "=d"(a[e].x), "=d"(a[e].y)
+                         : "r"(addr_of(e)));
+    };
+    auto store = [&](const double2 (&x)[16]) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr_of(e)), "d"(x[e].x),
+                         "d"(x[e].y)
                          : "memory");
+    };
+    const double *c = data + rd.data;
+    if (rd.type == RT_RUN) {
+        // Load, runs and store in each branch: no register is live across the joins.
+#define LQ_RUN(K)                                                \
+    {                                                            \
+        if constexpr (BWD) {                                     \
+            double sx, sy, sz;                                   \
+            grad3<K>(a, sx, sy, sz);                             \
+            grad_emit(go, NW, K, sx, sy, sz);                    \
+        }                                                        \
+        m1_inplace<K>(a, c + 8 * K);                             \
+    }
+        if (rd.nrun == 3) {
+            load();
+            LQ_RUN(0) LQ_RUN(1) LQ_RUN(2)
+            store(a);
+        } else if (rd.nrun == 2) {
+            load();
+            LQ_RUN(0) LQ_RUN(1)
+            store(a);
+        } else if (rd.nrun == 1) {
+            load();
+            LQ_RUN(0)
+            store(a);
+        } else if constexpr (!BWD) {
+            load();
+            LQ_RUN(0) LQ_RUN(1) LQ_RUN(2) LQ_RUN(3)
+            store(a);
+        }
+#undef LQ_RUN
+        return;
+    }
+    const uint64_t gbase = tile_base | (uint64_t)(tbase & 15) | ((uint64_t)(tbase >> 4) << h);
+    load();
+    if (rd.type == RT_DIAG) {
+        for (int k = 0; k < rd.ndiag; ++k) {
+            const AdjDiagOp &op = ((const AdjDiagOp *)c)[k];
+            const uint64_t fm = op.fix;
+            const uint64_t u0 = op.npat > 0 ? 1ull : 0ull, u1 = op.npat > 1 ? 1ull : 0ull;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const uint64_t gi = gbase | ((e & 1) ? rd.gpos[0] : 0ull) |
+                                    ((e & 2) ? rd.gpos[1] : 0ull) | ((e & 4) ? rd.gpos[2] : 0ull) |
+                                    ((e & 8) ? rd.gpos[3] : 0ull);
+                if ((gi & fm) != fm) continue;
+                const int pat = (int)((gi >> op.pb0) & u0) | (int)((gi >> op.pb1) & u1) << 1;
+                const double pr = op.ph[2 * pat], pi = op.ph[2 * pat + 1];
+                a[e] = make_double2(fma(-a[e].y, pi, a[e].x * pr), fma(a[e].x, pi, a[e].y * pr));
+            }
+        }
+        store(a);
+    } else if (rd.type == RT_CTRL) {
+        const AdjCtrlOp &op = *(const AdjCtrlOp *)c;
+        if ((gbase & op.gmask) != op.gmask) return;
+        double2 d[16];
+        if (op.is_x) pp_x<0>(a, d, op.cm);
+        else pp_m1<0>(a, d, op.m, op.cm);
+        store(d);
     } else {
-#pragma unroll
-        for (int e = 0; e < 16; ++e)
-            asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr_of(e)), "d"(a[e].x),
-                         "d"(a[e].y)
-                         : "memory");
+        double2 d[16];
+        pp_m2<0, 1, false>(a, d, c);
+        store(d);
     }
 }
 
+struct AdjProg {  // the device program
+    const AdjRound *rounds;
+    const double *data;
+    const AdjChunk *chunks;
+    const AdjMap *maps;
+};
+
+// Start the copy of one chunk's program into shared memory: round records, then data.
+template <int NT>
+__device__ __forceinline__ void adj_stage(uint32_t dst, const AdjChunk &ch, const AdjProg &pg) {
+    auto copy = [&](const void *src, int bytes) {
+        for (int o = (int)threadIdx.x * 16; o < bytes; o += NT * 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)o),
+                         "l"((const char *)src + o)
+                         : "memory");
+        dst += (uint32_t)bytes;
+    };
+    copy(pg.rounds + ch.round_begin, ch.nrounds * (int)sizeof(AdjRound));
+    copy(pg.data + ch.data_begin, ch.ndata * (int)sizeof(double));
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
 // All rounds of one pass on the tile, with the gradient runs' sums over the tile
-// written to part[(slot * 3 + c) * ntiles + tile].  FusedRound::pad holds the
-// round's first slot << 8 | its slot count.
+// written to part[(slot * 3 + c) * ntiles + tile].
+//
+// The program comes from shared memory, staged chunk by chunk (the caller has
+// started the first one): every circuit has its own, read by a few tiles only, so
+// a record read where it is used would miss the first-level cache every time.
 template <bool BWD, int NT>
 __device__ __forceinline__ void adj_rounds(uint32_t tile_a, int T, int h, uint64_t tile_base,
-                                           const FusedRound *__restrict__ rounds, int nrounds,
-                                           const PassOp *__restrict__ ops,
-                                           const double *__restrict__ coef, double *s_part,
+                                           const AdjProg &pg, int chunk, int nchunks,
+                                           unsigned char *stage, double *s_part,
                                            double *__restrict__ part, int ntiles, int tile) {
     constexpr int NW = NT / 32;
     const int tid = threadIdx.x;
@@ -336,43 +447,78 @@ __device__ __forceinline__ void adj_rounds(uint32_t tile_a, int T, int h, uint64
     go.mask = nthr >= 32 ? 0xffffffffu : (1u << nthr) - 1u;
     go.half = nthr >= 32 ? 16 : nthr >> 1;
     const int nw = nthr >= NT ? NW : nthr >= 32 ? nthr >> 5 : 1;  // warps that hold amplitudes
-    for (int r = 0; r < nrounds; ++r) {
-        const FusedRound &rd = rounds[r];
-        go.part = s_part + (r & 1) * (kRoundSlots * 3 * NW);
-        for (int v = tid; v < nthr; v += NT) {
-            go.add = v != tid;
-            adj_round<BWD, NW>(tile_a, rd, ops, coef, tile_base, h, v, go);
-        }
+    int parity = 0;
+    if (nchunks == 0) {  // permutations only: the map does it all
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
-        if (BWD) {
-            // (this half of s_part is written again two rounds on, after the next barrier)
-            const int cnt = (rd.pad & 0xff) * 3, first = (rd.pad >> 8) * 3;
-            for (int k = tid; k < cnt; k += NT) {
-                double sum = 0.0;
-                for (int w = 0; w < nw; ++w) sum += go.part[k * NW + w];
-                part[(int64_t)(first + k) * ntiles + tile] = sum;
+    }
+    for (int c = 0; c < nchunks; ++c) {
+        const AdjChunk ch = pg.chunks[chunk + c];
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        unsigned char *cur = stage + (c & 1) * kStageBytes;
+        if (c + 1 < nchunks)  // (that half was last read before the barrier above)
+            adj_stage<NT>(smem_u32(stage + ((c + 1) & 1) * kStageBytes), pg.chunks[chunk + c + 1],
+                          pg);
+        const AdjRound *rounds = (const AdjRound *)cur;
+        const double *data = (const double *)(rounds + ch.nrounds) - ch.data_begin;
+        for (int r = 0; r < ch.nrounds; ++r) {
+            const AdjRound &rd = rounds[r];
+            go.part = s_part + parity * (kRoundSlots * 3 * NW);
+            parity ^= 1;
+            for (int v = tid; v < nthr; v += NT) {
+                go.add = v != tid;
+                adj_round<BWD, NW>(tile_a, rd, data, tile_base, h, v, go);
+            }
+            __syncthreads();
+            if (BWD) {
+                // (this half of s_part is written again two rounds on, past a barrier)
+                // Runs with a parameter have the pass's next slots, in order.
+                const int first = rd.slots >> 8;
+                if (tid < 3 * kRoundSlots && (rd.slots >> (tid / 3) & 1)) {
+                    const int slot = first + __popc(rd.slots & ((1 << (tid / 3)) - 1));
+                    double sum = 0.0;
+                    for (int w = 0; w < nw; ++w) sum += go.part[tid * NW + w];
+                    part[(int64_t)(slot * 3 + tid % 3) * ntiles + tile] = sum;
+                }
             }
         }
     }
 }
 
-__device__ __forceinline__ void adj_sign_term(const AdjTerm &t, uint64_t i, double &al,
+__device__ __forceinline__ uint32_t map_base(const AdjMap &m, uint64_t tile_base) {
+    uint32_t b = m.base;
+    for (int j = 0; j < m.ncst; ++j)
+        b ^= m.cst_vec[j] & (0u - (uint32_t)((tile_base >> m.cst_bit[j]) & 1ull));
+    return b;
+}
+
+__device__ __forceinline__ uint32_t map_of(const AdjMap &m, uint32_t base, int l, int T) {
+    for (int j = 0; j < T; ++j) base ^= m.vec[j] & (0u - ((uint32_t)(l >> j) & 1u));
+    return base;
+}
+
+__device__ __forceinline__ double flip_sign(double x, uint32_t neg) {  // neg: bit 0 counts
+    return __hiloint2double(__double2hiint(x) ^ (int)(neg << 31), __double2loint(x));
+}
+
+__device__ __forceinline__ void adj_sign_term(const AdjTerm &t, uint32_t i, double &al,
                                               double &be) {
-    const bool neg = __popcll(i & t.z) & 1;
-    al += neg ? -t.ca : t.ca;
-    be += neg ? -t.cb : t.cb;
+    const uint32_t neg = (uint32_t)__popc(i & t.z);
+    al += flip_sign(t.ca, neg);
+    be += flip_sign(t.cb, neg);
 }
 
 // ---------------------------------------------------------------------------
 // Small circuits: everything in one CTA
 // ---------------------------------------------------------------------------
 constexpr size_t adj_small_smem(int T) {
-    return ((size_t)32 << T) + 1024 + sizeof(double) * 2 * kRoundSlots * 3 * (kAdjSmallThreads / 32);
+    return ((size_t)32 << T) + 1024 + 2 * kStageBytes +
+           sizeof(double) * 2 * kRoundSlots * 3 * (kAdjSmallThreads / 32);
 }
 
 __global__ void __launch_bounds__(kAdjSmallThreads, 1)
-    k_adj_small(const AdjInst *__restrict__ insts, const FusedRound *__restrict__ rounds,
-                const PassOp *__restrict__ ops, const double *__restrict__ coef,
+    k_adj_small(const AdjInst *__restrict__ insts, AdjProg pg,
                 const AdjGroup *__restrict__ groups, const AdjTerm *__restrict__ terms,
                 double *__restrict__ part, double *__restrict__ epart) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -380,36 +526,43 @@ __global__ void __launch_bounds__(kAdjSmallThreads, 1)
     const uint32_t tile_a = smem_u32(base);
     const AdjInst in = insts[blockIdx.x];
     const int T = in.n, tid = threadIdx.x, N = 1 << T;
-    double *s_part = (double *)(base + ((size_t)32 << T));
+    unsigned char *stage = base + ((size_t)32 << T);
+    double *s_part = (double *)(stage + 2 * kStageBytes);
     __shared__ double s_e[kAdjSmallThreads / 32];
     auto addr = [&](int l) { return tile_a + ((uint32_t)swz(l) << 4); };
+    if (in.f_nchunks) adj_stage<kAdjSmallThreads>(smem_u32(stage), pg.chunks[in.f_chunk], pg);
     for (int l = tid; l < N; l += kAdjSmallThreads)
         asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr(l)), "d"(l == 0 ? 1.0 : 0.0),
                      "d"(0.0)
                      : "memory");
     __syncthreads();
-    adj_rounds<false, kAdjSmallThreads>(tile_a, T, 4, 0ull, rounds + in.f_round, in.f_nrounds, ops,
-                                        coef, s_part, nullptr, 1, 0);
-    // lambda = H psi, and the energy
+    adj_rounds<false, kAdjSmallThreads>(tile_a, T, 4, 0ull, pg, in.f_chunk, in.f_nchunks, stage,
+                                        s_part, nullptr, 1, 0);
+    if (in.b_nchunks) adj_stage<kAdjSmallThreads>(smem_u32(stage), pg.chunks[in.b_chunk], pg);
+    // lambda = H psi, and the energy; lambda takes psi's layout
+    const AdjMap &mp = pg.maps[in.map];
+    const uint32_t sel = (uint32_t)swz(N) << 4;
     double e = 0.0;
     for (int l = tid; l < N; l += kAdjSmallThreads) {
+        const uint32_t at = map_of(mp, mp.base, l, T);
         double2 lam = make_double2(0.0, 0.0);
         for (int g = in.group_begin; g < in.group_begin + in.ngroups; ++g) {
             const AdjGroup gr = groups[g];
             double2 v;
             asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
                          : "=d"(v.x), "=d"(v.y)
-                         : "r"(addr(l ^ (int)gr.x)));
+                         : "r"(tile_a + (at ^ gr.vx)));
             double al = 0.0, be = 0.0;
             for (int t = gr.term_begin; t < gr.term_begin + gr.nterms; ++t)
-                adj_sign_term(terms[t], (uint64_t)l, al, be);
+                adj_sign_term(terms[t], (uint32_t)l, al, be);
             lam.x += fma(al, v.x, be * v.y);
             lam.y += fma(al, v.y, -(be * v.x));
         }
         double2 a;
-        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a.x), "=d"(a.y) : "r"(addr(l)));
+        asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(a.x), "=d"(a.y) : "r"(tile_a + at));
         e += fma(a.x, lam.x, a.y * lam.y);
-        asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(addr(l | N)), "d"(lam.x), "d"(lam.y)
+        asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(tile_a + (at ^ sel)), "d"(lam.x),
+                     "d"(lam.y)
                      : "memory");
     }
 #pragma unroll
@@ -421,28 +574,27 @@ __global__ void __launch_bounds__(kAdjSmallThreads, 1)
         for (int w = 0; w < kAdjSmallThreads / 32; ++w) sum += s_e[w];
         epart[in.epart] = sum;
     }
-    adj_rounds<true, kAdjSmallThreads>(tile_a, T, 4, 0ull, rounds + in.b_round, in.b_nrounds, ops,
-                                       coef, s_part, part + in.part, 1, 0);
+    adj_rounds<true, kAdjSmallThreads>(tile_a, T, 4, 0ull, pg, in.b_chunk, in.b_nchunks, stage,
+                                       s_part, part + in.part, 1, 0);
 }
 
 // ---------------------------------------------------------------------------
 // Large circuits: one launch per pass over the tiles of all circuits of a wave
 // ---------------------------------------------------------------------------
 static size_t adj_pass_smem(int T, bool bwd) {
-    return ((size_t)(bwd ? 32 : 16) << T) + 1024 +
+    return ((size_t)(bwd ? 32 : 16) << T) + 1024 + 2 * kStageBytes +
            sizeof(double) * 2 * kRoundSlots * 3 * (kAdjThreads / 32);
 }
 
 template <bool BWD>
 __global__ void __launch_bounds__(kAdjThreads, 3)
     k_adj_pass(const AdjInst *__restrict__ insts, const AdjPass *__restrict__ passes, int npasses,
-               const FusedRound *__restrict__ rounds, const PassOp *__restrict__ ops,
-               const double *__restrict__ coef, double2 *__restrict__ psi,
-               double2 *__restrict__ lam, double *__restrict__ part, int T, int first) {
+               AdjProg pg, double2 *__restrict__ psi, double2 *__restrict__ lam, double *__restrict__ part, int T, int first) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t tile_a = smem_u32(base);
-    double *s_part = (double *)(base + ((size_t)(BWD ? 32 : 16) << T));
+    unsigned char *stage = base + ((size_t)(BWD ? 32 : 16) << T);
+    double *s_part = (double *)(stage + 2 * kStageBytes);
     const int tid = threadIdx.x;
     int lo = 0, hi = npasses - 1;  // the pass whose tiles hold this block
     while (lo < hi) {
@@ -457,6 +609,7 @@ __global__ void __launch_bounds__(kAdjThreads, 3)
     const uint64_t tb = (c2 << 4) | (c4 << (h + T - 4));
     auto global_of = [&](int l) { return tb | (uint64_t)(l & 15) | ((uint64_t)(l >> 4) << h); };
     const int N = 1 << T;
+    if (ps.nchunks) adj_stage<kAdjThreads>(smem_u32(stage), pg.chunks[ps.chunk_begin], pg);
     if (!BWD && first) {  // |0...0>
         for (int l = tid; l < N; l += kAdjThreads)
             asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(tile_a + ((uint32_t)swz(l) << 4)),
@@ -476,35 +629,50 @@ __global__ void __launch_bounds__(kAdjThreads, 3)
                              : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    __syncthreads();
-    adj_rounds<BWD, kAdjThreads>(tile_a, T, h, tb, rounds + ps.round_begin, ps.nrounds, ops, coef,
-                                 s_part, part + ps.part, ps.ntiles, tile);
+    // (adj_rounds waits for every copy and synchronises before its first round)
+    adj_rounds<BWD, kAdjThreads>(tile_a, T, h, tb, pg, ps.chunk_begin, ps.nchunks, stage, s_part,
+                                 part + ps.part, ps.ntiles, tile);
     if (BWD && first) return;  // the last pass back: nothing reads the states again
-    for (int l = tid; l < N; l += kAdjThreads) {
-        const uint64_t g = global_of(l);
+    const AdjMap &mp = pg.maps[ps.map];
+    const uint32_t sel = (uint32_t)swz(N) << 4;
+    // (thread-index bits once, the upper ones by the loop count)
+    const uint32_t mb = map_of(mp, map_base(mp, tb), tid, 7);
+    static_assert(kAdjThreads == 128, "seven thread-index bits");
+    for (int k = 0; k < (N >> 7); ++k) {
+        uint32_t at = mb;
+        for (int j = 7; j < T; ++j) at ^= mp.vec[j] & (0u - ((uint32_t)(k >> (j - 7)) & 1u));
+        const uint64_t g = global_of(tid + (k << 7));
         double2 v;
         asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
                      : "=d"(v.x), "=d"(v.y)
-                     : "r"(tile_a + ((uint32_t)swz(l) << 4)));
+                     : "r"(tile_a + at));
         psi[off + g] = v;
         if (BWD) {
             asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];"
                          : "=d"(v.x), "=d"(v.y)
-                         : "r"(tile_a + ((uint32_t)swz(l | N) << 4)));
+                         : "r"(tile_a + (at ^ sel)));
             lam[off + g] = v;
         }
     }
 }
 
 // lambda = H psi and the energy's partial sums, one block per kHChunk amplitudes.
-__global__ void __launch_bounds__(256)
+// A thread takes the eight amplitudes i0 + 256 k: a term's sign at k is its sign at
+// i0 times the parity of k and its bits 8-10, so the parity is taken once per term, a
+// group without such bits has one coefficient for all eight, and the terms without X
+// fold into one 8-point Walsh-Hadamard transform.  Only groups with an odd number of
+// Y somewhere have an imaginary coefficient.  (6.3 M amplitudes of 13-16-qubit
+// chains: 371 us, 950 instructions per amplitude, with a sign per term and amplitude.)
+__global__ void __launch_bounds__(256, 2)
     k_adj_h(const AdjInst *__restrict__ insts, const int32_t *__restrict__ list, int count,
             const int64_t *__restrict__ chunk_begin, const AdjGroup *__restrict__ groups,
             const AdjTerm *__restrict__ terms, const double2 *__restrict__ psi,
             double2 *__restrict__ lam, double *__restrict__ epart) {
     __shared__ double s_e[8];
+    __shared__ __align__(16) unsigned char s_h[kHStage];
+    constexpr int kA = kHChunk / 256;
+    static_assert(kA == 8, "the fold is over index bits 8 to 10");
     const int64_t blk = blockIdx.x;
     int lo = 0, hi = count - 1;
     while (lo < hi) {
@@ -515,36 +683,96 @@ __global__ void __launch_bounds__(256)
     const AdjInst in = insts[list[lo]];
     const int64_t chunk = blk - chunk_begin[lo];
     const double2 *v = psi + in.off;
-    constexpr int kA = kHChunk / 256;
-    const uint64_t i0 = (uint64_t)chunk * kHChunk + threadIdx.x;
-    double2 acc[kA];
+    const uint32_t i0 = (uint32_t)chunk * kHChunk + threadIdx.x;
+    double2 acc[kA], own[kA];
 #pragma unroll
-    for (int k = 0; k < kA; ++k) acc[k] = make_double2(0.0, 0.0);
-    for (int g = in.group_begin; g < in.group_begin + in.ngroups; ++g) {
-        const AdjGroup gr = groups[g];
+    for (int k = 0; k < kA; ++k) {
+        acc[k] = make_double2(0.0, 0.0);
+        own[k] = v[i0 + 256u * k];
+    }
+    const AdjGroup *gp = groups + in.group_begin;
+    const AdjTerm *tp = terms + in.term_begin;
+    const int gb = in.ngroups * (int)sizeof(AdjGroup), tb = in.nterms * (int)sizeof(AdjTerm);
+    if (gb + tb <= kHStage) {
+        for (int o = (int)threadIdx.x * 8; o < gb; o += 256 * 8)
+            *(double *)(s_h + o) = *(const double *)((const char *)gp + o);
+        for (int o = (int)threadIdx.x * 8; o < tb; o += 256 * 8)
+            *(double *)(s_h + gb + o) = *(const double *)((const char *)tp + o);
+        __syncthreads();
+        gp = (const AdjGroup *)s_h;
+        tp = (const AdjTerm *)(s_h + gb);
+    }
+    for (int g = 0; g < in.ngroups; ++g) {
+        const AdjGroup gr = gp[g];
+        const AdjTerm *t0 = tp + (gr.term_begin - in.term_begin);
+        if (gr.x == 0) {
+            double c[8];
+            int t = 0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                c[q] = 0.0;
+                for (; t < gr.nterms && t0[t].p == q; ++t)
+                    c[q] += flip_sign(t0[t].ca, (uint32_t)__popc(i0 & t0[t].z));
+            }
+#pragma unroll
+            for (int hs = 1; hs < 8; hs <<= 1)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    if (q & hs) continue;
+                    const double x = c[q], y = c[q | hs];
+                    c[q] = x + y;
+                    c[q | hs] = x - y;
+                }
+#pragma unroll
+            for (int k = 0; k < kA; ++k) {
+                acc[k].x = fma(c[k], own[k].x, acc[k].x);
+                acc[k].y = fma(c[k], own[k].y, acc[k].y);
+            }
+            continue;
+        }
         double2 x[kA];
-        double al[kA], be[kA];
 #pragma unroll
-        for (int k = 0; k < kA; ++k) {
-            x[k] = v[(i0 + 256u * k) ^ gr.x];
-            al[k] = be[k] = 0.0;
+        for (int k = 0; k < kA; ++k) x[k] = v[(i0 + 256u * k) ^ gr.x];
+        if (gr.flat) {
+            double al = 0.0, be = 0.0;
+            for (int t = 0; t < gr.nterms; ++t) adj_sign_term(t0[t], i0, al, be);
+#pragma unroll
+            for (int k = 0; k < kA; ++k) {
+                acc[k].x = fma(al, x[k].x, acc[k].x);
+                acc[k].y = fma(al, x[k].y, acc[k].y);
+            }
+            if (gr.odd) {
+#pragma unroll
+                for (int k = 0; k < kA; ++k) {
+                    acc[k].x = fma(be, x[k].y, acc[k].x);
+                    acc[k].y = fma(-be, x[k].x, acc[k].y);
+                }
+            }
+            continue;
         }
-        for (int t = gr.term_begin; t < gr.term_begin + gr.nterms; ++t) {
-            const AdjTerm tm = terms[t];
+        for (int t = 0; t < gr.nterms; ++t) {
+            const AdjTerm tm = t0[t];
+            const uint32_t f = tm.flips ^ (0u - ((uint32_t)__popc(i0 & tm.z) & 1u));
 #pragma unroll
-            for (int k = 0; k < kA; ++k) adj_sign_term(tm, i0 + 256u * k, al[k], be[k]);
-        }
+            for (int k = 0; k < kA; ++k) {
+                const double al = flip_sign(tm.ca, f >> k);
+                acc[k].x = fma(al, x[k].x, acc[k].x);
+                acc[k].y = fma(al, x[k].y, acc[k].y);
+            }
+            if (gr.odd) {
 #pragma unroll
-        for (int k = 0; k < kA; ++k) {
-            acc[k].x += fma(al[k], x[k].x, be[k] * x[k].y);
-            acc[k].y += fma(al[k], x[k].y, -(be[k] * x[k].x));
+                for (int k = 0; k < kA; ++k) {
+                    const double be = flip_sign(tm.cb, f >> k);
+                    acc[k].x = fma(be, x[k].y, acc[k].x);
+                    acc[k].y = fma(-be, x[k].x, acc[k].y);
+                }
+            }
         }
     }
     double e = 0.0;
 #pragma unroll
     for (int k = 0; k < kA; ++k) {
-        const double2 a = v[i0 + 256u * k];
-        e += fma(a.x, acc[k].x, a.y * acc[k].y);
+        e += fma(own[k].x, acc[k].x, own[k].y * acc[k].y);
         lam[in.off + i0 + 256u * k] = acc[k];
     }
 #pragma unroll
@@ -613,14 +841,15 @@ public:
     int small_T = kAdjMinN;
     std::vector<AdjInst> insts;      // large circuits after the small ones
     std::vector<int> order;          // insts[k] is the caller's circuit order[k]
-    std::vector<FusedRound> rounds;
-    std::vector<PassOp> ops;
-    std::vector<double> coef;        // static part filled in; runs' entries written on the device
+    std::vector<AdjRound> rounds;
+    std::vector<double> data;        // static part filled in; runs' entries written on the device
+    std::vector<AdjMap> maps;
     std::vector<AdjAtom> atoms;
     std::vector<AdjRun> runs;
     std::vector<AdjGroup> groups;
     std::vector<AdjTerm> terms;
     std::vector<AdjPass> passes;
+    std::vector<AdjChunk> chunks;
     std::vector<int32_t> h_list;
     std::vector<int64_t> h_chunk;
     std::vector<AdjWave> waves;
@@ -630,21 +859,28 @@ public:
     double2 *states = nullptr;
     size_t blob_bytes = 0;
     AdjInst *d_insts = nullptr;
-    FusedRound *d_rounds = nullptr;
-    PassOp *d_ops = nullptr;
-    double *d_coef = nullptr, *d_wts = nullptr, *d_part = nullptr, *d_epart = nullptr;
+    AdjRound *d_rounds = nullptr;
+    AdjMap *d_maps = nullptr;
+    double *d_data = nullptr, *d_wts = nullptr, *d_part = nullptr, *d_epart = nullptr;
     double *d_theta = nullptr, *d_out = nullptr;
     AdjAtom *d_atoms = nullptr;
     AdjRun *d_runs = nullptr;
     AdjGroup *d_groups = nullptr;
     AdjTerm *d_terms = nullptr;
     AdjPass *d_passes = nullptr;
+    AdjChunk *d_chunks = nullptr;
     int32_t *d_hlist = nullptr;
     int64_t *d_hchunk = nullptr;
     double2 *psi = nullptr, *lam = nullptr;
     bool own_blob = false;
+    // the small circuits run beside the large ones
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 
     ~AdjProgram() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
         if (own_blob) cudaFree(blob);
         if (states) cudaFree(states);
     }
@@ -714,8 +950,8 @@ static bool gate_atoms(const lq_gate &g, int param_base, const GateOp &op, AdjPr
     AdjAtom a{};
     a.kind = AT_CONST;
     a.param = -1;
-    a.cmat = (int64_t)p.coef.size();
-    p.coef.insert(p.coef.end(), m, m + 8);
+    a.cmat = (int64_t)p.data.size();
+    p.data.insert(p.data.end(), m, m + 8);
     out.push_back(a);
     return true;
 }
@@ -731,50 +967,242 @@ static int angles_of(int kind) {
     }
 }
 
-// Encode the rounds of one planned pass.  op_run[i] is the run of planned op i
-// (-1: a gate with static coefficients); slots counts the pass's gradient runs.
-static void adj_encode_pass(const PlannedPass &ps, const std::vector<GateOp> &gops,
-                            const std::vector<int> &op_run, bool bwd, int T, AdjProgram &p,
-                            std::vector<int> &slot_runs) {
-    for (const PlannedRound &rd : ps.rounds) {
-        FusedRound fr{};
-        fill_round(fr, rd.rpos, T, ps.h);
-        auto open = [&]() {
-            fr.op_begin = (int)p.ops.size();
-            fr.pad = (int)slot_runs.size() << 8;
-        };
-        auto close = [&]() {
-            fr.op_end = (int)p.ops.size();
-            p.rounds.push_back(fr);
-        };
-        open();
-        for (int k : rd.ops) {
-            const int gi = ps.gates[k], run = op_run[gi];
-            const bool slot = bwd && run >= 0 && p.runs[run].ntiles > 0;
-            if (slot && (fr.pad & 0xff) == kRoundSlots) {  // same register bits, a new round
-                close();
-                open();
-            }
-            std::vector<FusedOp> one;
-            std::vector<double> c;
-            encode_op(gops[gi], ps.h, T - 4, rd.rpos, one, c);
-            PassOp po = pass_op(one[0]);
-            if (run >= 0) {
-                po.coef = (int32_t)(bwd ? p.runs[run].coef_b : p.runs[run].coef_f);
-                if (slot) {
-                    po.code += AC_GM1;
-                    po.bits = fr.pad & 0xff;
-                    slot_runs.push_back(run);
-                    ++fr.pad;
-                }
-            } else {
-                po.coef = (int32_t)p.coef.size();
-                p.coef.insert(p.coef.end(), c.begin(), c.end());
-            }
-            p.ops.push_back(po);
-        }
-        close();
+// A tile's map while its pass is planned (places unswizzled).
+struct PlanMap {
+    uint32_t vec[kMaxT + 1];
+    uint32_t base = 0;
+    std::vector<std::pair<int, uint32_t>> cst;  // outside bit, vector
+    explicit PlanMap(int T) {
+        for (int b = 0; b <= T; ++b) vec[b] = 1u << b;
     }
+};
+
+static uint32_t place(uint32_t v) { return (uint32_t)swz((int)v) << 4; }
+
+static bool linear_perm(const GateOp &g) {
+    return g.type == OP_SWAP || (g.type == OP_PERM1 && g.nctrl <= 1);
+}
+
+// Plan and encode the rounds of one pass (its gates in order) into chunks.  op_run[i]
+// is the run of op i (-1: a gate with static coefficients); slot_runs collects the
+// pass's gradient runs; map is the layout before and after.
+static void adj_encode_pass(const std::vector<int> &gates, const std::vector<GateOp> &gops,
+                            const std::vector<int> &op_run, bool bwd, int T, int h, PlanMap &map,
+                            AdjProgram &p, std::vector<int> &slot_runs) {
+    const int maxr = bwd ? 3 : 4, m = T - 4;
+    auto local = [&](int b) { return b < 4 ? b : b >= h && b < h + m ? 4 + (b - h) : -1; };
+    AdjChunk ch{(int)p.rounds.size(), 0, (int)p.data.size(), 0};
+    auto close_chunk = [&]() {
+        ch.nrounds = (int)p.rounds.size() - ch.round_begin;
+        ch.ndata = (int)p.data.size() - ch.data_begin;
+        if (ch.nrounds) p.chunks.push_back(ch);
+        ch = AdjChunk{(int)p.rounds.size(), 0, (int)p.data.size(), 0};
+    };
+    constexpr int kDiagsPerRound = 8;
+    auto emit = [&](int type, std::vector<int> bits, const std::vector<int> &ops) {
+        // the largest round: its record and kDiagsPerRound diagonal gates
+        constexpr size_t kMost = sizeof(AdjRound) + kDiagsPerRound * sizeof(AdjDiagOp);
+        static_assert(kMost <= kStageBytes, "a chunk holds any round");
+        if ((p.rounds.size() - ch.round_begin) * sizeof(AdjRound) +
+                (p.data.size() - ch.data_begin) * sizeof(double) + kMost > kStageBytes)
+            close_chunk();
+        AdjRound rd{};
+        rd.type = type;
+        rd.data = (int)p.data.size();
+        // Register bits: the op's, then pads.  Eight consecutive threads should touch
+        // eight 16-byte bank groups: pads are taken where the places' low bits (the
+        // bank group) stay spanned by the bits left to the threads.
+        std::vector<char> used(T, 0);
+        for (int b : bits) used[b] = 1;
+        auto bank = [&](int b) { return (uint32_t)swz((int)map.vec[b]) & 7u; };
+        auto rank_without = [&](int skip) {
+            uint32_t basis[3] = {0, 0, 0};
+            int r = 0;
+            for (int b = 0; b < T; ++b) {
+                if (used[b] || b == skip) continue;
+                uint32_t v = bank(b);
+                for (int k = 2; k >= 0 && v; --k) {
+                    if (!(v >> k & 1)) continue;
+                    if (!basis[k]) {
+                        basis[k] = v;
+                        ++r;
+                        break;
+                    }
+                    v ^= basis[k];
+                }
+            }
+            return r;
+        };
+        while ((int)bits.size() < maxr) {
+            int best = -1, best_rank = -1;
+            for (int b = T - 1; b >= 0; --b) {
+                if (used[b]) continue;
+                const int r = rank_without(b);
+                if (r > best_rank) best = b, best_rank = r;
+            }
+            used[best] = 1;
+            bits.push_back(best);
+        }
+        for (int k = 0; k < 4; ++k) {
+            const bool sel = k >= maxr;
+            rd.reg[k] = place(sel ? 1u << T : map.vec[bits[k]]);
+            rd.gpos[k] = sel ? 0ull : 1ull << global_pos(bits[k], h);
+        }
+        // thread-index bits: three that span the bank groups first
+        std::vector<int> lanes, rest;
+        uint32_t basis[3] = {0, 0, 0};
+        for (int b = 0; b < T; ++b) {
+            if (used[b]) continue;
+            uint32_t v = bank(b);
+            bool indep = false;
+            for (int k = 2; k >= 0 && v; --k) {
+                if (!(v >> k & 1)) continue;
+                if (!basis[k]) {
+                    basis[k] = v;
+                    indep = true;
+                    break;
+                }
+                v ^= basis[k];
+            }
+            (indep ? lanes : rest).push_back(b);
+        }
+        lanes.insert(lanes.end(), rest.begin(), rest.end());
+        rd.nlane = (int)lanes.size();
+        for (int j = 0; j < rd.nlane; ++j)
+            rd.lane[j] = place(map.vec[lanes[j]]) << 4 | (uint32_t)lanes[j];
+        rd.base = place(map.base);
+        rd.ncst = (int)map.cst.size();
+        for (int j = 0; j < rd.ncst; ++j) {
+            rd.cst_bit[j] = map.cst[j].first;
+            rd.cst_vec[j] = place(map.cst[j].second);
+        }
+        rd.slots = (int)slot_runs.size() << 8;
+        auto put = [&](const void *src, size_t doubles) {
+            const size_t o = p.data.size();
+            p.data.resize(o + doubles, 0.0);
+            if (src) memcpy(p.data.data() + o, src, doubles * sizeof(double));
+        };
+        for (size_t k = 0; k < ops.size(); ++k) {
+            const GateOp &g = gops[ops[k]];
+            if (type == RT_RUN) {
+                const int run = op_run[ops[k]];
+                (bwd ? p.runs[run].coef_b : p.runs[run].coef_f) = (int64_t)p.data.size();
+                put(nullptr, 8);
+                if (bwd && p.runs[run].ntiles > 0) {
+                    rd.slots |= 1 << k;
+                    slot_runs.push_back(run);
+                }
+            } else if (type == RT_DIAG) {
+                AdjDiagOp d{};
+                for (int q = 0; q < g.nfix; ++q) d.fix |= 1ull << g.fix[q];
+                d.npat = g.npat;
+                d.pb0 = g.npat > 0 ? g.pat[0] : 0;
+                d.pb1 = g.npat > 1 ? g.pat[1] : 0;
+                memcpy(d.ph, g.m, sizeof(d.ph));
+                put(&d, sizeof(d) / sizeof(double));
+            } else if (type == RT_CTRL) {
+                AdjCtrlOp c{};
+                c.is_x = g.type == OP_PERM1;
+                for (int q = 0; q < g.nctrl; ++q) {
+                    const int lb = local(g.ctrl[q]);
+                    const auto it = std::find(bits.begin(), bits.end(), lb);
+                    if (lb >= 0 && it != bits.end()) c.cm |= 1 << (int)(it - bits.begin());
+                    else c.gmask |= 1ull << g.ctrl[q];
+                }
+                memcpy(c.m, g.m, sizeof(c.m));
+                put(&c, sizeof(c) / sizeof(double));
+            } else {
+                put(g.m, 32);
+            }
+        }
+        rd.nrun = type == RT_RUN ? (int)ops.size() : 0;
+        rd.ndiag = type == RT_DIAG ? (int)ops.size() : 0;
+        p.rounds.push_back(rd);
+    };
+    std::vector<int> left(gates);
+    while (!left.empty()) {
+        std::vector<int> next, runs, diags, other;
+        std::vector<int> run_bits;
+        uint64_t blk = 0;
+        // permutations move into the map; the first free ops of each kind are found
+        for (int i : left) {
+            const GateOp &g = gops[i];
+            const uint64_t b = op_bits(g);
+            const bool free = (b & blk) == 0;
+            if (free && linear_perm(g)) {
+                if (g.type == OP_SWAP) {
+                    std::swap(map.vec[local(g.b0)], map.vec[local(g.b1)]);
+                    continue;
+                }
+                const uint32_t vt = map.vec[local(g.t)];
+                if (g.nctrl == 0) {
+                    map.base ^= vt;
+                    continue;
+                }
+                const int lc = local(g.ctrl[0]);
+                if (lc >= 0) {
+                    map.vec[lc] ^= vt;
+                    continue;
+                }
+                auto it = std::find_if(map.cst.begin(), map.cst.end(),
+                                       [&](const auto &c) { return c.first == g.ctrl[0]; });
+                if (it != map.cst.end()) {
+                    it->second ^= vt;
+                    continue;
+                }
+                if ((int)map.cst.size() < kMaxCst) {
+                    map.cst.push_back({g.ctrl[0], vt});
+                    continue;
+                }
+            }
+            if (free) {
+                if (op_run[i] >= 0) {
+                    if ((int)runs.size() < maxr) {
+                        runs.push_back(i);
+                        run_bits.push_back(local(g.t));
+                    }
+                } else if (g.type == OP_DIAG) {
+                    if ((int)diags.size() < kDiagsPerRound) diags.push_back(i);
+                } else {
+                    other.push_back(i);
+                }
+            }
+            next.push_back(i);
+            blk |= b;
+        }
+        left = std::move(next);
+        auto done = [&](const std::vector<int> &ops) {
+            for (int i : ops) left.erase(std::find(left.begin(), left.end(), i));
+        };
+        if (left.empty()) break;
+        // full rounds of runs first; with fewer, diagonal gates may free more of them
+        if ((int)runs.size() == maxr || (!runs.empty() && diags.empty())) {
+            emit(RT_RUN, run_bits, runs);
+            done(runs);
+        } else if (!diags.empty()) {
+            emit(RT_DIAG, {}, diags);
+            done(diags);
+        } else {
+            const GateOp &g = gops[other[0]];
+            if (g.type == OP_M2) emit(RT_M2, {local(g.b0), local(g.b1)}, {other[0]});
+            else emit(RT_CTRL, {local(g.t)}, {other[0]});
+            done({other[0]});
+        }
+    }
+    close_chunk();
+}
+
+static int push_map(AdjProgram &p, const PlanMap &map, int T) {
+    AdjMap am{};
+    for (int b = 0; b < T; ++b) am.vec[b] = place(map.vec[b]);
+    am.base = place(map.base);
+    am.ncst = (int)map.cst.size();
+    for (int j = 0; j < am.ncst; ++j) {
+        am.cst_bit[j] = map.cst[j].first;
+        am.cst_vec[j] = place(map.cst[j].second);
+    }
+    p.maps.push_back(am);
+    return (int)p.maps.size() - 1;
 }
 
 static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProgram &p,
@@ -840,9 +1268,6 @@ static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProg
         for (auto &a : ra) any = any || a.param >= 0;
         p.atoms.insert(p.atoms.end(), ra.begin(), ra.end());
         r.atom_end = (int32_t)p.atoms.size();
-        r.coef_f = (int64_t)p.coef.size();
-        r.coef_b = r.coef_f + 8;
-        p.coef.resize(p.coef.size() + 16, 0.0);
         r.part = -1;
         r.ntiles = any ? 1 << (n - T) : 0;
         p.runs.push_back(r);
@@ -855,6 +1280,8 @@ static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProg
         back.push_back(op_run[k] >= 0 ? gops[k] : inverse_op(gops[k]));
         back_run.push_back(op_run[k]);
     }
+    // (a small circuit's sweep back starts from the layout its way forward ended in)
+    PlanMap small_map(T);
     for (int dir = 0; dir < 2; ++dir) {
         const auto &go = dir ? back : gops;
         const auto &gr = dir ? back_run : op_run;
@@ -862,41 +1289,59 @@ static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProg
             if (!st.fused) return false;
             AdjPass ap{};
             ap.h = st.pass.h;
-            ap.round_begin = (int)p.rounds.size();
+            ap.chunk_begin = (int)p.chunks.size();
             ap.ntiles = 1 << (n - T);
             ap.part = p.npart;
             std::vector<int> slots;
-            adj_encode_pass(st.pass, go, gr, dir == 1, T, p, slots);
-            ap.nrounds = (int)p.rounds.size() - ap.round_begin;
+            PlanMap own(T);
+            PlanMap &map = n == T ? small_map : own;
+            adj_encode_pass(st.pass.gates, go, gr, dir == 1, T, st.pass.h, map, p, slots);
+            if (n != T) ap.map = push_map(p, map, T);
+            ap.nchunks = (int)p.chunks.size() - ap.chunk_begin;
             for (int r : slots) {
                 p.runs[r].part = p.npart;
                 p.npart += 3ll * ap.ntiles;
             }
             (dir ? bpass : fpass).push_back(ap);
         }
+        if (dir == 0 && n == T) in.map = push_map(p, small_map, T);
     }
     // the Pauli sum, by X mask in order of first appearance
     std::vector<char> taken(sp.nterms, 0);
     in.group_begin = (int)p.groups.size();
+    in.term_begin = (int)p.terms.size();
     for (int t = 0; t < sp.nterms; ++t) {
         if (taken[t]) continue;
-        AdjGroup gr{sp.terms[t].xmask, (int)p.terms.size(), 0};
+        AdjGroup gr{(uint32_t)sp.terms[t].xmask, (int)p.terms.size(), 0, 0, 0, 1};
+        if (n == T)
+            for (int b = 0; b < n; ++b)
+                if (gr.x >> b & 1) gr.vx ^= p.maps[in.map].vec[b];
         for (int u = t; u < sp.nterms; ++u) {
             const lq_pauli_term &pt = sp.terms[u];
-            if (taken[u] || pt.xmask != gr.x) continue;
+            if (taken[u] || pt.xmask != sp.terms[t].xmask) continue;
             if (!std::isfinite(pt.coefficient)) return false;
             taken[u] = 1;
             int k = pt.ny & 3;
             if (sp.yconv == LQ_Y_TEXTBOOK) k = (4 - k) & 3;
             const double a = k == 0 ? 1.0 : k == 2 ? -1.0 : 0.0;
             const double b = k == 1 ? -1.0 : k == 3 ? 1.0 : 0.0;
-            p.terms.push_back(AdjTerm{pt.zmask, pt.coefficient * a, pt.coefficient * b});
+            AdjTerm tm{pt.coefficient * a, pt.coefficient * b, (uint32_t)pt.zmask, 0, 0, 0};
+            tm.p = (uint8_t)((pt.zmask >> 8) & 7);
+            for (int q = 0; q < 8; ++q)
+                tm.flips |= (uint8_t)((__builtin_popcount(q & tm.p) & 1) << q);
+            if (k & 1) gr.odd = 1;
+            if (tm.p) gr.flat = 0;
+            p.terms.push_back(tm);
             ++gr.nterms;
         }
+        if (gr.x == 0)
+            std::stable_sort(p.terms.begin() + gr.term_begin, p.terms.end(),
+                             [](const AdjTerm &u, const AdjTerm &v) { return u.p < v.p; });
         p.groups.push_back(gr);
     }
+    in.nterms = (int)p.terms.size() - in.term_begin;
     in.ngroups = (int)p.groups.size() - in.group_begin;
-    return p.coef.size() < (size_t)1 << 30 && p.ops.size() < (size_t)1 << 30;
+    return p.data.size() < (size_t)1 << 30;
 }
 
 std::shared_ptr<AdjProgram> adj_plan(const std::vector<AdjSpec> &specs, int tile_bits,
@@ -928,8 +1373,8 @@ std::shared_ptr<AdjProgram> adj_plan(const std::vector<AdjSpec> &specs, int tile
             ++p.nsmall;
             p.small_T = std::max(p.small_T, in.n);
             if (fp[k].size() > 1 || bp[k].size() > 1) return nullptr;
-            if (!fp[k].empty()) in.f_round = fp[k][0].round_begin, in.f_nrounds = fp[k][0].nrounds;
-            if (!bp[k].empty()) in.b_round = bp[k][0].round_begin, in.b_nrounds = bp[k][0].nrounds;
+            if (!fp[k].empty()) in.f_chunk = fp[k][0].chunk_begin, in.f_nchunks = fp[k][0].nchunks;
+            if (!bp[k].empty()) in.b_chunk = bp[k][0].chunk_begin, in.b_nchunks = bp[k][0].nchunks;
             in.neparts = 1;
         } else {
             if (fp[k].empty()) return nullptr;  // no gate at all
@@ -994,16 +1439,17 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
         return o;
     };
     const size_t o_insts = take(p.insts.size() * sizeof(AdjInst));
-    const size_t o_rounds = take(p.rounds.size() * sizeof(FusedRound));
-    const size_t o_ops = take(p.ops.size() * sizeof(PassOp));
+    const size_t o_rounds = take(p.rounds.size() * sizeof(AdjRound));
+    const size_t o_maps = take(p.maps.size() * sizeof(AdjMap));
     const size_t o_atoms = take(p.atoms.size() * sizeof(AdjAtom));
     const size_t o_runs = take(p.runs.size() * sizeof(AdjRun));
     const size_t o_groups = take(p.groups.size() * sizeof(AdjGroup));
     const size_t o_terms = take(p.terms.size() * sizeof(AdjTerm));
     const size_t o_passes = take(p.passes.size() * sizeof(AdjPass));
+    const size_t o_chunks = take(p.chunks.size() * sizeof(AdjChunk));
     const size_t o_hlist = take(p.h_list.size() * sizeof(int32_t));
     const size_t o_hchunk = take(p.h_chunk.size() * sizeof(int64_t));
-    const size_t o_coef = take(p.coef.size() * sizeof(double));
+    const size_t o_data = take(p.data.size() * sizeof(double));
     const size_t upload = off;
     const size_t o_wts = take(p.atoms.size() * 3 * sizeof(double));
     const size_t o_part = take((size_t)p.npart * sizeof(double));
@@ -1038,32 +1484,39 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
     };
     put(o_insts, p.insts);
     put(o_rounds, p.rounds);
-    put(o_ops, p.ops);
+    put(o_maps, p.maps);
     put(o_atoms, p.atoms);
     put(o_runs, p.runs);
     put(o_groups, p.groups);
     put(o_terms, p.terms);
     put(o_passes, p.passes);
+    put(o_chunks, p.chunks);
     put(o_hlist, p.h_list);
     put(o_hchunk, p.h_chunk);
-    put(o_coef, p.coef);
+    put(o_data, p.data);
     char *b = (char *)p.blob;
     p.d_insts = (AdjInst *)(b + o_insts);
-    p.d_rounds = (FusedRound *)(b + o_rounds);
-    p.d_ops = (PassOp *)(b + o_ops);
+    p.d_rounds = (AdjRound *)(b + o_rounds);
+    p.d_maps = (AdjMap *)(b + o_maps);
     p.d_atoms = (AdjAtom *)(b + o_atoms);
     p.d_runs = (AdjRun *)(b + o_runs);
     p.d_groups = (AdjGroup *)(b + o_groups);
     p.d_terms = (AdjTerm *)(b + o_terms);
     p.d_passes = (AdjPass *)(b + o_passes);
+    p.d_chunks = (AdjChunk *)(b + o_chunks);
     p.d_hlist = (int32_t *)(b + o_hlist);
     p.d_hchunk = (int64_t *)(b + o_hchunk);
-    p.d_coef = (double *)(b + o_coef);
+    p.d_data = (double *)(b + o_data);
     p.d_wts = (double *)(b + o_wts);
     p.d_part = (double *)(b + o_part);
     p.d_epart = (double *)(b + o_epart);
     p.d_theta = (double *)(b + o_theta);
     p.d_out = (double *)(b + o_out);
+    if (p.nsmall && p.nsmall < p.ninst) {
+        LQ_CUDA_TRY(cudaStreamCreateWithFlags(&p.side, cudaStreamNonBlocking));
+        LQ_CUDA_TRY(cudaEventCreateWithFlags(&p.fork, cudaEventDisableTiming));
+        LQ_CUDA_TRY(cudaEventCreateWithFlags(&p.join, cudaEventDisableTiming));
+    }
     LQ_CUDA_TRY(cudaMemcpyAsync(p.blob, h.data(), upload, cudaMemcpyHostToDevice, st));
     LQ_CUDA_TRY(cudaFuncSetAttribute(k_adj_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)adj_small_smem(kAdjSmallMax)));
@@ -1083,12 +1536,21 @@ int adj_enqueue(AdjProgram &p, cudaStream_t st, const double *theta_and_shift, d
     // a parameter that no gate uses has gradient 0
     if (p.nparams) LQ_CUDA_TRY(cudaMemsetAsync(grad, 0, sizeof(double) * p.nparams, st));
     const int nruns = (int)p.runs.size();
+    const AdjProg pg{p.d_rounds, p.d_data, p.d_chunks, p.d_maps};
     if (nruns)
         k_adj_coef<<<(nruns + 127) / 128, 128, 0, st>>>(p.d_runs, nruns, p.d_atoms, p.d_theta,
-                                                       p.d_coef, p.d_wts);
-    if (p.nsmall)
-        k_adj_small<<<p.nsmall, kAdjSmallThreads, adj_small_smem(p.small_T), st>>>(
-            p.d_insts, p.d_rounds, p.d_ops, p.d_coef, p.d_groups, p.d_terms, p.d_part, p.d_epart);
+                                                       p.d_data, p.d_wts);
+    if (p.nsmall) {
+        cudaStream_t sm = st;
+        if (p.side) {
+            sm = p.side;
+            LQ_CUDA_TRY(cudaEventRecord(p.fork, st));
+            LQ_CUDA_TRY(cudaStreamWaitEvent(sm, p.fork, 0));
+        }
+        k_adj_small<<<p.nsmall, kAdjSmallThreads, adj_small_smem(p.small_T), sm>>>(
+            p.d_insts, pg, p.d_groups, p.d_terms, p.d_part, p.d_epart);
+        if (p.side) LQ_CUDA_TRY(cudaEventRecord(p.join, sm));
+    }
     double2 *psi = p.psi, *lam = p.lam;
     for (const AdjWave &w : p.waves) {
         for (size_t l = 0; l < w.f.size(); ++l) {
@@ -1096,8 +1558,7 @@ int adj_enqueue(AdjProgram &p, cudaStream_t st, const double *theta_and_shift, d
             const AdjPass &last = p.passes[b - 1];
             k_adj_pass<false><<<last.tile_begin + last.ntiles, kAdjThreads,
                                 adj_pass_smem(p.T, false), st>>>(
-                p.d_insts, p.d_passes + a, b - a, p.d_rounds, p.d_ops, p.d_coef, psi, lam,
-                p.d_part, p.T, l == 0);
+                p.d_insts, p.d_passes + a, b - a, pg, psi, lam, p.d_part, p.T, l == 0);
         }
         k_adj_h<<<(unsigned)w.h_blocks, 256, 0, st>>>(p.d_insts, p.d_hlist + w.h_begin, w.h_count,
                                                      p.d_hchunk + w.h_begin, p.d_groups, p.d_terms,
@@ -1106,10 +1567,11 @@ int adj_enqueue(AdjProgram &p, cudaStream_t st, const double *theta_and_shift, d
             const auto [a, b] = w.b[l];
             const AdjPass &last = p.passes[b - 1];
             k_adj_pass<true><<<last.tile_begin + last.ntiles, kAdjThreads, adj_pass_smem(p.T, true),
-                               st>>>(p.d_insts, p.d_passes + a, b - a, p.d_rounds, p.d_ops,
-                                     p.d_coef, psi, lam, p.d_part, p.T, l + 1 == w.b.size());
+                               st>>>(p.d_insts, p.d_passes + a, b - a, pg, psi, lam, p.d_part, p.T,
+                                     l + 1 == w.b.size());
         }
     }
+    if (p.nsmall && p.side) LQ_CUDA_TRY(cudaStreamWaitEvent(st, p.join, 0));
     const int warps = nruns + p.ninst;
     k_adj_final<<<(warps + 3) / 4, 128, 0, st>>>(p.d_runs, nruns, p.d_atoms, p.d_wts, p.d_part,
                                                 p.d_insts, p.ninst, p.d_epart,

@@ -908,7 +908,6 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
         int code = e == cudaErrorMemoryAllocation ? LQ_ERR_OOM : LQ_ERR_CUDA;
         if (s->d) cudaFree(s->d);
         if (s->d_red) cudaFree(s->d_red);
-        if (s->h_red) cudaFreeHost(s->h_red);
         if (s->d_flag) cudaFree(s->d_flag);
         if (s->stream) cudaStreamDestroy(s->stream);
         delete s;
@@ -922,8 +921,6 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
     if ((e = cudaMalloc(&s->d_red, sizeof(double) * kRedBlocks * 2 * kMaxTermsPerPass)) !=
         cudaSuccess)
         return fail(e, "cudaMalloc(reduction scratch)");
-    if ((e = cudaMallocHost(&s->h_red, sizeof(double) * 64)) != cudaSuccess)
-        return fail(e, "cudaMallocHost");
     if ((e = cudaMalloc(&s->d_flag, sizeof(unsigned) * 4)) != cudaSuccess)
         return fail(e, "cudaMalloc(flags)");
     if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(unsigned) * 4, s->stream)) != cudaSuccess)
@@ -951,7 +948,6 @@ int lq_state_destroy(lq_state *s) {
         g_alloc_in_use -= s->bytes;
     }
     if (s->d_red) cudaFree(s->d_red);
-    if (s->h_red) cudaFreeHost(s->h_red);
     if (s->d_flag) cudaFree(s->d_flag);
     if (s->d_prog) cudaFree(s->d_prog);
     free_plan_cache(s);
