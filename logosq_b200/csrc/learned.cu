@@ -20,104 +20,157 @@
 namespace lq {
 
 // ---------------------------------------------------------------------------
-// FP32 GEMM: C[M x N] = op(A) op(B) (+ bias[N]) (+ C if accumulate), with an
-// optional GELU epilogue that also stores the pre-activation Z.
-//   op(A) = A (M x K, lda) or A^T (A is K x M)
-//   op(B) = B (K x N, ldb) or B^T (B is N x K)
-// 64 x 64 block tile, 16 x 16 threads, 4 x 4 outputs per thread, K step 16.
+// FP32 GEMM: C[M x N] = op(A) op(B), the network's only contraction.
+//   op(A) = A (M x K, lda) or A^T (A is K x M);  op(B) likewise
+// Epilogues: + bias, then GELU with the pre-activation kept in Z; or times the GELU
+// derivative at Z (the next layer's gradient through its activation); row sums of
+// op(A) (the bias gradient, whose op(A) is dY^T).
+//
+// A batch of 256 through 256-wide layers is 17 MFMA a product: the chip would do it
+// in under a microsecond, so latency counts and not arithmetic.  32 x 32 output
+// tiles (64 blocks for 256 x 256, where 64 x 64 tiles gave 16) of 256 threads, four groups of
+// 64 that each take a quarter of every 32-deep K step on 4 x 4 outputs per thread and
+// are added at the end; the next K step is loaded into registers meanwhile.  The two
+// products of a backward layer, dW and dX, share one launch.  (Measured per product:
+// 31-47 us with 64 x 64 tiles of one group.)
 // ---------------------------------------------------------------------------
-constexpr int GB = 64, GK = 16;
+constexpr int GB = 32, GK = 32, GP = GB + 4;
 
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float *__restrict__ A,
-                                              int lda, const float *__restrict__ B, int ldb,
-                                              float *__restrict__ Cm, int ldc,
-                                              const float *__restrict__ bias, int accumulate,
-                                              int gelu, float *__restrict__ Z) {
-    __shared__ float As[GK][GB + 4];
-    __shared__ float Bs[GK][GB + 4];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int i = threadIdx.x; i < GK * GB; i += 256) {
-            const int kk = i / GB, mm = i % GB;
-            const int gm = m0 + mm, gk = k0 + kk;
-            float va = 0.f;
-            if (gm < M && gk < K) va = TA ? A[(size_t)gk * lda + gm] : A[(size_t)gm * lda + gk];
-            As[kk][mm] = va;
-            const int gn = n0 + mm;
-            float vb = 0.f;
-            if (gn < N && gk < K) vb = TB ? B[(size_t)gn * ldb + gk] : B[(size_t)gk * ldb + gn];
-            Bs[kk][mm] = vb;
+enum GemmEpilogue { EP_NONE = 0, EP_BIAS = 1, EP_BIAS_GELU = 2, EP_GELU_BWD = 3 };
+
+struct GemmJob {
+    int M, N, K;
+    const float *A;
+    int lda, ta;
+    const float *B;
+    int ldb, tb;
+    float *C;
+    int ldc;
+    int ep;
+    const float *bias;
+    float *Z;        // written (EP_BIAS_GELU) or read (EP_GELU_BWD), as C
+    float *row_sum;  // sums of op(A)'s rows, or null
+};
+
+// GELU'(z) = Phi(z) + z phi(z)
+__device__ __forceinline__ float gelu_slope(float z) {
+    const float cdf = 0.5f * (1.f + erff(z * 0.70710678118654752f));
+    const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
+    return cdf + z * pdf;
+}
+
+__global__ void __launch_bounds__(256)
+    k_gemm(const __grid_constant__ GemmJob j0, const __grid_constant__ GemmJob j1, int blocks0) {
+    __shared__ __align__(16) float sm[2][2][GK][GP];  // [buffer][A, B]
+    __shared__ float s_row[4][GB];
+    const bool second = (int)blockIdx.x >= blocks0;
+    const GemmJob &j = second ? j1 : j0;
+    const int tid = threadIdx.x, group = tid >> 6, tx = tid & 7, ty = (tid >> 3) & 7;
+    const int nt = (j.N + GB - 1) / GB, blk = (int)blockIdx.x - (second ? blocks0 : 0);
+    const int m0 = blk / nt * GB, n0 = blk % nt * GB;
+    // staging: four elements per thread and operand; consecutive threads run along the
+    // contiguous index of the operand
+    const int i = tid & 31, o = tid >> 5;
+    auto fetch = [&](int k0, float (&ra)[4], float (&rb)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int u = o + 8 * q;
+            const int am = m0 + (j.ta ? i : u), ak = k0 + (j.ta ? u : i);
+            ra[q] = am < j.M && ak < j.K
+                        ? (j.ta ? j.A[(size_t)ak * j.lda + am] : j.A[(size_t)am * j.lda + ak])
+                        : 0.f;
+            const int bn = n0 + (j.tb ? u : i), bk = k0 + (j.tb ? i : u);
+            rb[q] = bn < j.N && bk < j.K
+                        ? (j.tb ? j.B[(size_t)bn * j.ldb + bk] : j.B[(size_t)bk * j.ldb + bn])
+                        : 0.f;
         }
-        __syncthreads();
+    };
+    auto stash = [&](int buf, const float (&ra)[4], const float (&rb)[4]) {
 #pragma unroll
-        for (int kk = 0; kk < GK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int q = 0; q < 4; ++q) {
+            const int u = o + 8 * q;
+            sm[buf][0][j.ta ? u : i][j.ta ? i : u] = ra[q];
+            sm[buf][1][j.tb ? i : u][j.tb ? u : i] = rb[q];
         }
-        __syncthreads();
-    }
+    };
+    float acc[4][4] = {}, rsum[4] = {};
+    float ra[4], rb[4];
+    fetch(0, ra, rb);
+    stash(0, ra, rb);
+    __syncthreads();
+    int buf = 0;
+    for (int k0 = 0; k0 < j.K; k0 += GK) {
+        const bool more = k0 + GK < j.K;
+        if (more) fetch(k0 + GK, ra, rb);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
+        for (int kk = 0; kk < GK / 4; ++kk) {
+            const int k = group * (GK / 4) + kk;
+            const float4 a4 = *(const float4 *)&sm[buf][0][k][ty * 4];
+            const float4 b4 = *(const float4 *)&sm[buf][1][k][tx * 4];
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N) continue;
-            float v = acc[i][j];
-            if (bias) v += bias[gn];
-            if (accumulate) v += Cm[(size_t)gm * ldc + gn];
-            if (gelu) {
-                Z[(size_t)gm * ldc + gn] = v;
-                v = 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
+            for (int p = 0; p < 4; ++p) {
+                rsum[p] += a[p];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[p][q] = fmaf(a[p], b[q], acc[p][q]);
             }
-            Cm[(size_t)gm * ldc + gn] = v;
         }
+        if (more) stash(buf ^ 1, ra, rb);  // (last read before the previous barrier)
+        __syncthreads();
+        buf ^= 1;
     }
+    // add the four groups
+    float(*red)[GB][GB] = (float(*)[GB][GB])sm;
+    static_assert(sizeof(float) * 4 * GB * GB <= sizeof(sm), "the groups' sums fit the stages");
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+        *(float4 *)&red[group][ty * 4 + p][tx * 4] =
+            make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+    if (tx == 0)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) s_row[group][ty * 4 + p] = rsum[p];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int r = o + 8 * q, gm = m0 + r, gn = n0 + i;
+        if (gm >= j.M || gn >= j.N) continue;
+        float v = (red[0][r][i] + red[1][r][i]) + (red[2][r][i] + red[3][r][i]);
+        const size_t at = (size_t)gm * j.ldc + gn;
+        if (j.ep == EP_BIAS || j.ep == EP_BIAS_GELU) v += j.bias[gn];
+        if (j.ep == EP_BIAS_GELU) {
+            j.Z[at] = v;
+            v = 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
+        } else if (j.ep == EP_GELU_BWD) {
+            v *= gelu_slope(j.Z[at]);
+        }
+        j.C[at] = v;
+    }
+    if (j.row_sum && n0 == 0 && tid < GB && m0 + tid < j.M)
+        j.row_sum[m0 + tid] =
+            (s_row[0][tid] + s_row[1][tid]) + (s_row[2][tid] + s_row[3][tid]);
 }
 
-static void sgemm(cudaStream_t st, bool ta, bool tb, int M, int N, int K, const float *A, int lda,
-                  const float *B, int ldb, float *Cm, int ldc, const float *bias, bool acc,
-                  bool gelu, float *Z) {
-    dim3 grid((N + GB - 1) / GB, (M + GB - 1) / GB);
-    if (!ta && !tb)
-        k_sgemm<false, false><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, Cm, ldc, bias, acc,
-                                                    gelu, Z);
-    else if (!ta && tb)
-        k_sgemm<false, true><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, Cm, ldc, bias, acc,
-                                                   gelu, Z);
-    else if (ta && !tb)
-        k_sgemm<true, false><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, Cm, ldc, bias, acc,
-                                                   gelu, Z);
-    else
-        k_sgemm<true, true><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, Cm, ldc, bias, acc,
-                                                  gelu, Z);
+static int gemm_blocks(const GemmJob &j) {
+    return ((j.M + GB - 1) / GB) * ((j.N + GB - 1) / GB);
 }
 
-// dZ = dH * gelu'(Z)
-__global__ void k_gelu_bwd(const float *__restrict__ Z, float *__restrict__ dH, int count) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float z = Z[i];
-        const float cdf = 0.5f * (1.f + erff(z * 0.70710678118654752f));
-        const float pdf = 0.39894228040143268f * expf(-0.5f * z * z);
-        dH[i] *= cdf + z * pdf;
-    }
+static void gemm(cudaStream_t st, const GemmJob &j) {
+    const int b = gemm_blocks(j);
+    k_gemm<<<b, 256, 0, st>>>(j, j, b);
+}
+
+static void gemm2(cudaStream_t st, const GemmJob &a, const GemmJob &b) {
+    const int n = gemm_blocks(a);
+    k_gemm<<<n + gemm_blocks(b), 256, 0, st>>>(a, b, n);
 }
 
 // Periodic angle loss: sum mask * (1 - cos(y - t)) / sum(mask); dY = mask sin(y - t) / sum(mask).
+// One partial sum per block (the caller adds them in order).
+constexpr int kLossBlocks = 148;
+
 __global__ void k_angle_loss(const float *__restrict__ Y, const float *__restrict__ T,
                              const float *__restrict__ Mk, float *__restrict__ dY, int count,
-                             float inv_norm, double *__restrict__ loss_acc) {
+                             float inv_norm, double *__restrict__ loss_part) {
     __shared__ double sh[256];
     double acc = 0.0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
@@ -132,16 +185,7 @@ __global__ void k_angle_loss(const float *__restrict__ Y, const float *__restric
         if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
         __syncthreads();
     }
-    if (threadIdx.x == 0) atomicAdd(loss_acc, sh[0] * inv_norm);
-}
-
-// db[n] = sum_m dY[m][n]
-__global__ void k_bias_grad(const float *__restrict__ dY, float *__restrict__ db, int M, int N) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int m = 0; m < M; ++m) s += dY[(size_t)m * N + n];
-    db[n] = s;
+    if (threadIdx.x == 0) loss_part[blockIdx.x] = sh[0] * inv_norm;
 }
 
 __global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
@@ -306,8 +350,9 @@ static int mlp_forward_dev(lq_mlp *net, int batch) {
         const int K = net->dims[l], Nn = net->dims[l + 1];
         const bool last = l == L - 1;
         // H[l+1] = H[l] (batch x K) . W^T (W stored out x in) + b
-        sgemm(net->stream, false, true, batch, Nn, K, net->H[l], K, net->p + net->woff[l], K,
-              net->H[l + 1], Nn, net->p + net->boff[l], false, !last, net->Z[l + 1]);
+        gemm(net->stream,
+             GemmJob{batch, Nn, K, net->H[l], K, 0, net->p + net->woff[l], K, 1, net->H[l + 1], Nn,
+                     last ? EP_BIAS : EP_BIAS_GELU, net->p + net->boff[l], net->Z[l + 1], nullptr});
     }
     LQ_CUDA_TRY(cudaGetLastError());
     return LQ_OK;
@@ -321,20 +366,18 @@ static int mlp_backward_dev(lq_mlp *net, int batch) {
     const int L = (int)net->dims.size() - 1;
     for (int l = L - 1; l >= 0; --l) {
         const int K = net->dims[l], Nn = net->dims[l + 1];
-        if (l < L - 1) {  // through the GELU of layer l's output
-            k_gelu_bwd<<<std::max(1, std::min(1184, (batch * Nn + 255) / 256)), 256, 0, st>>>(
-                net->Z[l + 1], dY, batch * Nn);
+        // dW (Nn x K) = dY^T (Nn x batch) . H[l] (batch x K), and db = dY's column sums
+        const GemmJob dw{Nn, K, batch, dY, Nn, 1, net->H[l], K, 0, net->g + net->woff[l], K,
+                         EP_NONE, nullptr, nullptr, net->g + net->boff[l]};
+        if (l == 0) {
+            gemm(st, dw);
+            break;
         }
-        // dW (Nn x K) = dY^T (Nn x batch) . H[l] (batch x K)
-        sgemm(st, true, false, Nn, K, batch, dY, Nn, net->H[l], K, net->g + net->woff[l], K,
-              nullptr, false, false, nullptr);
-        k_bias_grad<<<(Nn + 127) / 128, 128, 0, st>>>(dY, net->g + net->boff[l], batch, Nn);
-        if (l > 0) {
-            // dX (batch x K) = dY (batch x Nn) . W (Nn x K)
-            sgemm(st, false, false, batch, K, Nn, dY, Nn, net->p + net->woff[l], K, dX, K,
-                  nullptr, false, false, nullptr);
-            std::swap(dY, dX);
-        }
+        // dX (batch x K) = dY (batch x Nn) . W (Nn x K), through the GELU of layer l-1
+        gemm2(st, dw,
+              GemmJob{batch, K, Nn, dY, Nn, 0, net->p + net->woff[l], K, 0, dX, K, EP_GELU_BWD,
+                      nullptr, net->Z[l], nullptr});
+        std::swap(dY, dX);
     }
     LQ_CUDA_TRY(cudaGetLastError());
     return LQ_OK;
@@ -393,7 +436,7 @@ int lq_mlp_create(int in_dim, int hidden, int depth, int out_dim, uint64_t seed,
     if ((e = cudaMalloc(&net->g, off * 4))) return fail(e);
     if ((e = cudaMalloc(&net->m, off * 4))) return fail(e);
     if ((e = cudaMalloc(&net->v, off * 4))) return fail(e);
-    if ((e = cudaMalloc(&net->loss_d, sizeof(double)))) return fail(e);
+    if ((e = cudaMalloc(&net->loss_d, sizeof(double) * kLossBlocks))) return fail(e);
     if ((e = cudaMemcpy(net->p, init.data(), off * 4, cudaMemcpyHostToDevice))) return fail(e);
     if ((e = cudaMemset(net->m, 0, off * 4)) || (e = cudaMemset(net->v, 0, off * 4)) ||
         (e = cudaMemset(net->g, 0, off * 4)))
@@ -473,8 +516,14 @@ int lq_mlp_loss_grad(lq_mlp *net, const float *x, const float *target, const flo
     LQ_TRY(mlp_reserve(net, batch));
     cudaStream_t st = net->stream;
     const int O = net->out_dim;
-    double msum = 0.0;
-    for (int i = 0; i < batch * O; ++i) msum += mask[i];
+    // (eight chains: one alone is 40 us of additions for a batch of 256)
+    double ms[8] = {0.0}, msum = 0.0;
+    const int64_t count = (int64_t)batch * O;
+    int64_t mi = 0;
+    for (; mi + 8 <= count; mi += 8)
+        for (int k = 0; k < 8; ++k) ms[k] += mask[mi + k];
+    for (; mi < count; ++mi) msum += mask[mi];
+    for (int k = 0; k < 8; ++k) msum += ms[k];
     if (msum <= 0) return set_error(LQ_ERR_INVALID_ARG, "empty mask");
     LQ_CUDA_TRY(cudaMemcpyAsync(net->H[0], x, sizeof(float) * batch * net->in_dim,
                                 cudaMemcpyHostToDevice, st));
@@ -483,14 +532,16 @@ int lq_mlp_loss_grad(lq_mlp *net, const float *x, const float *target, const flo
     LQ_CUDA_TRY(cudaMemcpyAsync(net->mask, mask, sizeof(float) * batch * O,
                                 cudaMemcpyHostToDevice, st));
     LQ_TRY(mlp_forward_dev(net, batch));
-    LQ_CUDA_TRY(cudaMemsetAsync(net->loss_d, 0, sizeof(double), st));
-    k_angle_loss<<<std::max(1, std::min(148, (batch * O + 255) / 256)), 256, 0, st>>>(
+    const int lb = std::max(1, std::min(kLossBlocks, (batch * O + 255) / 256));
+    k_angle_loss<<<lb, 256, 0, st>>>(
         net->H.back(), net->target, net->mask, net->dA, batch * O, (float)(1.0 / msum),
         net->loss_d);
     LQ_TRY(mlp_backward_dev(net, batch));
-    double lv = 0.0;
-    LQ_CUDA_TRY(cudaMemcpyAsync(&lv, net->loss_d, sizeof(double), cudaMemcpyDeviceToHost, st));
+    double part[kLossBlocks], lv = 0.0;
+    LQ_CUDA_TRY(cudaMemcpyAsync(part, net->loss_d, sizeof(double) * lb, cudaMemcpyDeviceToHost,
+                                st));
     LQ_CUDA_TRY(cudaStreamSynchronize(st));
+    for (int k = 0; k < lb; ++k) lv += part[k];
     if (loss) *loss = lv;
     return LQ_OK;
 }
