@@ -8,8 +8,10 @@
 #include <cstdarg>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "lq_internal.h"
+#include "reduce.cuh"
 
 namespace lq {
 
@@ -57,6 +59,31 @@ int ensure_prog(lq_state *s, size_t bytes) {
     return LQ_OK;
 }
 
+int take_work(lq_state *s, size_t bytes, void **out) {
+    *out = nullptr;
+    if (bytes > kKeptWork) {
+        LQ_CUDA_TRY(cudaMallocAsync(out, bytes, s->stream));
+        return LQ_OK;
+    }
+    if (s->work_cap < bytes) {
+        if (s->d_work) {
+            LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
+            LQ_CUDA_TRY(cudaFree(s->d_work));
+            s->d_work = nullptr;
+            s->work_cap = 0;
+        }
+        LQ_CUDA_TRY(cudaMalloc(&s->d_work, bytes));
+        s->work_cap = bytes;
+    }
+    *out = s->d_work;
+    return LQ_OK;
+}
+
+int give_work(lq_state *s, void *p) {
+    if (p && p != s->d_work) LQ_CUDA_TRY(cudaFreeAsync(p, s->stream));
+    return LQ_OK;
+}
+
 // ---------------------------------------------------------------------------
 // Kernels
 // ---------------------------------------------------------------------------
@@ -97,29 +124,6 @@ template <>
 __device__ __forceinline__ double2 load_amp<float2>(const float2 *v, uint64_t i) {
     float2 a = v[i];
     return make_double2(a.x, a.y);
-}
-
-// Block-wide sum of NC doubles; result valid in thread 0.
-template <int NC>
-__device__ __forceinline__ void block_sum(double (&x)[NC], double *sh /* 32*NC */) {
-#pragma unroll
-    for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x[c] += __shfl_down_sync(0xffffffffu, x[c], o);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) sh[warp * NC + c] = x[c];
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            x[c] = lane < nw ? sh[lane * NC + c] : 0.0;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x[c] += __shfl_down_sync(0xffffffffu, x[c], o);
-        }
-    }
 }
 
 template <class A>
@@ -168,20 +172,6 @@ __global__ void k_final_sum(const double *partials, int nparts, double *out) {
     if (threadIdx.x == 0)
 #pragma unroll
         for (int c = 0; c < NC; ++c) out[c] = acc[c];
-}
-
-// State::normalize: divide by sqrt(norm_sqr) when the norm exceeds 1e-10.
-template <class A>
-__global__ void k_scale_by_norm(A *__restrict__ v, uint64_t N, const double *norm_sqr) {
-    const double norm = sqrt(*norm_sqr);
-    if (!(norm > 1e-10)) return;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < N;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        A a = v[i];
-        a.x = a.x / norm;
-        a.y = a.y / norm;
-        v[i] = a;
-    }
 }
 
 // v *= sqrt(target / current) (both squared norms, FP64, on the device).
@@ -339,55 +329,207 @@ __global__ void k_pauli_group(const A *__restrict__ v, int n, uint64_t xmask,
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
 }
 
-// Terms without X bits (one group, X mask 0), for states of 12 or more qubits,
-// launched with 256 threads.  A block takes 4096-amplitude chunks; thread tid
-// handles the 16 indices i = chunk | k << 8 | tid, k = 0..15.  A term's sign
-// (-1)^popcount(i & z) is the sign of the bits the thread keeps fixed (chunk
-// and tid) times (-1)^popcount(k & p), p = bits 8-11 of z.  The terms arrive
-// sorted by p (pbeg[p] .. pbeg[p+1]), so each thread folds all of them into 16
-// coefficients C[p], and one 16-point Walsh-Hadamard transform of C gives the
-// sum of signed coefficients for all 16 k: a few operations per amplitude
-// instead of a popcount and a select per term per amplitude.
+// ---------------------------------------------------------------------------
+// Pauli sums by windows.  A tile is the 2^T amplitudes of the index bits [0,4) and
+// [h, h+T-4), held in shared memory as complex128; every group whose X bits lie in
+// that window is evaluated from it, so the state is read once per window instead of
+// once per X mask (a 24-qubit chain: 3 reads instead of 24), and a state of at most
+// 2^12 amplitudes needs one launch for the whole sum.
+//
+// Reading the tile once per group would make shared memory the bound (two 16-byte loads
+// for 2-4 FP64 instructions: 0.90 ms for that chain).  So the groups are taken in
+// rounds: a round has four vectors v_0..v_3 (tile-local X masks, in reduced echelon
+// form), a thread holds the 16 amplitudes l0 + span(v), and every group whose mask lies
+// in that span is formed from registers.  A chain's X, XX and YY terms need a round for
+// every three bits; arbitrary masks need one for every four of them.  All index work is
+// linear over XOR: a term's sign splits into the bits outside the window (the tile), the
+// thread's and the element's, of which the last is a mask made on the host.
+// ---------------------------------------------------------------------------
+constexpr int kWinT = 12, kWinMinT = 9;
+constexpr int kWinStage = 8192;  // bytes of rounds, groups and terms staged at a time
+
+struct WinTerm {
+    uint64_t z;      // Z bits outside the window
+    double c;
+    uint32_t lz;     // Z bits in the window, tile-local
+    uint32_t mask;   // bit k: the sign at pair k of the group; without X: the parities of
+                     // lz with the four vectors (by which these terms arrive sorted)
+    uint32_t odd;    // an odd number of Y
+    uint32_t pad;
+};
+
+struct WinGroup {
+    int32_t d;       // its X mask as a sum of vectors, 1..15
+    int32_t odd;     // some term has an odd number of Y
+    int32_t term, nterms;
+};
+
+struct WinRound {
+    uint32_t vec[4];   // places of the vectors
+    uint32_t lane[8];  // tile bit of each thread-index bit
+    int32_t group, ngroups;
+    int32_t zterm, nz;  // terms without X
+};
+
+struct WinChunk {  // one stage: rounds, then groups, then terms
+    int32_t offset, bytes;  // in the program
+    int32_t nrounds, groups, terms;  // the latter two: byte offsets in the stage
+};
+
+struct WinDesc {
+    int32_t h, chunk, nchunks;
+    int32_t work;  // first work index of the window
+};
+static_assert(sizeof(WinTerm) % 16 == 0 && sizeof(WinGroup) % 16 == 0 && sizeof(WinRound) % 16 == 0,
+              "staged in 16 bytes");
+
+// Byte offset of a tile index: any three bits of different residues mod 3 spread eight
+// threads over the eight 16-byte bank groups.
+__host__ __device__ __forceinline__ uint32_t win_place(uint32_t l) {
+    return (l ^ (((l >> 3) ^ (l >> 6) ^ (l >> 9)) & 7u)) << 4;
+}
+__device__ __forceinline__ double win_sign(double x, uint32_t neg) {  // bit 0 counts
+    return __hiloint2double(__double2hiint(x) ^ (int)(neg << 31), __double2loint(x));
+}
+// Pair k of the group of mask d: element k with a zero inserted at d's top bit, and that
+// element plus d.
+__host__ __device__ constexpr int win_pair(int k, int d) {
+    const int hb = d >= 8 ? 3 : d >= 4 ? 2 : d >= 2 ? 1 : 0;
+    return ((k >> hb) << (hb + 1)) | (k & ((1 << hb) - 1));
+}
+// W = conj(a) b of the 8 pairs; the pair's other orientation doubles it (k_pauli_group).
+template <int D>
+__device__ __forceinline__ void win_pairs(const double2 (&a)[16], bool odd, double (&wr)[8],
+                                          double (&wi)[8]) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double2 x = a[win_pair(k, D)], y = a[win_pair(k, D) ^ D];
+        wr[k] = fma(x.x, y.x, x.y * y.y);
+    }
+    if (odd)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const double2 x = a[win_pair(k, D)], y = a[win_pair(k, D) ^ D];
+            wi[k] = fma(x.x, y.y, -(x.y * y.x));
+        }
+}
+
 template <class A>
 __global__ void __launch_bounds__(256, 2)
-    k_pauli_zfold(const A *__restrict__ v, int n, const TermCoef *__restrict__ tc, int nt,
-                  const int *__restrict__ pbeg, double *partials) {
-    extern __shared__ TermCoef s_tc[];
+    k_pauli_windows(const A *__restrict__ v, int n, int T, const WinDesc *__restrict__ wins,
+                    int nwins, const WinChunk *__restrict__ chunks,
+                    const unsigned char *__restrict__ program, int nwork,
+                    double *__restrict__ partials) {
+    extern __shared__ __align__(16) unsigned char win_smem[];
     __shared__ double sh[32];
-    __shared__ int s_pbeg[17];
-    for (int t = threadIdx.x; t < nt; t += blockDim.x) s_tc[t] = tc[t];
-    if (threadIdx.x < 17) s_pbeg[threadIdx.x] = pbeg[threadIdx.x];
-    __syncthreads();
+    unsigned char *stage = win_smem + ((size_t)16 << T);
+    const uint32_t tid = threadIdx.x;
+    const uint64_t N = 1ull << n;
+    uint32_t on[8];  // all ones where the thread-index bit is set
+#pragma unroll
+    for (int j = 0; j < 8; ++j) on[j] = 0u - ((tid >> j) & 1u);
     double acc[1] = {0.0};
-    const uint64_t nchunks = 1ull << (n - 12);
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint64_t fixed = (c << 12) | (uint64_t)threadIdx.x;
-        double pr[16];  // |a|^2 of the 16 amplitudes
+    int held = -1, wi = 0;  // chunk in the stage; window
+    for (int w = (int)blockIdx.x; w < nwork; w += (int)gridDim.x) {
+        while (wi + 1 < nwins && wins[wi + 1].work <= w) ++wi;
+        const WinDesc win = wins[wi];
+        const int tile = w - win.work, h = win.h;
+        const uint64_t c2 = n > T ? (uint64_t)(tile & ((1 << (h - 4)) - 1)) : 0;
+        const uint64_t c4 = n > T ? (uint64_t)(tile >> (h - 4)) : 0;
+        const uint64_t tb = (c2 << 4) | (c4 << (h + T - 4));
+        __syncthreads();  // the previous tile has been read
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
-            const double2 a = load_amp(v, fixed | ((uint64_t)k << 8));
-            pr[k] = a.x * a.x + a.y * a.y;
+            const uint32_t l = tid | (uint32_t)k << (T - 4);
+            const uint64_t i = tb | (uint64_t)(l & 15u) | ((uint64_t)(l >> 4) << h);
+            *(double2 *)(win_smem + win_place(l)) = i < N ? load_amp(v, i) : make_double2(0.0, 0.0);
         }
-        double C[16];
+        for (int ci = win.chunk; ci < win.chunk + win.nchunks; ++ci) {
+            const WinChunk ch = chunks[ci];
+            if (held != ci) {
+                if (ci != win.chunk) __syncthreads();  // the previous chunk has been read
+                for (int o = (int)tid * 16; o < ch.bytes; o += (int)blockDim.x * 16)
+                    *(double2 *)(stage + o) = *(const double2 *)(program + ch.offset + o);
+                held = ci;
+            }
+            __syncthreads();
+            const WinGroup *groups = (const WinGroup *)(stage + ch.groups);
+            const WinTerm *terms = (const WinTerm *)(stage + ch.terms);
+            for (int r = 0; r < ch.nrounds; ++r) {
+                const WinRound &rd = ((const WinRound *)stage)[r];
+                uint32_t l0 = 0;
 #pragma unroll
-        for (int q = 0; q < 16; ++q) {
-            double cq = 0.0;
-            for (int t = s_pbeg[q]; t < s_pbeg[q + 1]; ++t)
-                cq += (__popcll(fixed & s_tc[t].z) & 1) ? -s_tc[t].ca : s_tc[t].ca;
-            C[q] = cq;
-        }
+                for (int j = 0; j < 8; ++j) l0 |= rd.lane[j] & on[j];
+                const uint32_t at = win_place(l0);
+                const uint32_t E0 = rd.vec[0], E1 = rd.vec[1], E2 = rd.vec[2], E3 = rd.vec[3];
+                auto amp = [&](int e) {
+                    return *(const double2 *)(win_smem +
+                                              (at ^ ((e & 1) ? E0 : 0u) ^ ((e & 2) ? E1 : 0u) ^
+                                               ((e & 4) ? E2 : 0u) ^ ((e & 8) ? E3 : 0u)));
+                };
+                auto neg = [&](const WinTerm &tm) {
+                    return (uint32_t)(__popcll(tb & tm.z) + __popc(l0 & tm.lz));
+                };
+                if (rd.nz) {
+                    // the terms add up by their parities with the vectors, and a 16-point
+                    // Walsh-Hadamard transform gives every element's coefficient
+                    double c[16];
+                    int t = rd.zterm;
+                    const int t1 = t + rd.nz;
 #pragma unroll
-        for (int hs = 1; hs < 16; hs <<= 1) {
+                    for (int q = 0; q < 16; ++q) {
+                        c[q] = 0.0;
+                        for (; t < t1 && terms[t].mask == (uint32_t)q; ++t)
+                            c[q] += win_sign(terms[t].c, neg(terms[t]));
+                    }
 #pragma unroll
-            for (int q = 0; q < 16; ++q) {
-                if (q & hs) continue;
-                const double x = C[q], y = C[q | hs];
-                C[q] = x + y;
-                C[q | hs] = x - y;
+                    for (int s = 1; s < 16; s <<= 1)
+#pragma unroll
+                        for (int q = 0; q < 16; ++q) {
+                            if (q & s) continue;
+                            const double x = c[q], y = c[q | s];
+                            c[q] = x + y;
+                            c[q | s] = x - y;
+                        }
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) {
+                        const double2 a = amp(e);
+                        acc[0] += (a.x * a.x + a.y * a.y) * c[e];
+                    }
+                }
+                if (rd.ngroups == 0) continue;
+                double2 a[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) a[e] = amp(e);
+                for (int g = rd.group; g < rd.group + rd.ngroups; ++g) {
+                    const WinGroup gr = groups[g];
+                    const bool odd = gr.odd != 0;
+                    double wr[8], wi_[8];
+                    // (else every mask's products are taken out of the loop, into memory)
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) asm volatile("" : "+d"(a[e].x), "+d"(a[e].y));
+                    switch (gr.d) {
+#define LQ_WIN(D) case D: win_pairs<D>(a, odd, wr, wi_); break;
+                        LQ_WIN(1) LQ_WIN(2) LQ_WIN(3) LQ_WIN(4) LQ_WIN(5) LQ_WIN(6) LQ_WIN(7)
+                        LQ_WIN(8) LQ_WIN(9) LQ_WIN(10) LQ_WIN(11) LQ_WIN(12) LQ_WIN(13) LQ_WIN(14)
+                        default: win_pairs<15>(a, odd, wr, wi_); break;
+#undef LQ_WIN
+                    }
+                    for (int t = gr.term; t < gr.term + gr.nterms; ++t) {
+                        const WinTerm tm = terms[t];
+                        double x = 0.0;  // a term counts the real or the imaginary parts
+                        if (tm.odd) {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) x += win_sign(wi_[k], tm.mask >> k);
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) x += win_sign(wr[k], tm.mask >> k);
+                        }
+                        acc[0] += 2.0 * win_sign(tm.c * x, neg(tm));
+                    }
+                }
             }
         }
-#pragma unroll
-        for (int k = 0; k < 16; ++k) acc[0] += pr[k] * C[k];
     }
     block_sum<1>(acc, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
@@ -414,36 +556,25 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
 // ---------------------------------------------------------------------------
 constexpr int kScanChunk = 1024;
 
-__global__ void __launch_bounds__(256) k_probs_exact_c128(const double2 *__restrict__ v,
-                                                          double *__restrict__ p, uint64_t N) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < N;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const double2 a = v[i];
-        p[i] = __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));  // no contraction
-    }
+// |a|^2 with no contraction, and plain doubles (the totals of a lower level).
+__device__ __forceinline__ double scan_value(double2 a) {
+    return __dadd_rn(__dmul_rn(a.x, a.x), __dmul_rn(a.y, a.y));
 }
-
-__global__ void __launch_bounds__(256) k_probs_exact_c64(const float2 *__restrict__ v,
-                                                         double *__restrict__ p, uint64_t N) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < N;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const float2 a = v[i];
-        const double x = a.x, y = a.y;
-        p[i] = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
-    }
+__device__ __forceinline__ double scan_value(float2 a) {
+    return scan_value(make_double2(a.x, a.y));
 }
+__device__ __forceinline__ double scan_value(double x) { return x; }
 
-__global__ void __launch_bounds__(256) k_scan_chunks(const double *__restrict__ in,
-                                                     double *__restrict__ out,
-                                                     double *__restrict__ chunk_total,
-                                                     uint64_t N) {
-    __shared__ double W[8];
+// The scan of one chunk (256 threads): v[j] of value base + j, base = 4 * thread
+// within the chunk.  W: 8 doubles of shared memory.
+template <class V>
+__device__ __forceinline__ void scan_chunk(const V *__restrict__ in, uint64_t base, uint64_t N,
+                                           double *W, double (&v)[4]) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint64_t base = (uint64_t)blockIdx.x * kScanChunk + 4u * t;
     double s[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const double x = base + j < N ? in[base + j] : 0.0;
+        const double x = base + j < N ? scan_value(in[base + j]) : 0.0;
         s[j] = j == 0 ? x : __dadd_rn(s[j - 1], x);
     }
     double incl = s[3];
@@ -467,11 +598,26 @@ __global__ void __launch_bounds__(256) k_scan_chunks(const double *__restrict__ 
     __syncthreads();
     const double off = __dadd_rn(W[warp], excl);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const double v = __dadd_rn(off, s[j]);
-        if (base + j < N) out[base + j] = v;
-        if (t == 255 && j == 3) chunk_total[blockIdx.x] = v;
+    for (int j = 0; j < 4; ++j) v[j] = __dadd_rn(off, s[j]);
+}
+
+// Chunk scans of in (amplitudes, or totals of a lower level) into out, if given, and
+// the chunk totals.
+template <class V>
+__global__ void __launch_bounds__(256) k_scan_chunks(const V *__restrict__ in,
+                                                     double *__restrict__ out,
+                                                     double *__restrict__ chunk_total,
+                                                     uint64_t N) {
+    __shared__ double W[8];
+    const uint64_t base = (uint64_t)blockIdx.x * kScanChunk + 4u * threadIdx.x;
+    double v[4];
+    scan_chunk(in, base, N, W, v);
+    if (out) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (base + j < N) out[base + j] = v[j];
     }
+    if (threadIdx.x == 255) chunk_total[blockIdx.x] = v[3];
 }
 
 __global__ void k_scan_add_base(double *__restrict__ cdf, const double *__restrict__ incl_total,
@@ -483,29 +629,77 @@ __global__ void k_scan_add_base(double *__restrict__ cdf, const double *__restri
     }
 }
 
-__global__ void k_sample(const double *__restrict__ cdf, uint64_t N, uint64_t nshots,
-                         uint64_t seed, uint64_t *__restrict__ out) {
-    const double total = cdf[N - 1];
+__device__ __forceinline__ double shot_uniform(uint64_t seed, uint64_t s, double total) {
+    const uint64_t r = splitmix64(seed ^ splitmix64(s));
+    return (double)(r >> 11) * (1.0 / 9007199254740992.0) * total;
+}
+
+// cdf(i) = scanned total of the chunks before i's + i's value in its chunk's scan: the
+// sum that a sweep adding the bases would store, formed at the values the search probes.
+__device__ __forceinline__ double chunk_base(const double *__restrict__ incl_total, uint64_t c,
+                                             double local) {
+    return c ? __dadd_rn(incl_total[c - 1], local) : local;
+}
+
+__global__ void k_sample(const double *__restrict__ local, const double *__restrict__ incl_total,
+                         uint64_t N, uint64_t nshots, uint64_t seed, uint64_t *__restrict__ out) {
+    auto cdf = [&](uint64_t i) { return chunk_base(incl_total, i / kScanChunk, local[i]); };
+    const double total = cdf(N - 1);
     for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < nshots;
          s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t r = splitmix64(seed ^ splitmix64(s));
-        const double u = (double)(r >> 11) * (1.0 / 9007199254740992.0) * total;
+        const double u = shot_uniform(seed, s, total);
         // first index with cdf > u
         uint64_t lo = 0, hi = N - 1;
         while (lo < hi) {
             const uint64_t mid = (lo + hi) >> 1;
-            if (cdf[mid] > u) hi = mid;
+            if (cdf(mid) > u) hi = mid;
             else lo = mid + 1;
         }
         out[s] = lo;
     }
 }
 
-static int red_grid(uint64_t N, int threads) {
-    uint64_t g = (N + threads - 1) / threads;
-    if (g > (uint64_t)kRedBlocks) g = kRedBlocks;
-    if (g < 1) g = 1;
-    return (int)g;
+// The same search without the stored scan (N a power of two of at least two chunks):
+// every probe above a chunk's width falls on a chunk's last value, which is its total;
+// the chunk it ends in is scanned again.  One block per shot.
+template <class A>
+__global__ void __launch_bounds__(256)
+    k_sample_rescan(const A *__restrict__ v, const double *__restrict__ chunk_total,
+                    const double *__restrict__ incl_total, uint64_t N, uint64_t nshots,
+                    uint64_t seed, uint64_t *__restrict__ out) {
+    __shared__ double W[8];
+    __shared__ double s_v[kScanChunk];
+    __shared__ uint64_t s_chunk;
+    const uint64_t nc = N / kScanChunk;
+    const double total = chunk_base(incl_total, nc - 1, chunk_total[nc - 1]);
+    for (uint64_t s = blockIdx.x; s < nshots; s += gridDim.x) {
+        const double u = shot_uniform(seed, s, total);
+        if (threadIdx.x == 0) {
+            uint64_t lo = 0, hi = nc - 1;
+            while (lo < hi) {
+                const uint64_t mid = (lo + hi) >> 1;
+                if (chunk_base(incl_total, mid, chunk_total[mid]) > u) hi = mid;
+                else lo = mid + 1;
+            }
+            s_chunk = lo;
+        }
+        __syncthreads();
+        const uint64_t c = s_chunk;
+        double x[4];
+        scan_chunk(v, c * kScanChunk + 4u * threadIdx.x, N, W, x);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s_v[4 * threadIdx.x + j] = x[j];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint64_t lo = 0, hi = kScanChunk - 1;
+            while (lo < hi) {
+                const uint64_t mid = (lo + hi) >> 1;
+                if (chunk_base(incl_total, c, s_v[mid]) > u) hi = mid;
+                else lo = mid + 1;
+            }
+            out[s] = c * kScanChunk + lo;
+        }
+    }
 }
 
 static int grid_for(uint64_t N, int threads) {
@@ -531,13 +725,26 @@ static int norm_sqr_device(const lq_state *s, double *d_out) {
 }
 
 int normalize_impl(lq_state *s) {
-    double *d_norm = s->d_red + kRedBlocks * 2 * kMaxTermsPerPass - 1;
-    LQ_TRY(norm_sqr_device(s, d_norm));
+    const uint64_t N = 1ull << s->n;
+    const int g = red_grid(N, 256);
+    prof_begin(s->stream, kProfReduce);
+    if (s->dtype == LQ_C128)
+        k_norm_partial<<<g, 256, 0, s->stream>>>((const double2 *)s->d, N, s->d_red);
+    else
+        k_norm_partial<<<g, 256, 0, s->stream>>>((const float2 *)s->d, N, s->d_red);
+    prof_end(s->stream, kProfReduce);
+    LQ_CUDA_TRY(cudaGetLastError());
+    return scale_by_partials(s, nullptr, g);
+}
+
+int scale_by_partials(lq_state *s, const void *src, int nparts) {
     const uint64_t N = 1ull << s->n;
     if (s->dtype == LQ_C128)
-        k_scale_by_norm<<<grid_for(N, 256), 256, 0, s->stream>>>((double2 *)s->d, N, d_norm);
+        k_scale_by_partials<<<red_grid(N, 256), 256, 0, s->stream>>>(
+            (double2 *)s->d, (const double2 *)src, N, s->d_red, nparts);
     else
-        k_scale_by_norm<<<grid_for(N, 256), 256, 0, s->stream>>>((float2 *)s->d, N, d_norm);
+        k_scale_by_partials<<<red_grid(N, 256), 256, 0, s->stream>>>(
+            (float2 *)s->d, (const float2 *)src, N, s->d_red, nparts);
     LQ_CUDA_TRY(cudaGetLastError());
     return LQ_OK;
 }
@@ -609,86 +816,279 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
     const uint64_t N = 1ull << n;
     const int th = 256;
     const int g = red_grid(std::max<uint64_t>(N / 2, 1), th);
-    // The X-mask-0 group of a state with 12 or more qubits runs the folded form
-    // (k_pauli_zfold): its terms sorted by bits 8-11 of the Z mask.
-    int zfold = -1;
-    int pbeg[17] = {0};
-    if (!per_term && n >= 12) {
-        for (size_t gi = 0; gi < groups.size(); ++gi)
-            if (groups[gi].first == 0) zfold = (int)gi;
-    }
-    if (zfold >= 0) {
-        auto pat = [&](int t) { return (int)((terms[t].zmask >> 8) & 15); };
-        std::vector<int> &ts = groups[zfold].second;
-        std::stable_sort(ts.begin(), ts.end(), [&](int x, int y) { return pat(x) < pat(y); });
-        for (int q = 0; q <= 16; ++q) {
-            int k = 0;
-            while (k < (int)ts.size() && pat(ts[k]) < q) ++k;
-            pbeg[q] = k;
+    // Windows: the fewest that hold every group's X bits (each is a sweep).  A group's X
+    // bits above bit 3 need h in [hi - m + 1, lo]; points stabbing every such interval,
+    // chosen greedily by right end, are a minimum set.  Groups with none go to the first
+    // window, and groups too wide for any keep a sweep of their own.
+    // Tile bits: the whole state up to 2^12 amplitudes (zeros above it below 2^9), else at
+    // least 2^7 tiles down to 2^10 amplitudes each, so that smaller states still fill the
+    // chip.
+    const int T = n <= kWinT ? std::max(n, kWinMinT) : std::max(10, std::min(kWinT, n - 7));
+    const int m = T - 4;
+    struct Need {
+        int a, b;
+        size_t group;
+    };
+    std::vector<Need> needs;
+    std::vector<size_t> anywhere, sweeps;
+    for (size_t gi = 0; gi < groups.size(); ++gi) {
+        const uint64_t up = groups[gi].first & ~0xFull;
+        if (per_term) {
+            sweeps.push_back(gi);
+        } else if (!up) {
+            anywhere.push_back(gi);
+        } else {
+            const int lo = __builtin_ctzll(up), hi = 63 - __builtin_clzll(up);
+            const int a = std::max(4, hi - m + 1), b = std::min(lo, std::max(4, n - m));
+            if (a <= b) needs.push_back(Need{a, b, gi});
+            else sweeps.push_back(gi);
         }
     }
-    // Host-side packed coefficients, uploaded once per call.
-    std::vector<TermCoef> tc(nterms);
+    std::stable_sort(needs.begin(), needs.end(),
+                     [](const Need &x, const Need &y) { return x.b < y.b; });
+    std::vector<std::pair<int, std::vector<size_t>>> wsets;
+    for (const Need &q : needs) {
+        if (wsets.empty() || wsets.back().first < q.a) wsets.push_back({q.b, {}});
+        wsets.back().second.push_back(q.group);
+    }
+    if (wsets.empty() && !anywhere.empty()) wsets.push_back({4, {}});
+    if (!wsets.empty())
+        wsets[0].second.insert(wsets[0].second.end(), anywhere.begin(), anywhere.end());
+    auto coef_of = [&](int t) {
+        double a, b;
+        selectors(terms[t].ny, a, b);
+        return TermCoef{terms[t].zmask, terms[t].coefficient * a, terms[t].coefficient * b};
+    };
+    std::vector<WinDesc> wins;
+    std::vector<WinChunk> chunks;
+    std::vector<unsigned char> program;
+    const int tiles = 1 << std::max(n - T, 0);
+    int nwork = 0;
+    for (const auto &ws : wsets) {
+        const int h = ws.first;
+        const uint64_t inside = 15ull | ((1ull << m) - 1) << h;
+        auto local = [&](uint64_t mask) {
+            return (uint32_t)(mask & 15u) | (uint32_t)((mask >> h) & ((1ull << m) - 1)) << 4;
+        };
+        auto parity = [](uint32_t x) { return (uint32_t)__builtin_popcount(x) & 1u; };
+        // rounds: in order of their masks, a group joins if it lies in the span of the
+        // vectors or there are fewer than four
+        struct Round {
+            uint32_t vec[4];
+            int piv[4], rank = 0;
+            std::vector<size_t> groups;
+        };
+        std::vector<Round> rounds;
+        std::vector<size_t> left = ws.second;
+        std::stable_sort(left.begin(), left.end(), [&](size_t x, size_t y) {
+            return local(groups[x].first) < local(groups[y].first);
+        });
+        while (!left.empty()) {
+            Round r;
+            std::vector<size_t> later;
+            for (size_t gi : left) {
+                uint32_t x = local(groups[gi].first);
+                for (int k = 0; k < r.rank; ++k)
+                    if ((x >> r.piv[k]) & 1u) x ^= r.vec[k];
+                if (x && r.rank == 4) {
+                    later.push_back(gi);
+                    continue;
+                }
+                if (x) {
+                    const int p = 31 - __builtin_clz(x);
+                    for (int k = 0; k < r.rank; ++k)
+                        if ((r.vec[k] >> p) & 1u) r.vec[k] ^= x;
+                    r.vec[r.rank] = x;
+                    r.piv[r.rank++] = p;
+                }
+                r.groups.push_back(gi);
+            }
+            for (int p = T - 1; r.rank < 4; --p) {
+                bool used = false;
+                for (int k = 0; k < r.rank; ++k) used |= r.piv[k] == p;
+                if (used) continue;
+                for (int k = 0; k < r.rank; ++k)
+                    if ((r.vec[k] >> p) & 1u) r.vec[k] ^= 1u << p;
+                r.vec[r.rank] = 1u << p;
+                r.piv[r.rank++] = p;
+            }
+            rounds.push_back(std::move(r));
+            left.swap(later);
+        }
+        // few tiles: the rounds are shared out among more blocks
+        const int share = std::max(1, 2 * 148 / (tiles * (int)wsets.size()));
+        const size_t parts = std::min<size_t>(rounds.size(), (size_t)share);
+        for (size_t part = 0; part < parts; ++part) {
+            WinDesc wd{h, (int)chunks.size(), 0, nwork};
+            nwork += tiles;
+            std::vector<WinRound> cr;
+            std::vector<WinGroup> cg;
+            std::vector<WinTerm> ct;
+            auto bytes = [&] {
+                return cr.size() * sizeof(WinRound) + cg.size() * sizeof(WinGroup) +
+                       ct.size() * sizeof(WinTerm);
+            };
+            auto close = [&] {
+                if (cr.empty()) return;
+                WinChunk c{(int)program.size(), (int)bytes(), (int)cr.size(),
+                           (int)(cr.size() * sizeof(WinRound)),
+                           (int)(cr.size() * sizeof(WinRound) + cg.size() * sizeof(WinGroup))};
+                program.resize(program.size() + bytes());
+                unsigned char *to = program.data() + c.offset;
+                memcpy(to, cr.data(), c.groups);
+                if (!cg.empty()) memcpy(to + c.groups, cg.data(), c.terms - c.groups);
+                memcpy(to + c.terms, ct.data(), c.bytes - c.terms);
+                chunks.push_back(c);
+                cr.clear(), cg.clear(), ct.clear();
+            };
+            for (size_t ri = part; ri < rounds.size(); ri += parts) {
+                const Round &r = rounds[ri];
+                WinRound hd{};
+                uint32_t pivots = 0;
+                for (int k = 0; k < 4; ++k) {
+                    hd.vec[k] = win_place(r.vec[k]);
+                    pivots |= 1u << r.piv[k];
+                }
+                // thread bits: first three whose places lie in different banks
+                std::vector<int> lanes;
+                for (int turn = 0; turn < 2; ++turn)
+                    for (int p = 0, seen = 0; p < T; ++p) {
+                        if (pivots >> p & 1u) continue;
+                        const bool first = !(seen >> (p % 3) & 1);
+                        seen |= 1 << (p % 3);
+                        if (first == (turn == 0)) lanes.push_back(p);
+                    }
+                for (size_t j = 0; j < lanes.size(); ++j) hd.lane[j] = 1u << lanes[j];
+                auto open = [&](size_t more) {
+                    if (!cr.empty() && bytes() + more > (size_t)kWinStage) close();
+                    hd.group = (int)cg.size(), hd.ngroups = 0;
+                    hd.zterm = (int)ct.size(), hd.nz = 0;
+                    cr.push_back(hd);
+                };
+                // (a piece of a group must fit a stage of its own)
+                constexpr size_t piece = (kWinStage - sizeof(WinRound) - sizeof(WinGroup)) / sizeof(WinTerm);
+                bool opened = false;
+                for (int zturn = 1; zturn >= 0; --zturn)  // a round's terms without X come first
+                    for (size_t gi : r.groups) {
+                        const uint32_t lx = local(groups[gi].first);
+                        if ((lx == 0) != (zturn == 1)) continue;
+                        WinGroup wg{};
+                        for (int k = 0; k < 4; ++k) wg.d |= (int)((lx >> r.piv[k]) & 1u) << k;
+                        std::vector<WinTerm> all;
+                        for (int t : groups[gi].second) {
+                            const TermCoef c = coef_of(t);
+                            const uint32_t odd = terms[t].ny & 1;
+                            WinTerm wt{c.z & ~inside, odd ? c.cb : c.ca, local(c.z), 0, odd, 0};
+                            uint32_t on = 0;
+                            for (int k = 0; k < 4; ++k) on |= parity(wt.lz & r.vec[k]) << k;
+                            if (lx == 0) wt.mask = on;
+                            else
+                                for (int k = 0; k < 8; ++k)
+                                    wt.mask |= parity(on & (uint32_t)win_pair(k, wg.d)) << k;
+                            wg.odd |= (int)odd;
+                            all.push_back(wt);
+                        }
+                        if (lx == 0)
+                            std::stable_sort(all.begin(), all.end(),
+                                             [](const WinTerm &x, const WinTerm &y) { return x.mask < y.mask; });
+                        for (size_t b = 0; b < all.size(); b += piece) {
+                            const size_t e = std::min(all.size(), b + piece);
+                            const size_t need = (e - b) * sizeof(WinTerm) + sizeof(WinGroup);
+                            if (!opened || bytes() + need > (size_t)kWinStage)
+                                open(need + sizeof(WinRound)), opened = true;
+                            WinRound &rd = cr.back();
+                            if (lx == 0) {
+                                rd.zterm = (int)ct.size();
+                                rd.nz = (int)(e - b);
+                            } else {
+                                wg.term = (int)ct.size();
+                                wg.nterms = (int)(e - b);
+                                cg.push_back(wg);
+                                ++rd.ngroups;
+                            }
+                            ct.insert(ct.end(), all.begin() + b, all.begin() + e);
+                        }
+                    }
+            }
+            close();
+            wd.nchunks = (int)chunks.size() - wd.chunk;
+            wins.push_back(wd);
+        }
+    }
+    // Host-side packed coefficients of the sweeps, uploaded with the windows' once per
+    // call, and the results: the windows' sum, then one per sweep.
     std::vector<int> offs;
-    int off = 0;
     std::vector<TermCoef> packed;
-    for (auto &gr : groups) {
-        offs.push_back(off);
-        for (int t : gr.second) {
-            double a, b;
-            selectors(terms[t].ny, a, b);
-            packed.push_back(TermCoef{terms[t].zmask, terms[t].coefficient * a,
-                                      terms[t].coefficient * b});
-        }
-        off += (int)gr.second.size();
+    for (size_t gi : sweeps) {
+        offs.push_back((int)packed.size());
+        for (int t : groups[gi].second) packed.push_back(coef_of(t));
     }
     lq_state *ms = const_cast<lq_state *>(s);
-    const size_t coef_bytes = packed.size() * sizeof(TermCoef);
-    const size_t res_bytes = groups.size() * sizeof(double);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    LQ_TRY(ensure_prog(ms, al(coef_bytes) + al(res_bytes) + sizeof(pbeg) + 256));
-    TermCoef *d_tc = (TermCoef *)ms->d_prog;
-    double *d_res = (double *)((char *)ms->d_prog + al(coef_bytes));
-    int *d_pbeg = (int *)((char *)ms->d_prog + al(coef_bytes) + al(res_bytes));
-    if (!packed.empty())
-        LQ_CUDA_TRY(cudaMemcpyAsync(d_tc, packed.data(), coef_bytes, cudaMemcpyHostToDevice,
-                                    s->stream));
-    if (zfold >= 0)
-        LQ_CUDA_TRY(cudaMemcpyAsync(d_pbeg, pbeg, sizeof(pbeg), cudaMemcpyHostToDevice,
-                                    s->stream));
+    const size_t o_win = al(packed.size() * sizeof(TermCoef));
+    const size_t o_chk = o_win + al(wins.size() * sizeof(WinDesc));
+    const size_t o_pgm = o_chk + al(chunks.size() * sizeof(WinChunk));
+    const size_t o_res = o_pgm + al(program.size());
+    const size_t nres = sweeps.size() + (wins.empty() ? 0 : 1);
+    LQ_TRY(ensure_prog(ms, o_res + al(nres * sizeof(double)) + 256));
+    char *dp = (char *)ms->d_prog;
+    const TermCoef *d_tc = (const TermCoef *)dp;
+    double *d_res = (double *)(dp + o_res);
+    {
+        std::vector<char> up(o_res, 0);
+        auto put = [&](size_t o, const auto &x) {
+            if (!x.empty()) memcpy(up.data() + o, x.data(), x.size() * sizeof(x[0]));
+        };
+        put(0, packed);
+        put(o_win, wins);
+        put(o_chk, chunks);
+        put(o_pgm, program);
+        LQ_CUDA_TRY(cudaMemcpyAsync(dp, up.data(), o_res, cudaMemcpyHostToDevice, s->stream));
+    }
     prof_begin(s->stream, kProfReduce);
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        const int nt = (int)groups[gi].second.size();
+    size_t ri = 0;
+    if (!wins.empty()) {
+        const int blocks = std::min(nwork, 2 * 148);
+        const size_t shm = ((size_t)16 << T) + kWinStage;
+        auto run = [&](auto *v) -> cudaError_t {
+            using A = std::remove_const_t<std::remove_pointer_t<decltype(v)>>;
+            const cudaError_t e =
+                cudaFuncSetAttribute(k_pauli_windows<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (16 << kWinT) + kWinStage);
+            if (e != cudaSuccess) return e;
+            k_pauli_windows<A><<<blocks, 1 << m, shm, s->stream>>>(
+                v, n, T, (const WinDesc *)(dp + o_win), (int)wins.size(),
+                (const WinChunk *)(dp + o_chk), (const unsigned char *)(dp + o_pgm), nwork,
+                ms->d_red);
+            return cudaGetLastError();
+        };
+        LQ_CUDA_TRY(s->dtype == LQ_C128 ? run((const double2 *)s->d) : run((const float2 *)s->d));
+        k_final_sum<1><<<1, 256, 0, s->stream>>>(s->d_red, blocks, d_res + ri++);
+    }
+    for (size_t k = 0; k < sweeps.size(); ++k) {
+        const auto &gr = groups[sweeps[k]];
+        const int nt = (int)gr.second.size();
         const size_t shm = nt * sizeof(TermCoef);
-        if ((int)gi == zfold) {
-            if (s->dtype == LQ_C128)
-                k_pauli_zfold<<<g, th, shm, s->stream>>>((const double2 *)s->d, n,
-                                                         d_tc + offs[gi], nt, d_pbeg, s->d_red);
-            else
-                k_pauli_zfold<<<g, th, shm, s->stream>>>((const float2 *)s->d, n,
-                                                         d_tc + offs[gi], nt, d_pbeg, s->d_red);
-        } else if (s->dtype == LQ_C128) {
-            k_pauli_group<<<g, th, shm, s->stream>>>((const double2 *)s->d, n, groups[gi].first,
-                                                     d_tc + offs[gi], nt, s->d_red);
-        } else {
-            k_pauli_group<<<g, th, shm, s->stream>>>((const float2 *)s->d, n, groups[gi].first,
-                                                     d_tc + offs[gi], nt, s->d_red);
-        }
-        k_final_sum<1><<<1, 256, 0, s->stream>>>(s->d_red, g, d_res + gi);
+        if (s->dtype == LQ_C128)
+            k_pauli_group<<<g, th, shm, s->stream>>>((const double2 *)s->d, n, gr.first,
+                                                     d_tc + offs[k], nt, s->d_red);
+        else
+            k_pauli_group<<<g, th, shm, s->stream>>>((const float2 *)s->d, n, gr.first,
+                                                     d_tc + offs[k], nt, s->d_red);
+        k_final_sum<1><<<1, 256, 0, s->stream>>>(s->d_red, g, d_res + ri++);
     }
     prof_end(s->stream, kProfReduce);
     LQ_CUDA_TRY(cudaGetLastError());
-    std::vector<double> res(groups.size());
-    if (!groups.empty())
-        LQ_CUDA_TRY(cudaMemcpyAsync(res.data(), d_res, res_bytes, cudaMemcpyDeviceToHost,
-                                    s->stream));
+    std::vector<double> res(nres);
+    if (nres)
+        LQ_CUDA_TRY(cudaMemcpyAsync(res.data(), d_res, nres * sizeof(double),
+                                    cudaMemcpyDeviceToHost, s->stream));
     LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
-    // Sum group results in term order (PauliObservable::expectation sums
-    // term.expectation in order, src/optimization/observable.rs:229-231).
     double sum = 0.0;
-    for (size_t gi = 0; gi < groups.size(); ++gi) {
-        sum += res[gi];
-        if (per_term) per_term[groups[gi].second[0]] = res[gi];
+    for (size_t k = 0; k < nres; ++k) {
+        sum += res[k];
+        // (with per-term values every term is a sweep of its own, in order)
+        if (per_term) per_term[groups[sweeps[k]].second[0]] = res[k];
     }
     *out = sum;
     return LQ_OK;
@@ -950,6 +1350,7 @@ int lq_state_destroy(lq_state *s) {
     if (s->d_red) cudaFree(s->d_red);
     if (s->d_flag) cudaFree(s->d_flag);
     if (s->d_prog) cudaFree(s->d_prog);
+    if (s->d_work) cudaFree(s->d_work);
     free_plan_cache(s);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -1258,31 +1659,52 @@ static uint64_t scan_scratch(uint64_t N) {  // doubles needed by scan_inclusive'
     return need + 2;
 }
 
+}  // extern "C"
+
+// The amplitudes' scan: chunk scans (kept or not), their totals, the totals scanned.
+template <class A>
+static int measure_shots_t(lq_state *s, const A *v, uint64_t n_shots, uint64_t seed,
+                           uint64_t *host_out) {
+    const uint64_t N = 1ull << s->n, nc = (N + kScanChunk - 1) / kScanChunk;
+    if (nc > 0x7fffffffull) return set_error(LQ_ERR_UNSUPPORTED, "scan too long");
+    cudaStream_t st = s->stream;
+    // The chunk scans are kept where they fit the handle's workspace, or where so many
+    // shots come that one chunk each would cost more.  Above that a call would allocate
+    // half the state's size for some probes (mapping 64 MB fresh and returning it takes
+    // 0.4 to 20 ms); a chunk scanned again costs a shot about 4 ns of the whole GPU.
+    const bool keep = N * 8 <= kKeptWork / 2 || n_shots > N / 64;
+    const uint64_t scratch = scan_scratch(N);
+    const uint64_t need = ((keep ? N : 0) + scratch + n_shots) * 8;
+    void *work = nullptr;
+    LQ_TRY(take_work(s, need, &work));
+    double *tot = (double *)work, *local = keep ? tot + scratch + n_shots : nullptr;
+    uint64_t *d_out = (uint64_t *)(tot + scratch);
+    double *incl = tot + nc;
+    k_scan_chunks<<<(unsigned)nc, 256, 0, st>>>(v, local, tot, N);
+    LQ_CUDA_TRY(cudaGetLastError());
+    if (nc > 1) LQ_TRY(scan_inclusive(tot, incl, incl + nc, nc, st));
+    if (keep)
+        k_sample<<<grid_for(n_shots, 256), 256, 0, st>>>(local, incl, N, n_shots, seed, d_out);
+    else
+        k_sample_rescan<<<(unsigned)std::min<uint64_t>(n_shots, 148 * 8), 256, 0, st>>>(
+            v, tot, incl, N, n_shots, seed, d_out);
+    LQ_CUDA_TRY(cudaGetLastError());
+    LQ_CUDA_TRY(cudaMemcpyAsync(host_out, d_out, n_shots * 8, cudaMemcpyDeviceToHost, st));
+    LQ_TRY(give_work(s, work));
+    LQ_CUDA_TRY(cudaStreamSynchronize(st));
+    return LQ_OK;
+}
+
+extern "C" {
+
 int lq_measure_shots(const lq_state *s, uint64_t n_shots, uint64_t seed, uint64_t *host_out) {
     LQ_TRY(check_state(s));
     if (!host_out && n_shots) return set_error(LQ_ERR_INVALID_ARG, "null output");
     if (n_shots == 0) return LQ_OK;
-    const uint64_t N = 1ull << s->n;
-    double *p = nullptr, *cdf = nullptr, *tot = nullptr;
-    uint64_t *d_out = nullptr;
-    LQ_CUDA_TRY(cudaMallocAsync(&p, N * 8, s->stream));
-    LQ_CUDA_TRY(cudaMallocAsync(&cdf, N * 8, s->stream));
-    LQ_CUDA_TRY(cudaMallocAsync(&tot, scan_scratch(N) * 8, s->stream));
-    LQ_CUDA_TRY(cudaMallocAsync(&d_out, n_shots * 8, s->stream));
+    lq_state *ms = const_cast<lq_state *>(s);  // (its workspace)
     if (s->dtype == LQ_C128)
-        k_probs_exact_c128<<<grid_for(N, 256), 256, 0, s->stream>>>((const double2 *)s->d, p, N);
-    else
-        k_probs_exact_c64<<<grid_for(N, 256), 256, 0, s->stream>>>((const float2 *)s->d, p, N);
-    LQ_TRY(scan_inclusive(p, cdf, tot, N, s->stream));
-    k_sample<<<grid_for(n_shots, 256), 256, 0, s->stream>>>(cdf, N, n_shots, seed, d_out);
-    LQ_CUDA_TRY(cudaGetLastError());
-    LQ_CUDA_TRY(cudaMemcpyAsync(host_out, d_out, n_shots * 8, cudaMemcpyDeviceToHost, s->stream));
-    LQ_CUDA_TRY(cudaFreeAsync(tot, s->stream));
-    LQ_CUDA_TRY(cudaFreeAsync(p, s->stream));
-    LQ_CUDA_TRY(cudaFreeAsync(cdf, s->stream));
-    LQ_CUDA_TRY(cudaFreeAsync(d_out, s->stream));
-    LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
-    return LQ_OK;
+        return measure_shots_t(ms, (const double2 *)s->d, n_shots, seed, host_out);
+    return measure_shots_t(ms, (const float2 *)s->d, n_shots, seed, host_out);
 }
 
 int lq_expectation_pauli(const lq_state *s, const lq_pauli_term *terms, int nterms,

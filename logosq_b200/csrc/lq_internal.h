@@ -75,6 +75,9 @@ struct lq_state {
     // Per-handle device buffer for gate programs of fused passes.
     void *d_prog = nullptr;
     size_t prog_cap = 0;
+    // Workspace of calls that need a few temporary arrays (take_work).
+    void *d_work = nullptr;
+    size_t work_cap = 0;
     // Statistics of the last circuit call.
     int last_launches = 0;
     int last_passes = 0;
@@ -108,8 +111,18 @@ int gate_matrix(const lq_gate *g, const double *theta, double *m /* 2*64 doubles
 enum GateClass { kClassGeneral = 0, kClassDiagonal = 1, kClassPermutation = 2 };
 int gate_class(int kind);
 
+// Temporary device memory for one call on s's stream.  Up to kKeptWork bytes stay with
+// the handle for its next call (one call at a time: the stream orders their use);
+// more is allocated and returned each time, so a large state never holds a second.
+constexpr size_t kKeptWork = 128ull << 20;
+int take_work(lq_state *s, size_t bytes, void **out);
+int give_work(lq_state *s, void *p);
+
 // api_state.cu
 int normalize_impl(lq_state *s);
+// The state, or src in its place, divided by the norm whose squared partial sums are
+// in s->d_red[0 .. nparts).
+int scale_by_partials(lq_state *s, const void *src, int nparts);
 // Record the state's FP64 squared norm; later rescale the state to it.
 int norm_snapshot(lq_state *s);
 int norm_restore(lq_state *s);
