@@ -11,6 +11,7 @@ const SOURCES: &[&str] = &[
     "api_state.cu",
     "gates.cu",
     "fused.cu",
+    "mapped.cu",
     "variational.cu",
     "profile.cu",
     "batch.cu",

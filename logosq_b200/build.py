@@ -21,6 +21,7 @@ SOURCES = [
     "api_state.cu",
     "gates.cu",
     "fused.cu",
+    "mapped.cu",
     "variational.cu",
     "profile.cu",
     "batch.cu",

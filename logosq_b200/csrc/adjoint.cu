@@ -42,7 +42,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <complex>
 #include <cstring>
 
 namespace lq {
@@ -886,20 +885,6 @@ public:
     }
 };
 
-using cd = std::complex<double>;
-
-static bool unitary(const double *m, int dim) {
-    for (int r = 0; r < dim; ++r)
-        for (int c = 0; c < dim; ++c) {
-            cd s = 0.0;
-            for (int k = 0; k < dim; ++k)
-                s += std::conj(cd(m[2 * (k * dim + r)], m[2 * (k * dim + r) + 1])) *
-                     cd(m[2 * (k * dim + c)], m[2 * (k * dim + c) + 1]);
-            if (!(std::abs(s - (r == c ? 1.0 : 0.0)) <= 1e-14)) return false;
-        }
-    return true;
-}
-
 // The inverse of a unitary op that is no run of single-qubit gates.
 static GateOp inverse_op(const GateOp &g) {
     GateOp r = g;
@@ -946,7 +931,7 @@ static bool gate_atoms(const lq_gate &g, int param_base, const GateOp &op, AdjPr
     } else {
         return false;
     }
-    if (!unitary(m, 2)) return false;
+    if (!unitary_matrix(m, 2)) return false;
     AdjAtom a{};
     a.kind = AT_CONST;
     a.param = -1;
@@ -1252,8 +1237,8 @@ static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProg
             continue;
         }
         if (bound) return false;
-        if (op.type == OP_M1 && !unitary(op.m, 2)) return false;
-        if (op.type == OP_M2 && !unitary(op.m, 4)) return false;
+        if (op.type == OP_M1 && !unitary_matrix(op.m, 2)) return false;
+        if (op.type == OP_M2 && !unitary_matrix(op.m, 4)) return false;
         const uint64_t bits = op_bits(op);
         for (int b = 0; b < 64; ++b)
             if ((bits >> b) & 1) open[b] = -1;

@@ -35,6 +35,7 @@
 
 #include "fused_plan.h"
 #include "fused_round.cuh"
+#include "mapped.h"
 
 namespace lq {
 
@@ -197,15 +198,6 @@ __device__ __forceinline__ void fused_pp_body(const CUtensorMap &tmap, int T, Ti
         // shared memory is released when the CTA exits: the store must have read it
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(256, 1)
-    k_fused_pp(const __grid_constant__ CUtensorMap tmap, int T, TileCoords tc,
-               const FusedRound *__restrict__ rounds, int nrounds, const PassOp *__restrict__ ops,
-               const double *__restrict__ coef, const uint16_t *__restrict__ tbtab,
-               unsigned *__restrict__ flag) {
-    fused_pp_body<MODE>(tmap, T, tc, rounds, nrounds, ops, coef, tbtab, flag);
 }
 
 // 168 registers: six 64-thread CTAs per SM at tile bits 10.  Measured on a
@@ -946,28 +938,12 @@ static int set_smem_attrs() {
     static bool done = false;
     if (done) return LQ_OK;
     const int mx = (int)fused_smem(kMaxT);
-    LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass<0>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass<1>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass<2>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass_narrow<0>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-    LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass_narrow<1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     LQ_CUDA_TRY(cudaFuncSetAttribute(k_fused_pass_narrow<2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
     done = true;
     return LQ_OK;
-}
-
-static int pp_engine() {  // 1: ping-pong register rounds over PassOp records
-    static const int v = [] {
-        const char *e = getenv("LQ_FUSED_ENGINE");
-        return e ? atoi(e) : 1;
-    }();
-    return v;
 }
 
 static int pair_index(int a, int b) {
@@ -1008,7 +984,6 @@ static int set_pp_attrs() {
     if (done) return LQ_OK;
     const int mx = (int)fused_smem(kMaxT);
 #define LQ_ATTR(K) LQ_CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
-    LQ_ATTR(k_fused_pp<1>);
     LQ_ATTR(k_fused_pp_narrow<1>);
 #undef LQ_ATTR
     done = true;
@@ -1032,16 +1007,16 @@ static int launch_pass_pp(lq_state *s, int T, int h, const FusedRound *d_rounds,
     K<<<ntiles, blk, smem, s->stream>>>(map, T, tc, d_rounds, nrounds, d_ops, d_coef, d_tb, \
                                         s->d_flag)
     (void)mode;  // one op set (4x4, pair and table ops included); blocks use launch_pass
-    if (T >= 12) LQ_FUSED_LAUNCH(k_fused_pp<1>);
-    else LQ_FUSED_LAUNCH(k_fused_pp_narrow<1>);
+    LQ_FUSED_LAUNCH(k_fused_pp_narrow<1>);
 #undef LQ_FUSED_LAUNCH
     prof_end(s->stream, kProfFused);
     LQ_CUDA_TRY(cudaGetLastError());
     return LQ_OK;
 }
 
-static int launch_pass(lq_state *s, int T, int h, const FusedRound *d_rounds, int nrounds,
-                       const FusedOp *d_ops, const double *d_coef, int mode) {
+// Block gates only (lq_apply_block): in-place rounds with 8x8 / 16x16 ops.
+static int launch_block_pass(lq_state *s, int T, int h, const FusedRound *d_rounds, int nrounds,
+                             const FusedOp *d_ops, const double *d_coef) {
     const int n = s->n;
     const int m = T - 4;
     CUtensorMap map;
@@ -1054,15 +1029,8 @@ static int launch_pass(lq_state *s, int T, int h, const FusedRound *d_rounds, in
     const dim3 blk(1u << (T - 4));
 #define LQ_FUSED_LAUNCH(K) \
     K<<<grid, blk, smem, s->stream>>>(map, T, tc, d_rounds, nrounds, d_ops, d_coef, s->d_flag)
-    if (T >= 12) {
-        if (mode == 2) LQ_FUSED_LAUNCH(k_fused_pass<2>);
-        else if (mode == 1) LQ_FUSED_LAUNCH(k_fused_pass<1>);
-        else LQ_FUSED_LAUNCH(k_fused_pass<0>);
-    } else {
-        if (mode == 2) LQ_FUSED_LAUNCH(k_fused_pass_narrow<2>);
-        else if (mode == 1) LQ_FUSED_LAUNCH(k_fused_pass_narrow<1>);
-        else LQ_FUSED_LAUNCH(k_fused_pass_narrow<0>);
-    }
+    if (T >= 12) LQ_FUSED_LAUNCH(k_fused_pass<2>);
+    else LQ_FUSED_LAUNCH(k_fused_pass_narrow<2>);
 #undef LQ_FUSED_LAUNCH
     prof_end(s->stream, kProfFused);
     LQ_CUDA_TRY(cudaGetLastError());
@@ -1218,6 +1186,9 @@ struct PlanCache {
         PassLaunch pl;
     };
     std::vector<Step> steps;
+    bool mapped = false;             // map holds the steps (mapped.cu), else steps does
+    MapProgram map;                  // (needs no device buffer)
+    bool normalize = false;          // State::normalize after the last step
 };
 
 void free_plan_cache(lq_state *s) {
@@ -1226,21 +1197,64 @@ void free_plan_cache(lq_state *s) {
     s->prog_valid = false;
 }
 
-static std::vector<unsigned char> plan_key(const lq_gate *ops, int nops, const double *theta,
-                                           int ntheta, int n, int T) {
-    const int32_t hdr[6] = {n, T, nops, ntheta, real_fold_mode(), pp_engine()};
-    std::vector<unsigned char> k(sizeof(hdr) + sizeof(lq_gate) * (size_t)nops +
-                                 sizeof(double) * (size_t)ntheta);
-    memcpy(k.data(), hdr, sizeof(hdr));
-    if (nops) memcpy(k.data() + sizeof(hdr), ops, sizeof(lq_gate) * (size_t)nops);
-    if (ntheta)
-        memcpy(k.data() + sizeof(hdr) + sizeof(lq_gate) * (size_t)nops, theta,
-               sizeof(double) * (size_t)ntheta);
-    return k;
+// What a plan depends on: sizes and settings, then the gates and the angles.
+struct PlanKeyView {
+    int32_t hdr[5];
+    const lq_gate *ops;
+    const double *theta;
+    size_t gates() const { return sizeof(lq_gate) * (size_t)hdr[2]; }
+    size_t angles() const { return sizeof(double) * (size_t)hdr[3]; }
+    bool equals(const std::vector<unsigned char> &k) const {
+        return k.size() == sizeof(hdr) + gates() + angles() &&
+               memcmp(k.data(), hdr, sizeof(hdr)) == 0 &&
+               (!gates() || memcmp(k.data() + sizeof(hdr), ops, gates()) == 0) &&
+               (!angles() || memcmp(k.data() + sizeof(hdr) + gates(), theta, angles()) == 0);
+    }
+    std::vector<unsigned char> copy() const {
+        std::vector<unsigned char> k(sizeof(hdr) + gates() + angles());
+        memcpy(k.data(), hdr, sizeof(hdr));
+        if (gates()) memcpy(k.data() + sizeof(hdr), ops, gates());
+        if (angles()) memcpy(k.data() + sizeof(hdr) + gates(), theta, angles());
+        return k;
+    }
+};
+
+// A renormalising gate scales the state by one number, and gates are linear: after a
+// unitary gate the division commutes with every later gate up to the next division.
+// So divisions by the norm after unitary gates are left out except the last, which
+// moves to the end of the circuit (returns true).  Before a gate that is not unitary and
+// does not renormalise itself it stays where it is.  (A zero vector, or one below the
+// 1e-10 threshold, keeps its norm through unitary gates and is left alone either way.)
+static bool defer_renorm(std::vector<GateOp> &gops) {
+    int last = -1;  // the gate that owes a division
+    for (size_t k = 0; k < gops.size(); ++k) {
+        GateOp &g = gops[k];
+        const bool uni = unitary_op(g);
+        if (!uni && last >= 0) {
+            gops[last].renorm = true;
+            last = -1;
+        }
+        if (uni && g.renorm) {
+            g.renorm = false;
+            last = (int)k;
+        }
+    }
+    return last >= 0;
 }
 
 static int launch_cached(lq_state *s, const PlanCache &pc) {
     const char *dp = (const char *)s->d_prog;
+    if (pc.mapped) {
+        for (const auto &st : pc.map.steps) {
+            if (st.fused) {
+                LQ_TRY(map_launch(s, pc.T, st.pass, pc.map.blob.data()));
+                s->last_passes += 1;
+            } else {
+                LQ_TRY(launch_gate_op(s, st.gate));
+            }
+            s->last_launches += 1;
+        }
+    }
     const FusedRound *d_rounds = (const FusedRound *)dp;
     const PassOp *d_ops = (const PassOp *)(dp + pc.off_ops);
     const double *d_coef = (const double *)(dp + pc.off_coef);
@@ -1256,6 +1270,10 @@ static int launch_cached(lq_state *s, const PlanCache &pc) {
         s->last_launches += 1;
         s->last_passes += 1;
     }
+    if (pc.normalize) {
+        LQ_TRY(normalize_impl(s));
+        s->last_launches += 2;
+    }
     return LQ_OK;
 }
 
@@ -1266,11 +1284,12 @@ int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *
     s->last_passes = 0;
     for (int i = 0; i < nops; ++i) LQ_TRY(validate_gate(&ops[i], n, ntheta));
     const bool can_fuse = mode == LQ_EXEC_FUSED && s->dtype == LQ_C128 && n >= 5;
-    std::vector<unsigned char> key;
-    if (can_fuse && pp_engine() == 1) {
-        key = plan_key(ops, nops, theta, ntheta, n, std::min(fusion_width(), n));
+    const PlanKeyView key{{n, std::min(fusion_width(), n), nops, ntheta, real_fold_mode()},
+                          ops, theta};
+    if (can_fuse) {
         const PlanCache *pc = static_cast<const PlanCache *>(s->plan_cache);
-        if (s->prog_valid && pc && pc->key == key) return launch_cached(s, *pc);
+        if (pc && (pc->mapped || s->prog_valid) && key.equals(pc->key))
+            return launch_cached(s, *pc);
     }
     std::vector<GateOp> gops(nops);
     for (int i = 0; i < nops; ++i) LQ_TRY(make_gate_op(&ops[i], theta, n, &gops[i]));
@@ -1282,6 +1301,19 @@ int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *
         return LQ_OK;
     }
     const int T = std::min(fusion_width(), n);
+    auto pc = std::make_unique<PlanCache>();
+    pc->key = key.copy();
+    pc->T = T;
+    pc->normalize = defer_renorm(gops);
+    // Mapped rounds where every gate has that form (mapped.cu), else op records.
+    MapProgram mp;
+    if (map_plan(gops, n, T, mp)) {
+        pc->mapped = true;
+        pc->map = std::move(mp);
+        free_plan_cache(s);
+        s->plan_cache = pc.release();
+        return launch_cached(s, *static_cast<const PlanCache *>(s->plan_cache));
+    }
     std::vector<int> orig;
     fold_pairs(gops, orig, T);
     std::vector<PlanStep> steps = plan_circuit(gops, n, T);
@@ -1290,106 +1322,71 @@ int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *
     std::vector<double> coef;
     std::vector<PassLaunch> launches;
     encode_steps(steps, gops, T, rounds, fops, coef, launches);
-    if (pp_engine() == 1) {
-        // Kernel records, round by round: a table followed by a pair op in the
-        // same round becomes one record (PC_TPAIR), so the round dispatches once.
-        std::vector<PassOp> pops;
-        pops.reserve(fops.size());
-        for (auto &fr : rounds) {
-            const int b0 = (int)pops.size();
-            for (int o = fr.op_begin; o < fr.op_end; ++o) {
-                const FusedOp &f = fops[o];
-                PassOp p = pass_op(f);
-                if (f.type == F_PAIR) {
-                    p.x0 = coef[f.coef];
-                    p.x1 = coef[f.coef + 1];
-                }
-                if (f.type == F_DTAB && o + 1 < fr.op_end && fops[o + 1].type == F_PAIR &&
-                    fops[o + 1].gmask == 0 && f.gmask == 0) {
-                    const FusedOp &g = fops[o + 1];
-                    p.code = PC_TPAIR + pair_index(g.k0, g.k1) * 4 + (g.cm >> 2);
-                    p.x0 = coef[g.coef];
-                    p.x1 = coef[g.coef + 1];
-                    ++o;  // the pair is part of this record
-                }
-                pops.push_back(p);
+    // Kernel records, round by round: a table followed by a pair op in the
+    // same round becomes one record (PC_TPAIR), so the round dispatches once.
+    std::vector<PassOp> pops;
+    pops.reserve(fops.size());
+    for (auto &fr : rounds) {
+        const int b0 = (int)pops.size();
+        for (int o = fr.op_begin; o < fr.op_end; ++o) {
+            const FusedOp &f = fops[o];
+            PassOp p = pass_op(f);
+            if (f.type == F_PAIR) {
+                p.x0 = coef[f.coef];
+                p.x1 = coef[f.coef + 1];
             }
-            fr.op_begin = b0;
-            fr.op_end = (int)pops.size();
-        }
-        // each thread's tile-local base index, per round (lanes from fill_round)
-        const int nthr = 1 << (T - 4), stride = tb_stride(nthr);
-        std::vector<uint16_t> tb(rounds.size() * stride, 0);
-        for (size_t r = 0; r < rounds.size(); ++r)
-            for (int t = 0; t < nthr; ++t) {
-                int v = 0;
-                for (int j = 0; j < rounds[r].nlane; ++j) v |= ((t >> j) & 1) << rounds[r].lane[j];
-                tb[r * stride + t] = (uint16_t)v;
+            if (f.type == F_DTAB && o + 1 < fr.op_end && fops[o + 1].type == F_PAIR &&
+                fops[o + 1].gmask == 0 && f.gmask == 0) {
+                const FusedOp &g = fops[o + 1];
+                p.code = PC_TPAIR + pair_index(g.k0, g.k1) * 4 + (g.cm >> 2);
+                p.x0 = coef[g.coef];
+                p.x1 = coef[g.coef + 1];
+                ++o;  // the pair is part of this record
             }
-        const size_t rb = rounds.size() * sizeof(FusedRound);
-        const size_t ob = pops.size() * sizeof(PassOp);
-        const size_t cb = coef.size() * sizeof(double);
-        const size_t tbb = tb.size() * sizeof(uint16_t);
-        auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-        LQ_TRY(ensure_prog(s, al(rb) + al(ob) + al(cb) + al(tbb) + 256));
-        char *dp = (char *)s->d_prog;
-        FusedRound *d_rounds = (FusedRound *)dp;
-        PassOp *d_ops = (PassOp *)(dp + al(rb));
-        double *d_coef = (double *)(dp + al(rb) + al(ob));
-        uint16_t *d_tb = (uint16_t *)(dp + al(rb) + al(ob) + al(cb));
-        // The program buffer may still be read by a previous call's kernels.
-        LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
-        if (rb) LQ_CUDA_TRY(cudaMemcpy(d_rounds, rounds.data(), rb, cudaMemcpyHostToDevice));
-        if (ob) LQ_CUDA_TRY(cudaMemcpy(d_ops, pops.data(), ob, cudaMemcpyHostToDevice));
-        if (cb) LQ_CUDA_TRY(cudaMemcpy(d_coef, coef.data(), cb, cudaMemcpyHostToDevice));
-        if (tbb) LQ_CUDA_TRY(cudaMemcpy(d_tb, tb.data(), tbb, cudaMemcpyHostToDevice));
-        auto pc = std::make_unique<PlanCache>();
-        pc->key = std::move(key);
-        pc->T = T;
-        pc->stride = stride;
-        pc->off_ops = (size_t)((char *)d_ops - dp);
-        pc->off_coef = (size_t)((char *)d_coef - dp);
-        pc->off_tb = (size_t)((char *)d_tb - dp);
-        size_t li = 0;
-        for (auto &st : steps) {
-            if (!st.fused) pc->steps.push_back({false, gops[st.gate], PassLaunch{}});
-            else pc->steps.push_back({true, GateOp{}, launches[li++]});
+            pops.push_back(p);
         }
-        free_plan_cache(s);
-        s->plan_cache = pc.release();
-        s->prog_valid = true;
-        return launch_cached(s, *static_cast<const PlanCache *>(s->plan_cache));
+        fr.op_begin = b0;
+        fr.op_end = (int)pops.size();
     }
+    // each thread's tile-local base index, per round (lanes from fill_round)
+    const int nthr = 1 << (T - 4), stride = tb_stride(nthr);
+    std::vector<uint16_t> tb(rounds.size() * stride, 0);
+    for (size_t r = 0; r < rounds.size(); ++r)
+        for (int t = 0; t < nthr; ++t) {
+            int v = 0;
+            for (int j = 0; j < rounds[r].nlane; ++j) v |= ((t >> j) & 1) << rounds[r].lane[j];
+            tb[r * stride + t] = (uint16_t)v;
+        }
     const size_t rb = rounds.size() * sizeof(FusedRound);
-    const size_t ob = fops.size() * sizeof(FusedOp);
+    const size_t ob = pops.size() * sizeof(PassOp);
     const size_t cb = coef.size() * sizeof(double);
+    const size_t tbb = tb.size() * sizeof(uint16_t);
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    LQ_TRY(ensure_prog(s, al(rb) + al(ob) + al(cb) + 256));
+    LQ_TRY(ensure_prog(s, al(rb) + al(ob) + al(cb) + al(tbb) + 256));
     char *dp = (char *)s->d_prog;
     FusedRound *d_rounds = (FusedRound *)dp;
-    FusedOp *d_ops = (FusedOp *)(dp + al(rb));
+    PassOp *d_ops = (PassOp *)(dp + al(rb));
     double *d_coef = (double *)(dp + al(rb) + al(ob));
+    uint16_t *d_tb = (uint16_t *)(dp + al(rb) + al(ob) + al(cb));
     // The program buffer may still be read by a previous call's kernels.
     LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
     if (rb) LQ_CUDA_TRY(cudaMemcpy(d_rounds, rounds.data(), rb, cudaMemcpyHostToDevice));
-    if (ob) LQ_CUDA_TRY(cudaMemcpy(d_ops, fops.data(), ob, cudaMemcpyHostToDevice));
+    if (ob) LQ_CUDA_TRY(cudaMemcpy(d_ops, pops.data(), ob, cudaMemcpyHostToDevice));
     if (cb) LQ_CUDA_TRY(cudaMemcpy(d_coef, coef.data(), cb, cudaMemcpyHostToDevice));
-    LQ_TRY(set_smem_attrs());
-
+    if (tbb) LQ_CUDA_TRY(cudaMemcpy(d_tb, tb.data(), tbb, cudaMemcpyHostToDevice));
+    pc->stride = stride;
+    pc->off_ops = (size_t)((char *)d_ops - dp);
+    pc->off_coef = (size_t)((char *)d_coef - dp);
+    pc->off_tb = (size_t)((char *)d_tb - dp);
     size_t li = 0;
     for (auto &st : steps) {
-        if (!st.fused) {
-            LQ_TRY(launch_gate_op(s, gops[st.gate]));
-            s->last_launches += gops[st.gate].renorm ? 3 : 1;
-            continue;
-        }
-        const PassLaunch &pl = launches[li++];
-        LQ_TRY(launch_pass(s, T, pl.h, d_rounds + pl.round_begin, pl.nrounds, d_ops, d_coef,
-                           pl.mode));
-        s->last_launches += 1;
-        s->last_passes += 1;
+        if (!st.fused) pc->steps.push_back({false, gops[st.gate], PassLaunch{}});
+        else pc->steps.push_back({true, GateOp{}, launches[li++]});
     }
-    return LQ_OK;
+    free_plan_cache(s);
+    s->plan_cache = pc.release();
+    s->prog_valid = true;
+    return launch_cached(s, *static_cast<const PlanCache *>(s->plan_cache));
 }
 
 int apply_block_impl(lq_state *s, int k, const int *qubits, const double *m) {
@@ -1441,7 +1438,7 @@ int apply_block_impl(lq_state *s, int k, const int *qubits, const double *m) {
     LQ_CUDA_TRY(cudaMemcpy(d_ops, &fo, sizeof(FusedOp), cudaMemcpyHostToDevice));
     LQ_CUDA_TRY(cudaMemcpy(d_coef, m, cb, cudaMemcpyHostToDevice));
     LQ_TRY(set_smem_attrs());
-    return launch_pass(s, T, h, d_rounds, 1, d_ops, d_coef, 2);
+    return launch_block_pass(s, T, h, d_rounds, 1, d_ops, d_coef);
 }
 
 }  // namespace lq
@@ -1489,9 +1486,8 @@ int lq_apply_block(lq_state *s, int k, const int *qubits, const double *m) {
     return apply_block_impl(s, k, qubits, m);
 }
 
-static int plan_for(int num_qubits, const lq_gate *ops, int nops, const double *theta,
-                    int ntheta, std::vector<GateOp> &gops, std::vector<PlanStep> &steps,
-                    int &T, std::vector<int> &orig) {
+static int gate_ops(int num_qubits, const lq_gate *ops, int nops, const double *theta, int ntheta,
+                    std::vector<GateOp> &gops) {
     if (nops < 0 || (nops > 0 && !ops)) return set_error(LQ_ERR_INVALID_ARG, "bad op list");
     if (num_qubits < 5 || num_qubits > 36)
         return set_error(LQ_ERR_UNSUPPORTED, "fused planning needs 5..36 qubits");
@@ -1505,6 +1501,15 @@ static int plan_for(int num_qubits, const lq_gate *ops, int nops, const double *
         LQ_TRY(validate_gate(&g, num_qubits, theta ? ntheta : 1 << 30));
         LQ_TRY(make_gate_op(&g, theta ? theta : zero_theta, num_qubits, &gops[i]));
     }
+    return LQ_OK;
+}
+
+// The op-record plan: what circuits without a mapped form run, and what lq_plan_dump
+// writes out.
+static int plan_for(int num_qubits, const lq_gate *ops, int nops, const double *theta,
+                    int ntheta, std::vector<GateOp> &gops, std::vector<PlanStep> &steps,
+                    int &T, std::vector<int> &orig) {
+    LQ_TRY(gate_ops(num_qubits, ops, nops, theta, ntheta, gops));
     T = std::min(fusion_width(), num_qubits);
     fold_pairs(gops, orig, T);
     steps = plan_circuit(gops, num_qubits, T);
@@ -1519,6 +1524,15 @@ int lq_plan_circuit(int num_qubits, const lq_gate *ops, int nops, int *passes, i
     int T;
     LQ_TRY(plan_for(num_qubits, ops, nops, nullptr, 0, gops, steps, T, orig));
     int p = 0, r = 0, s1 = 0;
+    MapProgram mp;
+    std::vector<GateOp> plain;
+    LQ_TRY(gate_ops(num_qubits, ops, nops, nullptr, 0, plain));
+    defer_renorm(plain);
+    if (map_plan(plain, num_qubits, T, mp)) {
+        steps.clear();
+        r = mp.rounds;
+        for (const MapStep &st : mp.steps) ++(st.fused ? p : s1);
+    }
     for (auto &st : steps) {
         if (st.fused) {
             ++p;

@@ -59,6 +59,10 @@ inline uint64_t op_bits(const GateOp &o) {
     return m;
 }
 
+// Whether m (dim x dim), or the op, is unitary to 1e-14.
+bool unitary_matrix(const double *m, int dim);
+bool unitary_op(const GateOp &op);
+
 // Launch the per-gate kernel of op on state s (complex128 or complex64).
 int launch_gate_op(lq_state *s, const GateOp &op);
 

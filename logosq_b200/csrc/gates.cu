@@ -252,6 +252,34 @@ int make_gate_op(const lq_gate *g, const double *theta, int n, GateOp *op) {
     return LQ_OK;
 }
 
+bool unitary_matrix(const double *m, int dim) {
+    for (int r = 0; r < dim; ++r)
+        for (int c = 0; c < dim; ++c) {
+            double re = r == c ? -1.0 : 0.0, im = 0.0;
+            for (int k = 0; k < dim; ++k) {
+                const double *x = m + 2 * (k * dim + r), *y = m + 2 * (k * dim + c);
+                re += x[0] * y[0] + x[1] * y[1];
+                im += x[0] * y[1] - x[1] * y[0];
+            }
+            if (!(std::fabs(re) <= 1e-14 && std::fabs(im) <= 1e-14)) return false;
+        }
+    return true;
+}
+
+bool unitary_op(const GateOp &g) {
+    switch (g.type) {
+    case OP_M1: return unitary_matrix(g.m, 2);
+    case OP_M2: return unitary_matrix(g.m, 4);
+    case OP_DIAG:
+        for (int k = 0; k < 1 << g.npat; ++k)
+            if (!(std::fabs(g.m[2 * k] * g.m[2 * k] + g.m[2 * k + 1] * g.m[2 * k + 1] - 1.0) <=
+                  1e-14))
+                return false;
+        return true;
+    default: return true;  // permutations
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Device kernels, templated on the amplitude type (double2 / float2).
 // ---------------------------------------------------------------------------
