@@ -11,15 +11,22 @@
 // X' (128 x 64) and the block is Y' = X' W' with the real 64 x 64 matrix
 // W' = [[Re U^T, Im U^T], [-Im U^T, Re U^T]] interleaved the same way.
 //
-// Thread m owns GEMM row m, which is also tensor-memory lane m: it splits its
-// row into TF32 hi / lo parts and writes them to tensor memory (tcgen05.st);
-// one elected thread issues 3 x 8 tcgen05.mma (K = 8 each) with A read from
-// tensor memory and B (W' hi / lo, prepared on the host in the swizzled K-major
-// byte order and brought in by one bulk copy) from shared memory, into a
-// 128-lane x 64-column FP32 accumulator; each thread reads its row back with
-// tcgen05.ld and scatters it into the tile.  CTAs are persistent (two per SM:
-// 97 KiB of shared memory and 256 tensor-memory columns each), prefetch their
-// next tile into a second buffer and store finished tiles asynchronously.
+// GEMM row m is also tensor-memory lane m.  Two threads share a row, each with half of
+// its columns: they split them into TF32 hi / lo parts and write them to tensor memory
+// (tcgen05.st); one elected thread issues 3 x 8 tcgen05.mma (K = 8 each) with A read from
+// tensor memory and B (W' hi / lo, prepared on the host in the swizzled K-major byte
+// order) from shared memory, into a 128-lane x 64-column FP32 accumulator; the threads
+// read it back with tcgen05.ld and scatter it into the tile.
+//
+// Bound: per SM a block of a tile takes some 860 cycles of the tensor pipe, 700 issue
+// slots per scheduler and 1000 cycles of shared memory (the tile read and written, B read
+// by the products); its chain split -> products -> read back is some 3000.  So tiles must
+// overlap.  Tensor memory holds 512 columns, and a tile needs 128 for A from the split to
+// the end of its products but 64 for D from there to the read back: three groups of 256
+// threads, each with its tile and its D region, take turns on two A regions.  A CTA per
+// SM is persistent.  One further warp moves tiles through five buffers, another brings
+// the B images (32 KiB) for all groups into two slots, where up to two blocks stay for the
+// whole pass.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -33,23 +40,29 @@
 namespace lq {
 
 constexpr int kTcT = 12;                  // tile bits
-constexpr int kTcThreads = 128;           // thread m owns GEMM row m = TMEM lane m
+constexpr int kTcGroup = 256;             // two threads per GEMM row = TMEM lane
+constexpr int kTcGroups = 3;
+constexpr int kTcThreads = kTcGroups * kTcGroup + 64;  // and two warps that move tiles and B
+constexpr int kTcBuffers = 5;              // tiles in shared memory (one more for one block)
+constexpr int kTcSlots = 2;                // B images
 constexpr uint32_t kTileBytes = 8u << kTcT;  // 32 KiB complex64 tile
 constexpr uint32_t kBBytes = 64 * 64 * 4;    // 16 KiB per B part (hi / lo)
-// shared memory: two tile buffers, B hi + lo, barriers
-constexpr uint32_t kTcSmem = 2 * kTileBytes + 2 * kBBytes + 1024 + 128;
-// tensor memory columns: D (FP32 accumulator) [0,64), A hi [64,128), A lo [128,192)
-constexpr uint32_t kTmemCols = 256;
-constexpr uint32_t kColD = 0, kColAh = 64, kColAl = 128;
+// shared memory: tiles, B images, barriers
+constexpr uint32_t kTcSmem = kTcBuffers * kTileBytes + kTcSlots * 2 * kBBytes + 1024 + 256;
+static_assert(kTcSmem + 1024 <= 227 * 1024, "one CTA per SM");
+// tensor memory columns: two A regions, hi [0,64) and lo [64,128), then the groups' D (FP32
+// accumulator), 64 each
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kColA = 128, kColAl = 64, kColD = 256;
 
 struct TcBlock {
-    int32_t k[5];     // tile-local bit of block bit j (block index bit j)
-    int32_t pad[3];
-    uint32_t row_bits[7];  // tile-local positions of the 7 row bits
-    uint32_t pad2;
-    uint64_t b_offset;  // offset (bytes) of this block's 32 KiB B image (hi then lo)
-    uint32_t col_bits[32];  // tile-local index bits of block column c (its 5 bits placed)
+    uint32_t row[7];    // byte offset in the tile of each row bit
+    uint32_t col[5];    // and of each block index bit
+    uint32_t pair;      // block bit 0 is tile bit 0: columns 2c, 2c+1 are 16 bytes
+    uint32_t b_offset;  // of the block's 32 KiB B image (hi then lo), in bytes / 16
+    uint32_t pad[2];
 };
+static_assert(sizeof(TcBlock) == 64, "read in four pieces");
 
 static bool tc_restore_norm() {
     static const int v = [] {
@@ -71,7 +84,8 @@ __device__ __forceinline__ uint32_t tc_smem_u32(const void *p) {
 
 // Byte offset of complex64 tile element l in the TMA 128-byte-swizzled tile:
 // 128-byte rows hold 16 amplitudes (bits 0-3); 16-byte chunks hold 2.
-__device__ __forceinline__ uint32_t tile_off(uint32_t l) {
+// Linear over XOR.
+__host__ __device__ __forceinline__ uint32_t tile_off(uint32_t l) {
     const uint32_t row = l >> 4, chunk = (l & 15) >> 1;
     return row * 128 + ((chunk ^ (row & 7)) << 4) + ((l & 1) << 3);
 }
@@ -145,255 +159,370 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-// Persistent CTAs (two per SM), each walking tiles t = blockIdx.x, +gridDim.x.
-// Per tile: TMA load (prefetched one tile ahead into the other buffer), then per
-// 5-qubit block: B image (one bulk copy), A split into TF32 hi / lo written to
-// tensor memory by the owning threads (row m = TMEM lane m), 3 x 8 tcgen05.mma
-// with A from tensor memory, tcgen05.ld of the 128 x 64 FP32 result and scatter
-// into the tile; finally an asynchronous TMA store, waited for only before its
-// buffer is reloaded.
-__global__ void __launch_bounds__(kTcThreads, 2)
+__device__ __forceinline__ float4 lds4(uint32_t a) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 lds2(uint32_t a) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts4(uint32_t a, float x, float y, float z, float w) {
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x), "f"(y), "f"(z),
+                 "f"(w)
+                 : "memory");
+}
+__device__ __forceinline__ void sts2(uint32_t a, float x, float y) {
+    asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y) : "memory");
+}
+
+// Byte offset in the tile of the thread's column c (0..15 of its half), over XOR, from its
+// row's first.
+struct TcCols {
+    uint32_t b[4];
+    __device__ __forceinline__ uint32_t off(int c) const {
+        return ((c & 1) ? b[0] : 0u) ^ ((c & 2) ? b[1] : 0u) ^ ((c & 4) ? b[2] : 0u) ^
+               ((c & 8) ? b[3] : 0u);
+    }
+};
+
+template <bool PAIR>
+__device__ __forceinline__ void tc_split(uint32_t tile, uint32_t at, const TcCols &cols,
+                                         uint32_t tm) {
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float hi[16], lo[16];
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            float x[4];
+            if (PAIR) {
+                const float4 v = lds4(tile + (at ^ cols.off(q * 8 + c)));
+                x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+            } else {
+                const float2 v = lds2(tile + (at ^ cols.off(q * 8 + c)));
+                const float2 w = lds2(tile + (at ^ cols.off(q * 8 + c + 1)));
+                x[0] = v.x, x[1] = v.y, x[2] = w.x, x[3] = w.y;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float hx = to_tf32(x[u]);
+                hi[2 * c + u] = hx;
+                lo[2 * c + u] = to_tf32(x[u] - hx);
+            }
+        }
+        tmem_st16(tm + q * 16, hi);
+        tmem_st16(tm + kColAl + q * 16, lo);
+    }
+}
+
+template <bool PAIR>
+__device__ __forceinline__ void tc_back(uint32_t tile, uint32_t at, const TcCols &cols,
+                                        uint32_t tm) {
+    float d[2][16];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) tmem_ld16(tm + q * 16, d[q]);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(d[q][i]));  // (read after the wait)
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            const uint32_t p = tile + (at ^ cols.off(q * 8 + c));
+            if (PAIR) {
+                sts4(p, d[q][2 * c], d[q][2 * c + 1], d[q][2 * c + 2], d[q][2 * c + 3]);
+            } else {
+                sts2(p, d[q][2 * c], d[q][2 * c + 1]);
+                sts2(tile + (at ^ cols.off(q * 8 + c + 1)), d[q][2 * c + 2], d[q][2 * c + 3]);
+            }
+        }
+}
+
+// Whether any thread of the group says so: the same answer for all of them.
+__device__ __forceinline__ bool tc_any(int g, bool x) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)x), "r"(1 + g), "n"(kTcGroup)
+        : "memory");
+    return r != 0;
+}
+
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r));
+    return r != 0;
+}
+
+// The CTA's tiles are blockIdx.x + q gridDim.x, q = 0, 1, ...; group q % 3 takes tile q in
+// buffer q mod their number.  Step s = 3 j + g is the j-th block of group g in all its
+// tiles; it uses A region s % 2, when the products of step s - 2 are done.  A group without
+// a tile in the last round goes through its steps without work.
+// Every barrier is awaited, phase by phase, by the same threads: a phase's parity alone
+// does not tell it from the one two before or after.  So there are two barriers per group
+// and purpose, in turn: a group's next step, or tile, may be done before the last is seen.
+// Waits are bounded; one that ran out is carried to the group's next barrier, where all its
+// threads leave.  The others of the CTA then run into their own limits.
+// The operands of the products are the same for the warp and known to be (shfl): else each
+// took a loop over the warp's values, 83 cycles instead of the tensor pipe's 36.
+__global__ void __launch_bounds__(kTcThreads, 1)
     k_tc_pass(const __grid_constant__ CUtensorMap tmap, int32_t h, int32_t ntiles,
               const TcBlock *__restrict__ blocks, int nblocks,
               const unsigned char *__restrict__ bimg, unsigned *__restrict__ flag) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char *tiles = base;                       // 2 x 32 KiB
-    unsigned char *b_hi = tiles + 2 * kTileBytes;      // 16 KiB, then b_lo
-    unsigned char *b_lo = b_hi + kBBytes;
-    uint64_t *bars = (uint64_t *)(b_lo + kBBytes);     // [0],[1] tile loads, [2] B, [3] MMA
-    uint32_t *tmem_slot = (uint32_t *)(bars + 4);
-    int *s_abort = (int *)(tmem_slot + 1);
-    const uint32_t bar_load0 = tc_smem_u32(&bars[0]);
-    const uint32_t bar_b = tc_smem_u32(&bars[2]);
-    const uint32_t bar_mma = tc_smem_u32(&bars[3]);
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t tiles = (tc_smem_u32(smem_raw) + 1023u) & ~1023u;
+    // (slots from the end: a pass of one block has the other for a sixth tile)
+    const uint32_t images = tiles + (kTcBuffers + kTcSlots - 1) * kTileBytes;  // B: hi, then lo
+    const uint32_t bars = images + kTileBytes;
+    const uint32_t bar_load = bars;                          // [2][group]: a tile is there
+    const uint32_t bar_mma = bar_load + 16 * kTcGroups;      // [2][group]: products are done
+    const uint32_t bar_done = bar_mma + 16 * kTcGroups;      // [2][group]: a tile is finished
+    const uint32_t bar_full = bar_done + 16 * kTcGroups;     // [slot]: the image is there
+    const uint32_t bar_free = bar_full + 8 * kTcSlots;       // [slot]: all groups are done
+    const int nbuf = nblocks == 1 ? kTcBuffers + 1 : kTcBuffers;
+    __shared__ uint32_t tmem_slot;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int32_t zero = 0;
+    const bool resident = nblocks <= kTcSlots;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                         tc_smem_u32(tmem_slot)),
+                         tc_smem_u32(&tmem_slot)),
                      "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < 4; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(tc_smem_u32(&bars[i])),
-                         "r"(1)
+        constexpr int ones = 6 * kTcGroups + kTcSlots;
+        for (int i = 0; i < ones + kTcSlots; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * i),
+                         "r"(i < ones ? 1 : kTcGroups)
                          : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *s_abort = 0;
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = *tmem_slot;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-
-    auto issue_load = [&](int t, int buf) {
-        const int32_t c1 = t & ((1 << (h - 4)) - 1), c3 = t >> (h - 4);
-        const uint32_t bar = bar_load0 + 8u * buf;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                     "r"(kTileBytes)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(tc_smem_u32(tiles + buf * kTileBytes)),
-            "l"((uint64_t)&tmap), "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(bar)
-            : "memory");
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    const int mine = (int)blockIdx.x < ntiles
+                         ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles
+    const int rounds = (mine + kTcGroups - 1) / kTcGroups;
+    // event k of group g (a tile or a step) on one of its two barriers
+    auto of = [&](uint32_t bar, int g, int k) { return bar + 8u * (g + kTcGroups * (k & 1)); };
+    auto seen = [&](uint32_t bar, int g, int k) {
+        return tc_wait(of(bar, g, k), (uint32_t)(k >> 1) & 1u);
+    };
+    auto arrive = [&](uint32_t bar) {
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
     };
 
-    // B hi + lo of block bi: one 32 KiB bulk copy of the host-prepared swizzled image
-    auto issue_b = [&](int bi) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar_b),
-                     "r"(2 * kBBytes)
-                     : "memory");
-        asm volatile(
-            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes"
-            " [%0], [%1], %2, [%3];" ::"r"(tc_smem_u32(b_hi)),
-            "l"((uint64_t)(bimg + blocks[bi].b_offset)), "r"(2 * kBBytes), "r"(bar_b)
-            : "memory");
-    };
-
-    uint32_t load_phase[2] = {0u, 0u}, b_phase = 0u, mma_phase = 0u;
-    bool load_pending[2] = {false, false};  // thread 0: a tile load not yet waited for
-    bool mma_pending = false, b_pending = false;
-    if (tid == 0 && (int)blockIdx.x < ntiles && nblocks > 0) {
-        issue_b(0);
-        b_pending = true;
-    }
-    int buf = 0;
-    if (tid == 0 && (int)blockIdx.x < ntiles) {
-        issue_load(blockIdx.x, 0);
-        load_pending[0] = true;
-    }
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        if (!tc_wait(bar_load0 + 8u * buf, load_phase[buf])) atomicExch(s_abort, 1);
-        load_phase[buf] ^= 1u;
-        if (tid == 0) load_pending[buf] = false;
-        __syncthreads();
-        if (*s_abort) break;
-        const int tn = t + gridDim.x;
-        if (tid == 0 && tn < ntiles) {
-            // the other buffer's store (previous tile) must have left shared memory
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            issue_load(tn, buf ^ 1);
-            load_pending[buf ^ 1] = true;
+    if (warp == kTcGroups * kTcGroup / 32) {
+        // ---- the B images, in the order of use
+        if ((tid & 31) == 0) {
+            const int total = nblocks * (resident ? std::min(rounds, 1) : rounds);
+            int slot = 0, use = 0, bi = 0, sent = 0;
+            bool bad = false;
+            for (; sent < total; ++sent) {
+                if (use > 0 && !tc_wait(bar_free + 8u * slot, (uint32_t)(use - 1) & 1u)) {
+                    bad = true;
+                    break;
+                }
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                 bar_full + 8u * slot),
+                             "r"(2 * kBBytes)
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes"
+                    " [%0], [%1], %2, [%3];" ::"r"(images - slot * 2 * kBBytes),
+                    "l"((uint64_t)(bimg + ((uint64_t)blocks[bi].b_offset << 4))),
+                    "r"(2 * kBBytes), "r"(bar_full + 8u * slot)
+                    : "memory");
+                if (++bi == nblocks) bi = 0;
+                if (++slot == kTcSlots) slot = 0, ++use;
+            }
+            // the copies have landed before the CTA's memory is released
+            for (int k = std::max(0, sent - kTcSlots); k < sent; ++k)
+                bad |= !tc_wait(bar_full + 8u * (k % kTcSlots), (uint32_t)(k / kTcSlots) & 1u);
+            if (bad) atomicOr(flag, kFlagTimeout);
         }
-        unsigned char *tile = tiles + buf * kTileBytes;
-        const uint32_t tile_a = tc_smem_u32(tile);
-        for (int bi = 0; bi < nblocks; ++bi) {
-            const TcBlock &blk = blocks[bi];
-            // (this block's B image was requested when the previous block's MMAs
-            // had finished reading the buffer, or before the first tile)
-            // A row m = tid: the block's 32 complex entries, split hi / lo into TMEM
-            uint32_t lbase = 0;
-#pragma unroll
-            for (int j = 0; j < 7; ++j) lbase |= (((uint32_t)tid >> j) & 1u) << blk.row_bits[j];
-            // tile_off is linear over XOR on disjoint bits: the offset of column c is
-            // the XOR of the offsets of its five block bits (five loads, not 32)
-            const uint32_t rowoff = tile_off(lbase);
-            const uint32_t cb0 = tile_off(1u << blk.k[0]), cb1 = tile_off(1u << blk.k[1]),
-                           cb2 = tile_off(1u << blk.k[2]), cb3 = tile_off(1u << blk.k[3]),
-                           cb4 = tile_off(1u << blk.k[4]);
-            auto col_off = [&](int c) {
-                return ((c & 1) ? cb0 : 0u) ^ ((c & 2) ? cb1 : 0u) ^ ((c & 4) ? cb2 : 0u) ^
-                       ((c & 8) ? cb3 : 0u) ^ ((c & 16) ? cb4 : 0u);
+    } else if (warp == kTcGroups * kTcGroup / 32 + 1) {
+        // ---- the tiles: a finished one is stored, and its buffer loaded again
+        if ((tid & 31) == 0) {
+            auto coords = [&](int q, int32_t &c1, int32_t &c3) {
+                const int t = (int)blockIdx.x + q * (int)gridDim.x;
+                c1 = t & ((1 << (h - 4)) - 1), c3 = t >> (h - 4);
             };
-            // Block bit 0 on tile bit 0: columns 2c, 2c+1 share a 16-byte chunk
-            // (one 128-bit access for both, and the lane bits then cover the
-            // chunk slots without bank conflicts).
-            const bool pair = blk.k[0] == 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float hi[16], lo[16];
-#pragma unroll
-                for (int c = 0; c < 8; c += 2) {
-                    float4 v;
-                    if (pair) {
-                        v = *(const float4 *)(tile + (rowoff ^ col_off(q * 8 + c)));
-                    } else {
-                        const float2 v0 = *(const float2 *)(tile + (rowoff ^ col_off(q * 8 + c)));
-                        const float2 v1 =
-                            *(const float2 *)(tile + (rowoff ^ col_off(q * 8 + c + 1)));
-                        v = make_float4(v0.x, v0.y, v1.x, v1.y);
+            bool bad = false;
+            int asked = 0;
+            for (int q = 0; q < mine + nbuf; ++q) {
+                const uint32_t buf = tiles + (uint32_t)(q % nbuf) * kTileBytes;
+                int32_t c1, c3;
+                if (q >= nbuf && q - nbuf < mine) {
+                    if (!seen(bar_done, (q - nbuf) % kTcGroups, (q - nbuf) / kTcGroups)) {
+                        bad = true;
+                        break;
                     }
-                    const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const float hx = to_tf32(x[u]);
-                        hi[2 * c + u] = hx;
-                        lo[2 * c + u] = to_tf32(x[u] - hx);
-                    }
-                }
-                tmem_st16(lane_base + kColAh + q * 16, hi);
-                tmem_st16(lane_base + kColAl + q * 16, lo);
-            }
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (tid == 0) {
-                if (!tc_wait(bar_b, b_phase)) {
-                    atomicExch(s_abort, 1);
-                } else {
-                    b_pending = false;
-                    const uint32_t bh = tc_smem_u32(b_hi), bl = tc_smem_u32(b_lo);
-#pragma unroll
-                    for (int prod = 0; prod < 3; ++prod) {
-                        // hi.Bhi + hi.Blo + lo.Bhi
-                        const uint32_t acol = prod == 2 ? kColAl : kColAh;
-                        const uint32_t bsrc = prod == 1 ? bl : bh;
-#pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) {
-                            const uint32_t boff = (kk >> 2) * (64 * 128) + (kk & 3) * 32;
-                            const uint64_t db = make_sdesc(bsrc + boff, 1024);
-                            const uint32_t acc = (prod | kk) ? 1u : 0u;
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\t"
-                                "setp.ne.b32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::
-                                    "r"(tmem + kColD),
-                                "r"(tmem + acol + kk * 8), "l"(db), "r"(kIdesc), "r"(acc)
-                                : "memory");
-                        }
-                    }
+                    coords(q - nbuf, c1, c3);
                     asm volatile(
-                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
-                        "[%0];" ::"r"(bar_mma)
+                        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group"
+                        " [%0, {%1, %2, %3, %4}], [%5];" ::"l"((uint64_t)&tmap),
+                        "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(buf)
                         : "memory");
-                    mma_pending = true;
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
-                b_phase ^= 1u;
-            }
-            __syncthreads();
-            if (*s_abort) break;
-            // every thread decides to stop only after the barrier, so the CTA
-            // leaves the loop together
-            if (!tc_wait(bar_mma, mma_phase)) atomicExch(s_abort, 1);
-            __syncthreads();
-            if (*s_abort) break;
-            mma_phase ^= 1u;
-            if (tid == 0) {
-                mma_pending = false;
-                // the MMAs have read B: request the next block's image now, so the
-                // copy overlaps this block's readback and the next block's split
-                const int nb = bi + 1 < nblocks ? bi + 1 : 0;
-                if (bi + 1 < nblocks || t + (int)gridDim.x < ntiles) {
-                    issue_b(nb);
-                    b_pending = true;
+                if (q < mine) {
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    const uint32_t bar = of(bar_load, q % kTcGroups, q / kTcGroups);
+                    coords(q, c1, c3);
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                                 "r"(kTileBytes)
+                                 : "memory");
+                    asm volatile(
+                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx"
+                        "::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(buf),
+                        "l"((uint64_t)&tmap), "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(bar)
+                        : "memory");
+                    asked = q + 1;
                 }
             }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // D row m = tid back into the tile
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                float d[16];
-                tmem_ld16(lane_base + kColD + q * 16, d);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                for (int c = 0; c < 8; c += 2) {
-                    unsigned char *p0 = tile + (rowoff ^ col_off(q * 8 + c));
-                    if (pair) {
-                        *(float4 *)p0 = make_float4(d[2 * c], d[2 * c + 1], d[2 * c + 2],
-                                                    d[2 * c + 3]);
-                    } else {
-                        *(float2 *)p0 = make_float2(d[2 * c], d[2 * c + 1]);
-                        *(float2 *)(tile + (rowoff ^ col_off(q * 8 + c + 1))) =
-                            make_float2(d[2 * c + 2], d[2 * c + 3]);
+            if (bad) {
+                atomicOr(flag, kFlagTimeout);
+                for (int q = std::max(0, asked - nbuf); q < asked; ++q)
+                    seen(bar_load, q % kTcGroups, q / kTcGroups);
+            }
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        }
+    } else {
+        const int g = warp / (kTcGroup / 32), gtid = tid & (kTcGroup - 1);
+        const int half = gtid >> 7, row = gtid & 127;
+        const uint32_t lane = ((uint32_t)(row & ~31) << 16) + 32u * half;
+        const uint32_t tm_d = tmem + kColD + 64u * g;
+        // step s - 2: of the next group but one, a step earlier unless that is group 0
+        const int before = (g + 1) % kTcGroups, later = g >= 2 ? 0 : 1;
+        int slot = 0;
+        uint32_t full_phase = 0;
+        int step = 0;
+        auto next_slot = [&] {
+            if (++slot == (resident ? nblocks : kTcSlots)) slot = 0, full_phase ^= resident ? 0u : 1u;
+        };
+        bool bad = false;
+        const uint4 *desc = (const uint4 *)blocks;
+        for (int j = 0; j < rounds; ++j) {
+            const int q = j * kTcGroups + g;
+            if (q >= mine) {  // (the last round)
+                if (gtid == 0)
+                    for (int bi = 0; bi < nblocks; ++bi, ++step) {
+                        if (step >= later && !seen(bar_mma, before, step - later)) break;
+                        if (!resident) {
+                            if (!tc_wait(bar_full + 8u * slot, full_phase)) break;
+                            arrive(bar_free + 8u * slot);
+                            next_slot();
+                        }
+                        arrive(of(bar_mma, g, step));
                     }
-                }
+                break;
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
+            const uint32_t tile = tiles + (uint32_t)(q % nbuf) * kTileBytes;
+            bad = !seen(bar_load, g, j);
+            uint4 d0 = __ldg(desc), d1 = __ldg(desc + 1), d2 = __ldg(desc + 2), d3 = __ldg(desc + 3);
+            for (int bi = 0; bi < nblocks; ++bi, ++step) {
+                auto on = [&](int j) { return 0u - ((uint32_t)(row >> j) & 1u); };
+                const uint32_t at = (d0.x & on(0)) ^ (d0.y & on(1)) ^ (d0.z & on(2)) ^
+                                    (d0.w & on(3)) ^ (d1.x & on(4)) ^ (d1.y & on(5)) ^
+                                    (d1.z & on(6)) ^ (half ? d2.w : 0u);
+                const TcCols cols{{d1.w, d2.x, d2.y, d2.z}};
+                const bool pair = d3.x != 0;
+                const uint32_t tm_a = tmem + kColA * ((step + g) & 1);
+                if (step >= later) bad |= !seen(bar_mma, before, step - later);
+                __syncwarp();  // the .aligned instructions want the warp together
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (pair) tc_split<true>(tile, at, cols, tm_a + lane);
+                else tc_split<false>(tile, at, cols, tm_a + lane);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(kTcGroup) : "memory");
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (warp == g * (kTcGroup / 32)) {
+                    bad |= !tc_wait(bar_full + 8u * slot, full_phase);
+                    const uint32_t bh = images - slot * 2 * kBBytes;
+                    const uint64_t d64 = make_sdesc(bh, 1024);
+                    const uint32_t dl = __shfl_sync(0xffffffffu, (uint32_t)d64, 0);
+                    const uint32_t dhi = __shfl_sync(0xffffffffu, (uint32_t)(d64 >> 32), 0);
+                    const uint32_t ta = __shfl_sync(0xffffffffu, tm_a, 0);
+                    const uint32_t done = __shfl_sync(0xffffffffu, of(bar_mma, g, step), 0);
+                    const uint32_t freed = __shfl_sync(0xffffffffu, bar_free + 8u * slot, 0);
+                    if (!__any_sync(0xffffffffu, bad) && tc_elect()) {
+#pragma unroll
+                        for (int prod = 0; prod < 3; ++prod) {
+                            // hi.Bhi + hi.Blo + lo.Bhi
+                            const uint32_t acol = prod == 2 ? kColAl : 0u;
+#pragma unroll
+                            for (int kk = 0; kk < 8; ++kk) {
+                                const uint32_t boff =
+                                    (prod == 1 ? kBBytes : 0u) + (kk >> 2) * (64 * 128) + (kk & 3) * 32;
+                                const uint64_t db = (uint64_t)dhi << 32 | (dl + (boff >> 4));
+                                const uint32_t acc = (prod | kk) ? 1u : 0u;
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\t"
+                                    "setp.ne.b32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::
+                                        "r"(tm_d),
+                                    "r"(ta + acol + kk * 8), "l"(db), "r"(kIdesc), "r"(acc)
+                                    : "memory");
+                            }
+                        }
+                        asm volatile(
+                            "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 "
+                            "[%0];" ::"r"(done)
+                            : "memory");
+                        if (!resident)
+                            asm volatile(
+                                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster"
+                                ".b64 [%0];" ::"r"(freed)
+                                : "memory");
+                    }
+                    __syncwarp();
+                }
+                // (the next block's descriptor, while the products run)
+                const uint4 *dn = desc + 4 * (bi + 1 < nblocks ? bi + 1 : 0);
+                d0 = __ldg(dn), d1 = __ldg(dn + 1), d2 = __ldg(dn + 2), d3 = __ldg(dn + 3);
+                bad |= !seen(bar_mma, g, step);
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (pair) tc_back<true>(tile, at, cols, tm_d + lane);
+                else tc_back<false>(tile, at, cols, tm_d + lane);
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (bi + 1 == nblocks) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                bad = tc_any(g, bad);
+                if (bad) break;
+                next_slot();
+            }
+            if (bad) break;
+            if (gtid == 0) arrive(of(bar_done, g, j));
         }
-        if (*s_abort) break;
-        // tile -> HBM (asynchronous; waited for before this buffer is reloaded)
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        if (tid == 0) {
-            const int32_t c1 = t & ((1 << (h - 4)) - 1), c3 = t >> (h - 4);
-            asm volatile(
-                "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group"
-                " [%0, {%1, %2, %3, %4}], [%5];" ::"l"((uint64_t)&tmap),
-                "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(tile_a)
-                : "memory");
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        }
-        buf ^= 1;
-    }
-    if (tid == 0) {
-        if (*s_abort) {
+        if (bad && gtid == 0) {
             atomicOr(flag, kFlagTimeout);
-            // let work in flight finish before the CTA's memory is released
-            if (mma_pending) tc_wait(bar_mma, mma_phase);
-            if (b_pending) tc_wait(bar_b, b_phase);
-            for (int b = 0; b < 2; ++b)
-                if (load_pending[b]) tc_wait(bar_load0 + 8u * b, load_phase[b]);
+            // let products in flight finish before the CTA's memory is released
+            seen(bar_mma, g, step);
         }
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -442,7 +571,7 @@ static int tc_tile_map(CUtensorMap *map, void *d, int n, int h) {
 
 using cd = std::complex<double>;
 
-// SM count of the current device (persistent grid: two CTAs per SM).
+// SM count of the current device (persistent grid: one CTA per SM).
 static int tc_sm_count() {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
@@ -661,12 +790,13 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
                     W[2 * c + 1][2 * r + 1] = U[r][c].real();
                 }
             TcBlock tb{};
-            for (int j = 0; j < 5; ++j) tb.k[j] = local_pos(gbit[j], st.pass.h);
-            for (int c = 0; c < 32; ++c) {
-                tb.col_bits[c] = 0;
-                for (int j = 0; j < 5; ++j) tb.col_bits[c] |= (uint32_t)((c >> j) & 1) << tb.k[j];
+            int k[5];
+            for (int j = 0; j < 5; ++j) {
+                k[j] = local_pos(gbit[j], st.pass.h);
+                tb.col[j] = tile_off(1u << k[j]);
             }
-            // Row bits: thread m's bit j goes to tile bit row_bits[j].  The row order
+            tb.pair = k[0] == 0;
+            // Row bits: thread m's bit j goes to the tile bit order[j].  The row order
             // is free (each thread writes back the row it read), so the five lane
             // bits (j < 5) take tile bits whose 8-byte bank slots in the swizzled
             // tile are linearly independent: slot(l) = (l0, l1^l4, l2^l5, l3^l6), so
@@ -675,7 +805,7 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
             std::vector<int> free_bits;
             for (int l = 0; l < kTcT; ++l) {
                 bool inb = false;
-                for (int j = 0; j < 5; ++j) inb |= tb.k[j] == l;
+                for (int j = 0; j < 5; ++j) inb |= k[j] == l;
                 if (!inb) free_bits.push_back(l);
             }
             auto slot_vec = [](int b) { return b < 7 ? 1u << (b < 4 ? b : b - 3) : 0u; };
@@ -693,10 +823,10 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
             }
             for (int b : free_bits)
                 if (std::find(order.begin(), order.end(), b) == order.end()) order.push_back(b);
-            for (int j = 0; j < 7; ++j) tb.row_bits[j] = (uint32_t)order[j];
-            tb.b_offset = bimg.size();
+            for (int j = 0; j < 7; ++j) tb.row[j] = tile_off(1u << order[j]);
+            tb.b_offset = (uint32_t)(bimg.size() >> 4);
             bimg.resize(bimg.size() + 2 * kBBytes);
-            write_b_image(W, bimg.data() + tb.b_offset, bimg.data() + tb.b_offset + kBBytes);
+            write_b_image(W, bimg.data() + bimg.size() - 2 * kBBytes, bimg.data() + bimg.size() - kBBytes);
             blocks.push_back(tb);
         }
         step_pass[si] = (int)passes.size();
@@ -736,7 +866,7 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
         LQ_TRY(tc_tile_map(&map, s->d, n, tp.h));
         const int ntiles = 1 << (n - kTcT);
         prof_begin(s->stream, kProfTc);
-        k_tc_pass<<<std::min(ntiles, 2 * tc_sm_count()), kTcThreads, kTcSmem, s->stream>>>(
+        k_tc_pass<<<std::min(ntiles, tc_sm_count()), kTcThreads, kTcSmem, s->stream>>>(
             map, tp.h, ntiles, d_blocks + tp.block_begin, tp.nblocks, d_bimg, s->d_flag);
         prof_end(s->stream, kProfTc);
         LQ_CUDA_TRY(cudaGetLastError());
