@@ -22,9 +22,9 @@
 // slots per scheduler and 1000 cycles of shared memory (the tile read and written, B read
 // by the products); its chain split -> products -> read back is some 3000.  So tiles must
 // overlap.  Tensor memory holds 512 columns, and a tile needs 128 for A from the split to
-// the end of its products but 64 for D from there to the read back: three groups of 256
-// threads, each with its tile and its D region, take turns on two A regions.  A CTA per
-// SM is persistent.  One further warp moves tiles through five buffers, another brings
+// the end of its products and 64 for D from their start to the read back: three groups of
+// 256 threads, each with its tile and its A region, take turns on two D regions.  (Two A
+// regions and three of D: 3 % slower.)  A CTA per SM is persistent.  One further warp moves tiles through five buffers, another brings
 // the B images (32 KiB) for all groups into two slots, where up to two blocks stay for the
 // whole pass.
 #include <cuda.h>
@@ -50,10 +50,10 @@ constexpr uint32_t kBBytes = 64 * 64 * 4;    // 16 KiB per B part (hi / lo)
 // shared memory: tiles, B images, barriers
 constexpr uint32_t kTcSmem = kTcBuffers * kTileBytes + kTcSlots * 2 * kBBytes + 1024 + 256;
 static_assert(kTcSmem + 1024 <= 227 * 1024, "one CTA per SM");
-// tensor memory columns: two A regions, hi [0,64) and lo [64,128), then the groups' D (FP32
+// tensor memory columns: the groups' A, hi [0,64) and lo [64,128), then two D regions (FP32
 // accumulator), 64 each
 constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColA = 128, kColAl = 64, kColD = 256;
+constexpr uint32_t kColA = 128, kColAl = 64, kColD = 384;
 
 struct TcBlock {
     uint32_t row[7];    // byte offset in the tile of each row bit
@@ -82,11 +82,13 @@ __device__ __forceinline__ uint32_t tc_smem_u32(const void *p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-// Byte offset of complex64 tile element l in the TMA 128-byte-swizzled tile:
-// 128-byte rows hold 16 amplitudes (bits 0-3); 16-byte chunks hold 2.
-// Linear over XOR.
+// Byte offset of complex64 tile element l in the TMA 128-byte-swizzled tile: 128-byte rows
+// hold 16 amplitudes (bits 0-3), 16-byte chunks hold 2; the row's number has tile bits
+// 9-11 lowest, so that these are the ones that the swizzle adds to the chunk.  A block on
+// neighbouring low bits then leaves its rows on different banks (with bits 4-6 there, a
+// block on bits 0-4 or 1-5 had up to four-way conflicts).  Linear over XOR.
 __host__ __device__ __forceinline__ uint32_t tile_off(uint32_t l) {
-    const uint32_t row = l >> 4, chunk = (l & 15) >> 1;
+    const uint32_t row = (l >> 9) | (((l >> 4) & 31) << 3), chunk = (l & 15) >> 1;
     return row * 128 + ((chunk ^ (row & 7)) << 4) + ((l & 1) << 3);
 }
 
@@ -192,37 +194,49 @@ struct TcCols {
 };
 
 template <bool PAIR>
-__device__ __forceinline__ void tc_split(uint32_t tile, uint32_t at, const TcCols &cols,
-                                         uint32_t tm) {
+__device__ __forceinline__ void tc_read(uint32_t tile, uint32_t at, const TcCols &cols,
+                                        float (&x)[32]) {
+#pragma unroll
+    for (int c = 0; c < 16; c += 2) {
+        if (PAIR) {
+            const float4 v = lds4(tile + (at ^ cols.off(c)));
+            x[2 * c] = v.x, x[2 * c + 1] = v.y, x[2 * c + 2] = v.z, x[2 * c + 3] = v.w;
+        } else {
+            const float2 v = lds2(tile + (at ^ cols.off(c)));
+            const float2 w = lds2(tile + (at ^ cols.off(c + 1)));
+            x[2 * c] = v.x, x[2 * c + 1] = v.y, x[2 * c + 2] = w.x, x[2 * c + 3] = w.y;
+        }
+    }
+}
+
+__device__ __forceinline__ void tc_split(const float (&x)[32], uint32_t tm) {
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
         float hi[16], lo[16];
 #pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-            float x[4];
-            if (PAIR) {
-                const float4 v = lds4(tile + (at ^ cols.off(q * 8 + c)));
-                x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
-            } else {
-                const float2 v = lds2(tile + (at ^ cols.off(q * 8 + c)));
-                const float2 w = lds2(tile + (at ^ cols.off(q * 8 + c + 1)));
-                x[0] = v.x, x[1] = v.y, x[2] = w.x, x[3] = w.y;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float hx = to_tf32(x[u]);
-                hi[2 * c + u] = hx;
-                lo[2 * c + u] = to_tf32(x[u] - hx);
-            }
+        for (int u = 0; u < 16; ++u) {
+            hi[u] = to_tf32(x[16 * q + u]);
+            lo[u] = to_tf32(x[16 * q + u] - hi[u]);
         }
         tmem_st16(tm + q * 16, hi);
         tmem_st16(tm + kColAl + q * 16, lo);
     }
 }
 
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r));
+    return r != 0;
+}
+
+// The row's half from D, which is free for other products then (bar), into the tile.
 template <bool PAIR>
 __device__ __forceinline__ void tc_back(uint32_t tile, uint32_t at, const TcCols &cols,
-                                        uint32_t tm) {
+                                        uint32_t tm, uint32_t bar) {
     float d[2][16];
 #pragma unroll
     for (int q = 0; q < 2; ++q) tmem_ld16(tm + q * 16, d[q]);
@@ -231,6 +245,8 @@ __device__ __forceinline__ void tc_back(uint32_t tile, uint32_t at, const TcCols
     for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int i = 0; i < 16; ++i) asm volatile("" : "+f"(d[q][i]));  // (read after the wait)
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    if (tc_elect()) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 #pragma unroll
     for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -259,20 +275,10 @@ __device__ __forceinline__ bool tc_any(int g, bool x) {
     return r != 0;
 }
 
-__device__ __forceinline__ bool tc_elect() {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "elect.sync _|p, 0xffffffff;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(r));
-    return r != 0;
-}
-
 // The CTA's tiles are blockIdx.x + q gridDim.x, q = 0, 1, ...; group q % 3 takes tile q in
 // buffer q mod their number.  Step s = 3 j + g is the j-th block of group g in all its
-// tiles; it uses A region s % 2, when the products of step s - 2 are done.  A group without
-// a tile in the last round goes through its steps without work.
+// tiles; it uses D region s % 2, when that of step s - 2 was read.  A group without a tile in
+// the last round goes through its steps without work.
 // Every barrier is awaited, phase by phase, by the same threads: a phase's parity alone
 // does not tell it from the one two before or after.  So there are two barriers per group
 // and purpose, in turn: a group's next step, or tile, may be done before the last is seen.
@@ -291,7 +297,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const uint32_t bars = images + kTileBytes;
     const uint32_t bar_load = bars;                          // [2][group]: a tile is there
     const uint32_t bar_mma = bar_load + 16 * kTcGroups;      // [2][group]: products are done
-    const uint32_t bar_done = bar_mma + 16 * kTcGroups;      // [2][group]: a tile is finished
+    const uint32_t bar_read = bar_mma + 16 * kTcGroups;      // [2][group]: and D was read
+    const uint32_t bar_done = bar_read + 16 * kTcGroups;     // [2][group]: a tile is finished
     const uint32_t bar_full = bar_done + 16 * kTcGroups;     // [slot]: the image is there
     const uint32_t bar_free = bar_full + 8 * kTcSlots;       // [slot]: all groups are done
     const int nbuf = nblocks == 1 ? kTcBuffers + 1 : kTcBuffers;
@@ -308,11 +315,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        constexpr int ones = 6 * kTcGroups + kTcSlots;
-        for (int i = 0; i < ones + kTcSlots; ++i)
+        constexpr int all = 8 * kTcGroups + kTcSlots;
+        for (int i = 0; i < all + kTcSlots; ++i) {
+            const bool warps = i >= 4 * kTcGroups && i < 6 * kTcGroups;  // bar_read
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bars + 8u * i),
-                         "r"(i < ones ? 1 : kTcGroups)
+                         "r"(i >= all ? kTcGroups : warps ? kTcGroup / 32 : 1)
                          : "memory");
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
@@ -380,9 +389,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                     }
                     coords(q - nbuf, c1, c3);
                     asm volatile(
-                        "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group"
-                        " [%0, {%1, %2, %3, %4}], [%5];" ::"l"((uint64_t)&tmap),
-                        "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(buf)
+                        "cp.async.bulk.tensor.5d.global.shared::cta.tile.bulk_group"
+                        " [%0, {%1, %1, %1, %2, %3}], [%4];" ::"l"((uint64_t)&tmap),
+                        "r"(zero), "r"(c1), "r"(c3), "r"(buf)
                         : "memory");
                     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 }
@@ -394,9 +403,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                  "r"(kTileBytes)
                                  : "memory");
                     asm volatile(
-                        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx"
-                        "::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(buf),
-                        "l"((uint64_t)&tmap), "r"(zero), "r"(c1), "r"(zero), "r"(c3), "r"(bar)
+                        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx"
+                        "::bytes [%0], [%1, {%2, %2, %2, %3, %4}], [%5];" ::"r"(buf),
+                        "l"((uint64_t)&tmap), "r"(zero), "r"(c1), "r"(c3), "r"(bar)
                         : "memory");
                     asked = q + 1;
                 }
@@ -412,7 +421,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         const int g = warp / (kTcGroup / 32), gtid = tid & (kTcGroup - 1);
         const int half = gtid >> 7, row = gtid & 127;
         const uint32_t lane = ((uint32_t)(row & ~31) << 16) + 32u * half;
-        const uint32_t tm_d = tmem + kColD + 64u * g;
+        const uint32_t tm_a = tmem + kColA * g;
         // step s - 2: of the next group but one, a step earlier unless that is group 0
         const int before = (g + 1) % kTcGroups, later = g >= 2 ? 0 : 1;
         int slot = 0;
@@ -428,13 +437,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
             if (q >= mine) {  // (the last round)
                 if (gtid == 0)
                     for (int bi = 0; bi < nblocks; ++bi, ++step) {
-                        if (step >= later && !seen(bar_mma, before, step - later)) break;
+                        if (step >= later && !seen(bar_read, before, step - later)) break;
                         if (!resident) {
                             if (!tc_wait(bar_full + 8u * slot, full_phase)) break;
                             arrive(bar_free + 8u * slot);
                             next_slot();
                         }
-                        arrive(of(bar_mma, g, step));
+                        for (int w = 0; w < kTcGroup / 32; ++w) arrive(of(bar_read, g, step));
                     }
                 break;
             }
@@ -448,23 +457,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                     (d1.z & on(6)) ^ (half ? d2.w : 0u);
                 const TcCols cols{{d1.w, d2.x, d2.y, d2.z}};
                 const bool pair = d3.x != 0;
-                const uint32_t tm_a = tmem + kColA * ((step + g) & 1);
-                if (step >= later) bad |= !seen(bar_mma, before, step - later);
+                const uint32_t tm_d = tmem + kColD + 64u * ((step + g) & 1);
+                float x[32];
+                if (pair) tc_read<true>(tile, at, cols, x);
+                else tc_read<false>(tile, at, cols, x);
                 __syncwarp();  // the .aligned instructions want the warp together
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (pair) tc_split<true>(tile, at, cols, tm_a + lane);
-                else tc_split<false>(tile, at, cols, tm_a + lane);
+                tc_split(x, tm_a + lane);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "n"(kTcGroup) : "memory");
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (warp == g * (kTcGroup / 32)) {
                     bad |= !tc_wait(bar_full + 8u * slot, full_phase);
+                    if (step >= later) bad |= !seen(bar_read, before, step - later);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t bh = images - slot * 2 * kBBytes;
                     const uint64_t d64 = make_sdesc(bh, 1024);
                     const uint32_t dl = __shfl_sync(0xffffffffu, (uint32_t)d64, 0);
                     const uint32_t dhi = __shfl_sync(0xffffffffu, (uint32_t)(d64 >> 32), 0);
-                    const uint32_t ta = __shfl_sync(0xffffffffu, tm_a, 0);
+                    const uint32_t td = __shfl_sync(0xffffffffu, tm_d, 0);
                     const uint32_t done = __shfl_sync(0xffffffffu, of(bar_mma, g, step), 0);
                     const uint32_t freed = __shfl_sync(0xffffffffu, bar_free + 8u * slot, 0);
                     if (!__any_sync(0xffffffffu, bad) && tc_elect()) {
@@ -482,8 +492,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                                     "{\n\t.reg .pred p;\n\t"
                                     "setp.ne.b32 p, %4, 0;\n\t"
                                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::
-                                        "r"(tm_d),
-                                    "r"(ta + acol + kk * 8), "l"(db), "r"(kIdesc), "r"(acc)
+                                        "r"(td),
+                                    "r"(tm_a + acol + kk * 8), "l"(db), "r"(kIdesc), "r"(acc)
                                     : "memory");
                             }
                         }
@@ -505,9 +515,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                 bad |= !seen(bar_mma, g, step);
                 __syncwarp();
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (pair) tc_back<true>(tile, at, cols, tm_d + lane);
-                else tc_back<false>(tile, at, cols, tm_d + lane);
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                if (pair) tc_back<true>(tile, at, cols, tm_d + lane, of(bar_read, g, step));
+                else tc_back<false>(tile, at, cols, tm_d + lane, of(bar_read, g, step));
                 if (bi + 1 == nblocks) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 bad = tc_any(g, bad);
                 if (bad) break;
@@ -551,17 +560,18 @@ static PFN_cuTensorMapEncodeTiled_v12000 tc_encode() {
 
 // complex64 tile map for the window [0,4) U [h, h+8):
 //   dim0: 32 floats (16 amplitudes, bits 0-3), box 32 (128 B)
-//   dim1: 2^(h-4) (bits 4..h-1), box 1
-//   dim2: 2^8 (bits h..h+7), box 256
-//   dim3: 2^(n-h-8) (bits h+8..), box 1
+//   dim1: 2^3 (bits h+5..h+7), box 8
+//   dim2: 2^5 (bits h..h+4), box 32
+//   dim3: 2^(h-4) (bits 4..h-1), box 1
+//   dim4: 2^(n-h-8) (bits h+8..), box 1
 static int tc_tile_map(CUtensorMap *map, void *d, int n, int h) {
     auto enc = tc_encode();
     if (!enc) return set_error(LQ_ERR_CUDA, "cuTensorMapEncodeTiled is unavailable");
-    cuuint64_t dims[4] = {32, 1ull << (h - 4), 256, 1ull << (n - h - 8)};
-    cuuint64_t strides[3] = {128, 8ull << h, 8ull << (h + 8)};
-    cuuint32_t box[4] = {32, 1, 256, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d, dims, strides, box, estr,
+    cuuint64_t dims[5] = {32, 8, 32, 1ull << (h - 4), 1ull << (n - h - 8)};
+    cuuint64_t strides[4] = {8ull << (h + 5), 8ull << h, 128, 8ull << (h + 8)};
+    cuuint32_t box[5] = {32, 8, 32, 1, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, d, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
@@ -799,8 +809,7 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
             // Row bits: thread m's bit j goes to the tile bit order[j].  The row order
             // is free (each thread writes back the row it read), so the five lane
             // bits (j < 5) take tile bits whose 8-byte bank slots in the swizzled
-            // tile are linearly independent: slot(l) = (l0, l1^l4, l2^l5, l3^l6), so
-            // tile bit b moves slot bit (b < 4 ? b : b - 3) for b < 7 and none above.
+            // tile are linearly independent: slot(l) = (l0, l1^l9, l2^l10, l3^l11).
             // Up to 16 distinct slots per warp access = the two-wavefront minimum.
             std::vector<int> free_bits;
             for (int l = 0; l < kTcT; ++l) {
@@ -808,7 +817,7 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
                 for (int j = 0; j < 5; ++j) inb |= k[j] == l;
                 if (!inb) free_bits.push_back(l);
             }
-            auto slot_vec = [](int b) { return b < 7 ? 1u << (b < 4 ? b : b - 3) : 0u; };
+            auto slot_vec = [](int b) { return b < 4 ? 1u << b : b < 9 ? 0u : 1u << (b - 8); };
             std::vector<int> order;
             std::vector<uint32_t> basis;  // reduced slot vectors of the chosen lane bits
             for (int b : free_bits) {
