@@ -1138,6 +1138,114 @@ static int static_scratch_address(unsigned char **out) {
 
 using namespace lq;
 
+namespace lq {
+
+// ---------------------------------------------------------------------------
+// Spare resources of small handles.  Creating and destroying a handle costs 52 + 64 us
+// for its stream, and up to some milliseconds for its buffers when no other allocation
+// keeps the driver's memory block mapped: a gradient of a 4-qubit circuit, which makes a
+// handle of its own, took 2.6 ms, nearly all of it there (0.075 ms now).  So a destroyed handle of
+// at most 1 MiB leaves its stream, scratch and buffers, once the device is idle (as
+// cudaFree would have waited for it: others may still read the amplitudes), to the next
+// one on its device.  At most four sets of at most 4 MiB are kept; an allocation that
+// fails frees them.
+// ---------------------------------------------------------------------------
+constexpr size_t kSpares = 4, kSpareBytes = 1 << 20;
+
+struct Spare {
+    int device;
+    size_t bytes;  // of d
+    void *d, *d_prog, *d_work;
+    size_t prog_cap, work_cap;
+    double *d_red;
+    unsigned *d_flag;
+    cudaStream_t stream;
+};
+
+static std::mutex g_spare_mu;
+static std::vector<Spare> &spares() {  // (never destroyed: the driver may be gone by then)
+    static auto *v = new std::vector<Spare>();
+    return *v;
+}
+
+static void free_resources(lq_state *s) {
+    if (s->d) cudaFree(s->d);
+    if (s->d_red) cudaFree(s->d_red);
+    if (s->d_flag) cudaFree(s->d_flag);
+    if (s->d_prog) cudaFree(s->d_prog);
+    if (s->d_work) cudaFree(s->d_work);
+    if (s->stream) cudaStreamDestroy(s->stream);
+}
+
+static void move_spare(lq_state *s, const Spare &x) {
+    s->d = x.d;
+    s->d_red = x.d_red;
+    s->d_flag = x.d_flag;
+    s->d_prog = x.d_prog;
+    s->prog_cap = x.prog_cap;
+    s->d_work = x.d_work;
+    s->work_cap = x.work_cap;
+    s->stream = x.stream;
+}
+
+static void free_spares(size_t keep) {
+    std::lock_guard<std::mutex> lk(g_spare_mu);
+    while (spares().size() > keep) {
+        lq_state t;
+        move_spare(&t, spares().back());
+        spares().pop_back();
+        free_resources(&t);
+    }
+}
+
+// A spare for s (its device), with a buffer of its size if there is one.
+static bool take_spare(lq_state *s) {
+    if (s->bytes > kSpareBytes) return false;
+    Spare x;
+    {
+        std::lock_guard<std::mutex> lk(g_spare_mu);
+        auto &v = spares();
+        size_t best = v.size();
+        for (size_t k = 0; k < v.size(); ++k)
+            if (v[k].device == s->device && (best == v.size() || v[k].bytes == s->bytes)) best = k;
+        if (best == v.size()) return false;
+        x = v[best];
+        v.erase(v.begin() + best);
+    }
+    move_spare(s, x);
+    if (x.bytes != s->bytes) {
+        cudaFree(s->d);
+        s->d = nullptr;
+    }
+    return true;
+}
+
+static bool give_spare(lq_state *s) {
+    if (s->bytes > kSpareBytes || !s->d || !s->d_red || !s->d_flag || !s->stream) return false;
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess || device != s->device ||
+        cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    auto trim = [](void *&p, size_t &cap) {
+        if (p && cap > kSpareBytes) {
+            cudaFree(p);
+            p = nullptr;
+            cap = 0;
+        }
+    };
+    trim(s->d_prog, s->prog_cap);
+    trim(s->d_work, s->work_cap);
+    std::lock_guard<std::mutex> lk(g_spare_mu);
+    if (spares().size() >= kSpares) return false;
+    spares().push_back(Spare{device, s->bytes, s->d, s->d_prog, s->d_work, s->prog_cap, s->work_cap,
+                             s->d_red, s->d_flag, s->stream});
+    return true;
+}
+
+}  // namespace lq
+
 extern "C" {
 
 int lq_expectation_pauli_static(const void *d_amplitudes, int num_qubits, int dtype,
@@ -1304,27 +1412,29 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
     s->dtype = dtype;
     s->bytes = bytes;
     cudaGetDevice(&s->device);
-    auto fail = [&](cudaError_t e, const char *what) {
-        int code = e == cudaErrorMemoryAllocation ? LQ_ERR_OOM : LQ_ERR_CUDA;
-        if (s->d) cudaFree(s->d);
-        if (s->d_red) cudaFree(s->d_red);
-        if (s->d_flag) cudaFree(s->d_flag);
-        if (s->stream) cudaStreamDestroy(s->stream);
+    cudaError_t e = cudaSuccess;
+    if (!take_spare(s)) {
+        e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+        if (e == cudaSuccess)
+            e = cudaMalloc(&s->d_red, sizeof(double) * kRedBlocks * 2 * kMaxTermsPerPass);
+        if (e == cudaSuccess) e = cudaMalloc(&s->d_flag, sizeof(unsigned) * 4);
+    }
+    if (e == cudaSuccess && !s->d) {
+        e = cudaMalloc(&s->d, bytes);
+        if (e == cudaErrorMemoryAllocation) {  // (the spares go first)
+            cudaGetLastError();
+            free_spares(0);
+            e = cudaMalloc(&s->d, bytes);
+        }
+    }
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->d_flag, 0, sizeof(unsigned) * 4, s->stream);
+    if (e != cudaSuccess) {
+        const int code = e == cudaErrorMemoryAllocation ? LQ_ERR_OOM : LQ_ERR_CUDA;
+        free_resources(s);
         delete s;
         cudaGetLastError();
-        return set_error(code, "%s: %s", what, cudaGetErrorString(e));
-    };
-    cudaError_t e;
-    if ((e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking)) != cudaSuccess)
-        return fail(e, "cudaStreamCreate");
-    if ((e = cudaMalloc(&s->d, bytes)) != cudaSuccess) return fail(e, "cudaMalloc(state)");
-    if ((e = cudaMalloc(&s->d_red, sizeof(double) * kRedBlocks * 2 * kMaxTermsPerPass)) !=
-        cudaSuccess)
-        return fail(e, "cudaMalloc(reduction scratch)");
-    if ((e = cudaMalloc(&s->d_flag, sizeof(unsigned) * 4)) != cudaSuccess)
-        return fail(e, "cudaMalloc(flags)");
-    if ((e = cudaMemsetAsync(s->d_flag, 0, sizeof(unsigned) * 4, s->stream)) != cudaSuccess)
-        return fail(e, "cudaMemset");
+        return set_error(code, "creating a %d-qubit state: %s", num_qubits, cudaGetErrorString(e));
+    }
     {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         g_alloc_in_use += bytes;
@@ -1343,16 +1453,11 @@ int lq_state_destroy(lq_state *s) {
     if (!s) return LQ_OK;
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->d) {
-        cudaFree(s->d);
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         g_alloc_in_use -= s->bytes;
     }
-    if (s->d_red) cudaFree(s->d_red);
-    if (s->d_flag) cudaFree(s->d_flag);
-    if (s->d_prog) cudaFree(s->d_prog);
-    if (s->d_work) cudaFree(s->d_work);
     free_plan_cache(s);
-    if (s->stream) cudaStreamDestroy(s->stream);
+    if (!give_spare(s)) free_resources(s);
     delete s;
     return LQ_OK;
 }

@@ -1,6 +1,7 @@
 """GPU: the size-dependent branches of sampling, Pauli sums, damping and the network's
 products, at the edges where each one starts."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -129,3 +130,39 @@ def test_network_products_at_tile_edges(shape, batch):
     assert abs(loss - want_loss) <= 1e-5 * want_loss
     assert np.abs(net.grads() - want_g).max() <= 1e-4 * np.abs(want_g).max()
     net.close()
+
+
+@pytest.mark.parametrize("threads", [1, 6])
+def test_handles_that_take_over_from_destroyed_ones(threads):
+    # sizes below, at and above the kept ones, both types, more handles than are kept
+    sizes = [(4, abi.LQ_C128), (16, abi.LQ_C128), (4, abi.LQ_C64), (17, abi.LQ_C128),
+             (17, abi.LQ_C64), (4, abi.LQ_C128), (9, abi.LQ_C128)]
+    wrong = []
+
+    def work(seed):
+        for turn in range(8):
+            held = []
+            for n, dtype in sizes:
+                st = State(n, dtype)
+                v = st.vector()
+                if v[0] != 1.0 or np.count_nonzero(v) != 1:
+                    wrong.append(("fresh", n, dtype))
+                g = _ry(seed % n, 0.3 + seed + turn)
+                call("lq_apply_circuit", st.handle, n, abi.gate_ptr(g), 1, None, 0,
+                     abi.EXEC_FUSED)
+                held.append((st, n, dtype, 0.3 + seed + turn))
+                if len(held) > 3:
+                    held.pop(0)[0].close()
+            for st, n, dtype, angle in held:
+                v = st.vector()
+                w = [abs(np.cos(angle / 2)), abs(np.sin(angle / 2))]
+                if not np.allclose([abs(v[0]), abs(v[1 << (n - 1 - seed % n)])], w, atol=1e-6):
+                    wrong.append((n, dtype, angle))
+                st.close()
+
+    pool = [threading.Thread(target=work, args=(k,)) for k in range(threads)]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join()
+    assert not wrong
