@@ -249,19 +249,8 @@ def run_vqe_batch(args):
     # amplitudes only); the energy sweeps are not counted
     flops = sum((2 * 8 * r["n"] + 1) * 4 * r["n"] * 14.0 * (1 << r["n"]) for r in recs)
     flops = replicas.max_over_ranks(flops)
-    # With shared prefixes a shifted circuit starts at its parameter's merged
-    # op (layer l, qubit q: op l*n + q of 4n), so it executes the 4n - (l*n + q)
-    # ops from there on; the base circuit runs all 4n.  (A lower bound: the
-    # engine starts at the register round holding that op, a few ops earlier.)
-    if tune.get("shared_prefixes"):
-        executed = 0.0
-        for r in recs:
-            n = r["n"]
-            ops = 4 * n + sum(2 * (4 * n - (p // 2)) for p in range(8 * n))
-            executed += ops * 14.0 * (1 << n)
-        executed = replicas.max_over_ranks(executed)
-    else:
-        executed = flops
+    # The reverse sweep applies each circuit once and undoes it on two states.
+    executed = replicas.max_over_ranks(sum(3 * 4 * r["n"] * 14.0 * (1 << r["n"]) for r in recs))
     cpu = None
     if rank == 0 and ws == 1:
         import oracle
@@ -309,7 +298,7 @@ def run_vqe_batch(args):
                                   "sampled_s_by_qubits": plain_time},
             "speedup_vs_plain": plain_s / batched_s,
             "max_abs_gradient_diff_vs_plain": max_err,
-            "roofline": {"kernel": "k_batch", "bound": "fp64",
+            "roofline": {"kernel": "k_adj_pass", "bound": "fp64",
                          "achieved": executed / batched_s / 1e12, "peak": FP64_PEAK_TFLOPS,
                          "unit": "TFLOP/s",
                          "frac": executed / batched_s / 1e12 / FP64_PEAK_TFLOPS,
@@ -317,14 +306,15 @@ def run_vqe_batch(args):
                          "flops_per_step": executed,
                          "all_circuits_in_full_flops_per_step": flops,
                          "effective_tflops": flops / batched_s / 1e12, "traffic": None,
-                         "note": "gate arithmetic the engine executes (shared prefixes "
-                                 "counted once); energy sweeps not counted; latency bound"},
+                         "note": "gate arithmetic of one circuit forward and two states back; "
+                                 "the Pauli sum and the inner products not counted"},
             "e2e": {"value": total_params / batched_s, "unit": "gradients/s",
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                     "result": "the step is already timed end to end: angles uploaded from "
                               "host memory, energies and gradients read back every call"},
             "cpu_baseline": cpu, "clocks": clocks,
-            "gpu_launches": args.steps * (2 if tune["shared_prefixes"] else 1),
+            # at least: coefficients, a pass forward, the Pauli sum, a pass back, the sums
+            "gpu_launches": args.steps * 5,
             "first_call_s": first_s, "create_s": create_s}
     if rank == 0:
         print(json.dumps(line), flush=True)
@@ -557,7 +547,7 @@ def run_qft(args):
                                    f"({len(g)} gates)", "algorithmic_bytes": algo,
                        "l2_policy": "256 MiB written between timed steps (the 16 MiB state "
                                     "starts each step in HBM; later passes find it in L2)"},
-            "roofline": {"kernel": "k_fused_pp (fused passes)", "bound": "hbm",
+            "roofline": {"kernel": "k_mapped_pass (fused passes)", "bound": "hbm",
                          "achieved": 2 * S / (launch_ms / 1e3) / 1e9 if f_n else None,
                          "peak": peak, "unit": "GB/s",
                          "frac": 2 * S / (launch_ms / 1e3) / 1e9 / peak if f_n else None,
@@ -629,6 +619,8 @@ def run_kernels(args):
     heis = workloads.heisenberg_terms(n, jrng[0:n - 1], jrng[n - 1:2 * (n - 1)],
                                       jrng[2 * (n - 1):3 * (n - 1)], 0.5 * jrng[-1])
     heis_groups = len({int(x) for x in heis["xmask"]})
+    # windows of 12 bits that share one with the next
+    heis_reads = 1 + max(0, -(-(n - 12) // 7))
     m2 = unitary(4)
     m4 = unitary(16)
     # block qubits: bits 2, n-12, n-8, n-5 (the bits above 3 must fit one
@@ -660,12 +652,12 @@ def run_kernels(args):
          lambda: call("lq_apply_block", st.handle, 4, q4, abi.f64_ptr(m4)), 2 * S, PROF_FUSED),
         ("k_norm_partial", "norm_sqr", lambda: call("lq_norm_sqr", st.handle, C.byref(out1)),
          S, PROF_REDUCE),
-        ("k_pauli_zfold", "one Z-string term",
+        ("k_pauli_windows", "one Z-string term",
          lambda: call("lq_expectation_pauli", st.handle, abi.term_ptr(zstring), 1,
                       abi.Y_REFERENCE, C.byref(out1), None), S, PROF_REDUCE),
-        ("k_pauli_group + k_pauli_zfold", f"XYZ chain ({len(heis)} terms, {heis_groups} X-mask groups)",
+        ("k_pauli_windows", f"XYZ chain ({len(heis)} terms, {heis_groups} X-mask groups, {heis_reads} reads)",
          lambda: call("lq_expectation_pauli", st.handle, abi.term_ptr(heis), len(heis),
-                      abi.Y_REFERENCE, C.byref(out1), None), heis_groups * S, PROF_REDUCE),
+                      abi.Y_REFERENCE, C.byref(out1), None), heis_reads * S, PROF_REDUCE),
         ("k_inner_partial", "inner product of two states",
          lambda: call("lq_inner_product", st.handle, other.handle, out2), 2 * S, PROF_REDUCE),
     ]
@@ -1096,10 +1088,10 @@ def main():
     peak, peak_kind = hbm_peak()
     fused_launch_ms = fused_ms.value / max(fused_n.value, 1)
     achieved = 2 * S / (fused_launch_ms / 1e3) / 1e9 if fused_n.value else None
-    traffic, traffic_q = ncu_traffic("k_fused_pass", n)
+    traffic, traffic_q = ncu_traffic("k_mapped_pass", n)
     n_u3 = int(np.sum(gates["kind"] == abi.U3))
     fp64_flops_step = 14.0 * n_u3 * (1 << n)  # 2x2 complex matrix: 14 flops per amplitude
-    roofline = {"kernel": "k_fused_pp (TMA-staged 2^T-amplitude tiles, ping-pong register rounds)",
+    roofline = {"kernel": "k_mapped_pass (2^T-amplitude tiles, mapped register rounds)",
                 "bound": "hbm",
                 "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": (achieved / peak) if achieved else None, "peak_source": peak_kind,

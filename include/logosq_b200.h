@@ -309,8 +309,9 @@ int lq_get_fusion_width(int *tile_bits);
  * standalone per-gate sweeps. */
 int lq_plan_circuit(int num_qubits, const lq_gate *ops, int nops, int *passes, int *rounds,
                     int *standalone);
-/* Host-only dump of the fused program lq_apply_circuit would run (for tests and
- * inspection): int32 counts {steps, rounds, ops, coefficients, T}, then per
+/* Host-only dump of the record-driven program of a gate list, which
+ * lq_apply_circuit runs where some gate has no mapped form (Toffoli, arbitrary
+ * 4x4, non-unitary matrices; for tests and inspection): int32 counts {steps, rounds, ops, coefficients, T}, then per
  * step int32 {fused, gate, h, round_begin, nrounds}, the round records, the op
  * records and the FP64 coefficients.  *used receives the size needed. */
 int lq_plan_dump(int num_qubits, const lq_gate *ops, int nops, const double *theta, int ntheta,
@@ -337,7 +338,10 @@ int lq_ansatz_energy(lq_state *work, const lq_gate *ops, int nops, const double 
                      int nparams, const lq_pauli_term *terms, int nterms, int y_convention,
                      double *energy);
 /* ParameterShift::compute_gradient (src/optimization/gradient.rs:44-78):
- * grad_i = (E(theta + shift e_i) - E(theta - shift e_i)) / 2. */
+ * grad_i = (E(theta + shift e_i) - E(theta - shift e_i)) / 2.  By one reverse
+ * sweep over the state and the observable times it where every parameter turns
+ * one angle of an RX, RY, RZ, PHASE or U3 gate and all gates are unitary, else
+ * by two circuits per parameter. */
 int lq_parameter_shift(lq_state *work, const lq_gate *ops, int nops, const double *theta,
                        int nparams, const lq_pauli_term *terms, int nterms, int y_convention,
                        double shift, double *grad);
@@ -379,7 +383,8 @@ int lq_batch_tuning(const lq_batch *b, int *smem_max_qubits, int *tile_bits);
  * 2^12 amplitudes, or 0 to autotune again on the next lq_batch_gradients call.
  * No reference counterpart (tuning control of this engine). */
 int lq_batch_set_tile_bits(lq_batch *b, int tile_bits);
-/* Whether the batch shares circuit prefixes (each shifted circuit starts from
+/* Whether the engine of shifted circuits (which runs the circuits that the
+ * reverse sweep does not take) shares circuit prefixes (each shifted circuit starts from
  * the unshifted circuit's state just before its parameter's first gate; off
  * when LQ_BATCH_PREFIX=0 at creation or when the checkpoints would not fit)
  * and the device bytes its checkpoints take.  No reference counterpart. */
