@@ -329,6 +329,60 @@ __global__ void k_pauli_group(const A *__restrict__ v, int n, uint64_t xmask,
     if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
 }
 
+// Terms without X bits (one group, X mask 0), for states of 12 or more qubits,
+// launched with 256 threads.  A block takes 4096-amplitude chunks; thread tid
+// handles the 16 indices i = chunk | k << 8 | tid, k = 0..15.  A term's sign
+// (-1)^popcount(i & z) is the sign of the bits the thread keeps fixed (chunk
+// and tid) times (-1)^popcount(k & p), p = bits 8-11 of z.  The terms arrive
+// sorted by p (pbeg[p] .. pbeg[p+1]), so each thread folds all of them into 16
+// coefficients C[p], and one 16-point Walsh-Hadamard transform of C gives the
+// sum of signed coefficients for all 16 k: a few operations per amplitude
+// instead of a popcount and a select per term per amplitude.
+template <class A>
+__global__ void __launch_bounds__(256, 2)
+    k_pauli_zfold(const A *__restrict__ v, int n, const TermCoef *__restrict__ tc, int nt,
+                  const int *__restrict__ pbeg, double *partials) {
+    extern __shared__ TermCoef s_tc[];
+    __shared__ double sh[32];
+    __shared__ int s_pbeg[17];
+    for (int t = threadIdx.x; t < nt; t += blockDim.x) s_tc[t] = tc[t];
+    if (threadIdx.x < 17) s_pbeg[threadIdx.x] = pbeg[threadIdx.x];
+    __syncthreads();
+    double acc[1] = {0.0};
+    const uint64_t nchunks = 1ull << (n - 12);
+    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        const uint64_t fixed = (c << 12) | (uint64_t)threadIdx.x;
+        double pr[16];  // |a|^2 of the 16 amplitudes
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            const double2 a = load_amp(v, fixed | ((uint64_t)k << 8));
+            pr[k] = a.x * a.x + a.y * a.y;
+        }
+        double C[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+            double cq = 0.0;
+            for (int t = s_pbeg[q]; t < s_pbeg[q + 1]; ++t)
+                cq += (__popcll(fixed & s_tc[t].z) & 1) ? -s_tc[t].ca : s_tc[t].ca;
+            C[q] = cq;
+        }
+#pragma unroll
+        for (int hs = 1; hs < 16; hs <<= 1) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                if (q & hs) continue;
+                const double x = C[q], y = C[q | hs];
+                C[q] = x + y;
+                C[q | hs] = x - y;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 16; ++k) acc[0] += pr[k] * C[k];
+    }
+    block_sum<1>(acc, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = acc[0];
+}
+
 // ---------------------------------------------------------------------------
 // Pauli sums by windows.  A tile is the 2^T amplitudes of the index bits [0,4) and
 // [h, h+T-4), held in shared memory as complex128; every group whose X bits lie in
@@ -851,6 +905,43 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         if (wsets.empty() || wsets.back().first < q.a) wsets.push_back({q.b, {}});
         wsets.back().second.push_back(q.group);
     }
+    // A window reads the state at 0.74 of the copy peak, a sweep at the peak (28 qubits, one
+    // term: 0.89 and 0.60 ms; of complex64 a sweep is half of that).  So a window for one
+    // group of few terms, or two of complex64, is sweeps instead where the state is large
+    // enough for that to count more than the launches (20 qubits, two windows of a group
+    // each: 38 us, two sweeps 46), or it is the only group (16 qubits: 30 us, a window 33);
+    // and a sum of terms without X alone is one folded sweep, as far as that goes (n >= 12).
+    constexpr int kSweepQubits = 22;
+    constexpr size_t kSweepTerms = 4;
+    auto few = [&](const std::vector<size_t> &gs) {
+        bool ok = (n >= kSweepQubits || groups.size() == 1) &&
+                  gs.size() <= (s->dtype == LQ_C64 ? 2 : 1);
+        for (size_t gi : gs) ok = ok && groups[gi].second.size() <= kSweepTerms;
+        return ok;
+    };
+    auto to_sweeps = [&](std::vector<size_t> &gs) {
+        sweeps.insert(sweeps.end(), gs.begin(), gs.end());
+        gs.clear();
+    };
+    for (auto &ws : wsets)
+        if (few(ws.second)) to_sweeps(ws.second);
+    wsets.erase(std::remove_if(wsets.begin(), wsets.end(),
+                               [](const auto &ws) { return ws.second.empty(); }),
+                wsets.end());
+    if (wsets.empty() && (few(anywhere) || (anywhere.size() == 1 && n >= 12 &&
+                                            groups[anywhere[0]].first == 0)))
+        to_sweeps(anywhere);
+    int pbeg[17] = {0};  // k_pauli_zfold: its terms sorted by bits 8-11 of the Z mask
+    int zfold = -1;
+    for (size_t k = 0; k < sweeps.size() && !per_term && n >= 12; ++k) {
+        if (groups[sweeps[k]].first != 0) continue;
+        zfold = (int)k;
+        auto pat = [&](int t) { return (int)((terms[t].zmask >> 8) & 15); };
+        std::vector<int> &ts = groups[sweeps[k]].second;
+        std::stable_sort(ts.begin(), ts.end(), [&](int x, int y) { return pat(x) < pat(y); });
+        for (int t : ts)
+            for (int q = pat(t) + 1; q <= 16; ++q) ++pbeg[q];
+    }
     if (wsets.empty() && !anywhere.empty()) wsets.push_back({4, {}});
     if (!wsets.empty())
         wsets[0].second.insert(wsets[0].second.end(), anywhere.begin(), anywhere.end());
@@ -1028,7 +1119,8 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
     const size_t o_win = al(packed.size() * sizeof(TermCoef));
     const size_t o_chk = o_win + al(wins.size() * sizeof(WinDesc));
     const size_t o_pgm = o_chk + al(chunks.size() * sizeof(WinChunk));
-    const size_t o_res = o_pgm + al(program.size());
+    const size_t o_beg = o_pgm + al(program.size());
+    const size_t o_res = o_beg + al(sizeof(pbeg));
     const size_t nres = sweeps.size() + (wins.empty() ? 0 : 1);
     LQ_TRY(ensure_prog(ms, o_res + al(nres * sizeof(double)) + 256));
     char *dp = (char *)ms->d_prog;
@@ -1043,6 +1135,7 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         put(o_win, wins);
         put(o_chk, chunks);
         put(o_pgm, program);
+        memcpy(up.data() + o_beg, pbeg, sizeof(pbeg));
         LQ_CUDA_TRY(cudaMemcpyAsync(dp, up.data(), o_res, cudaMemcpyHostToDevice, s->stream));
     }
     prof_begin(s->stream, kProfReduce);
@@ -1069,7 +1162,13 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         const auto &gr = groups[sweeps[k]];
         const int nt = (int)gr.second.size();
         const size_t shm = nt * sizeof(TermCoef);
-        if (s->dtype == LQ_C128)
+        if ((int)k == zfold && s->dtype == LQ_C128)
+            k_pauli_zfold<<<g, th, shm, s->stream>>>((const double2 *)s->d, n, d_tc + offs[k], nt,
+                                                     (const int *)(dp + o_beg), s->d_red);
+        else if ((int)k == zfold)
+            k_pauli_zfold<<<g, th, shm, s->stream>>>((const float2 *)s->d, n, d_tc + offs[k], nt,
+                                                     (const int *)(dp + o_beg), s->d_red);
+        else if (s->dtype == LQ_C128)
             k_pauli_group<<<g, th, shm, s->stream>>>((const double2 *)s->d, n, gr.first,
                                                      d_tc + offs[k], nt, s->d_red);
         else

@@ -352,9 +352,9 @@ __global__ void __launch_bounds__(256, 2)
         default:
             for (int k = 0; k < rd.npre; ++k) map_table(pl, tabs[rd.pre + k], data, gbase);
             if (rd.nslot) map_any(pl, rd, tabs, data, gbase, gwarp);
-            for (int k = 0; k < rd.ntail; ++k) map_table(pl, tabs[rd.tail + k], data, gbase);
             break;
         }
+        for (int k = 0; k < rd.ntail; ++k) map_table(pl, tabs[rd.tail + k], data, gbase);
         __syncthreads();
     }
     // Back in logical order through the map.
@@ -1060,7 +1060,7 @@ public:
                 return k;
             }
         }
-        bool line = rd.nslot > 0 && !tail;
+        bool line = rd.nslot > 0;
         for (int k = 0; k < rd.nslot; ++k) {
             const MapSlot &d = rd.slot[k];
             line = line && d.kind == 1 && d.ntab <= (k == 0 ? 1 : 0);
@@ -1088,7 +1088,7 @@ public:
         }
         for (int k = 0; k < rd.nslot; ++k) rd.signs |= rd.slot[k].smask != 0;
         if (line) rd.path = rd.nslot + (rd.slot[0].ntab ? 0 : 4);
-        rd.bases = !line || rd.signs;
+        rd.bases = !line || rd.signs || rd.ntail;
         rounds.push_back(rd);
         return slots.size();
     }
@@ -1235,6 +1235,25 @@ private:
 };
 
 bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
+    // A two-qubit rotation whose bits fit no window would take three passes (it is two
+    // permutations around a rotation; 26 qubits: 983 us) where its own sweep takes 317.
+    // A controlled rotation is a whole rotation and a table here, and one record there
+    // (40 of CRX and CRY on 26, 18 and 8 qubits: 4.55, 0.091 and 0.061 ms against 3.76, 0.073
+    // and 0.034; a third of them among single-qubit gates 2.62 against 2.15 on 26): more than
+    // a fifth of them go there.  RXX and RYY are two such rotations in one, and better here
+    // except in small states without much besides (40 on 26, 18 and 11 qubits: 3.9, 0.050 and
+    // 0.059 ms against 4.3, 0.058 and 0.044; three Trotter steps, half of whose gates are
+    // diagonal: 12.1, 0.144 and 0.069 against 19.4, 0.193 and 0.095).
+    size_t controlled = 0, blocks = 0;
+    for (const GateOp &g : gops) {
+        controlled += g.type == OP_M1 && g.nctrl > 0;
+        blocks += g.type == OP_M2;
+        if (g.type == OP_M2 && n > T && std::min(g.b0, g.b1) >= 4 &&
+            std::abs(g.b0 - g.b1) >= T - 4)
+            return false;
+    }
+    if (5 * controlled > gops.size()) return false;
+    if (n < 20 && 3 * (controlled + blocks) > 2 * gops.size()) return false;
     std::vector<MapOp> ops;
     if (!map_lower(gops, ops)) return false;
     std::vector<GateOp> shapes;
@@ -1260,6 +1279,7 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
             continue;
         }
         std::vector<int> left = st.pass.gates;
+        bool closed = false;
         pb.begin(st.pass.h);
         while (!left.empty()) {
             std::vector<int> next;
@@ -1280,7 +1300,9 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
             }
             const bool stuck = next.size() == left.size();
             left = std::move(next);
-            pb.close_round(false);
+            // (the circuit's last round takes what still waits, if there is room)
+            closed = left.empty() && si + 1 == steps.size() && pb.bytes() <= kMapProgram / 2;
+            pb.close_round(closed);
             // a map or program that is full: the pass ends here and goes on as another
             // over the same window
             if (!left.empty() && (stuck || pb.bytes() > kMapProgram)) {
@@ -1288,7 +1310,7 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
                 pb.begin(st.pass.h);
             }
         }
-        if (si + 1 == steps.size()) {
+        if (si + 1 == steps.size() && !closed) {
             if (pb.bytes() > kMapProgram) {
                 pb.finish(out);
                 pb.begin(st.pass.h);

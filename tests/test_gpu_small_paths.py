@@ -101,6 +101,31 @@ def test_pauli_sums_of_many_terms(n):
     st.close()
 
 
+@pytest.mark.parametrize("c64", [False, True])
+@pytest.mark.parametrize("n", [11, 12, 21, 22])
+@pytest.mark.parametrize("xs", [(0,), (1 << 2,), (0, 1 << 2), (1 << 9,), (1 << 5, 1 << 10, 0)])
+def test_pauli_sums_that_are_sweeps(n, xs, c64):
+    # lone groups above and below the size where a sweep takes them; Z strings alone
+    r = np.random.default_rng(n)
+    rows = [(float(r.normal()), x, int(r.integers(0, 1 << n))) for x in xs for _ in range(3)]
+    rows += [(float(r.normal()), xs[0], int(r.integers(0, 1 << n)))
+             for _ in range(0 if xs[0] else 20)]
+    terms = np.zeros(len(rows), dtype=abi.TERM_DTYPE)
+    for t, (c, x, z) in zip(terms, rows):
+        t["coefficient"], t["xmask"], t["zmask"], t["ny"] = c, x, z, bin(x & z).count("1")
+    v = random_state(n, 70 + n)
+    if c64:
+        v = v.astype(np.complex64).astype(np.complex128)
+    st = State(n, abi.LQ_C64 if c64 else abi.LQ_C128)
+    st.set_vector(v)
+    out = C.c_double()
+    call("lq_expectation_pauli", st.handle, abi.term_ptr(terms), len(terms), abi.Y_TEXTBOOK,
+         C.byref(out), None)
+    want = oracle.expectation(v, terms, abi.Y_TEXTBOOK)
+    assert abs(out.value - want) < 1e-12 * np.abs(terms["coefficient"]).sum()
+    st.close()
+
+
 @pytest.mark.parametrize("n,qubits", [(1, [0]), (5, [2, 2, 4]), (12, None), (13, [12, 0])])
 def test_amplitude_damping_target_lists(n, qubits):
     v = random_state(n, n)
