@@ -508,8 +508,17 @@ static bool map_single(const GateOp &g, int &bit, cd u[4], bool &diag) {
 
 static bool unit(cd z) { return std::abs(std::abs(z) - 1.0) <= 1e-12; }
 
+// What the window planner sees: a gate or a run of single-qubit gates, with the map ops
+// that it became.  (Planned op by op, a 2x2 with a quarter turn counted twice, and 60
+// single-qubit gates on 24 qubits took five passes instead of three: 480 us, now 326.)
+struct MapUnit {
+    GateOp shape;
+    int begin, end;
+};
+
 // The circuit as map ops; runs of single-qubit gates on a bit become one 2x2 first.
-static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out) {
+static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
+                      std::vector<MapUnit> &units) {
     struct Run {
         int bit;
         cd u[4];
@@ -548,19 +557,27 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out) 
         list.push_back(Entry{-1, &g});
     }
     for (const Entry &en : list) {
+        if (!units.empty()) units.back().end = (int)out.size();
+        units.push_back(MapUnit{GateOp{}, (int)out.size(), 0});
+        GateOp &shape = units.back().shape;
         if (en.run >= 0) {
             const Run &r = runs[en.run];
             if (r.x) {
                 out.push_back(map_perm_x(r.bit, -1));
+                shape = out.back().g;
             } else if (r.diag) {
                 if (!unit(r.u[0]) || !unit(r.u[3])) return false;
                 out.push_back(map_diag(-1, r.bit, r.u[0], r.u[3], 0.0, 0.0));
-            } else if (!map_rotation(r.u, r.u, r.bit, -1, out)) {
-                return false;
+                shape = out.back().g;
+            } else {
+                if (!map_rotation(r.u, r.u, r.bit, -1, out)) return false;
+                shape.type = OP_M1;
+                shape.t = r.bit;
             }
             continue;
         }
         const GateOp &g = *en.g;
+        shape = g;
         switch (g.type) {
         case OP_PERM1:
             if (g.nctrl != 1) return false;
@@ -617,6 +634,7 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out) 
         default: return false;
         }
     }
+    if (!units.empty()) units.back().end = (int)out.size();
     return true;
 }
 
@@ -1235,8 +1253,6 @@ private:
 };
 
 bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
-    // A two-qubit rotation whose bits fit no window would take three passes (it is two
-    // permutations around a rotation; 26 qubits: 983 us) where its own sweep takes 317.
     // A controlled rotation is a whole rotation and a table here, and one record there
     // (40 of CRX and CRY on 26, 18 and 8 qubits: 4.55, 0.091 and 0.061 ms against 3.76, 0.073
     // and 0.034; a third of them among single-qubit gates 2.62 against 2.15 on 26): more than
@@ -1248,17 +1264,17 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     for (const GateOp &g : gops) {
         controlled += g.type == OP_M1 && g.nctrl > 0;
         blocks += g.type == OP_M2;
-        if (g.type == OP_M2 && n > T && std::min(g.b0, g.b1) >= 4 &&
-            std::abs(g.b0 - g.b1) >= T - 4)
-            return false;
     }
     if (5 * controlled > gops.size()) return false;
     if (n < 20 && 3 * (controlled + blocks) > 2 * gops.size()) return false;
     std::vector<MapOp> ops;
-    if (!map_lower(gops, ops)) return false;
+    std::vector<MapUnit> units;
+    if (!map_lower(gops, ops, units)) return false;
     std::vector<GateOp> shapes;
-    for (const MapOp &o : ops) shapes.push_back(o.g);
+    for (const MapUnit &u : units) shapes.push_back(u.shape);
     const std::vector<PlanStep> steps = plan_circuit(shapes, n, T);
+    // (a two-qubit rotation across windows would be three passes here, 983 us on 26 qubits
+    // where its own sweep takes 317)
     for (const PlanStep &st : steps)
         if (!st.fused && shapes[st.gate].type != OP_SWAP) return false;
     out.T = T;
@@ -1278,7 +1294,9 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
             }
             continue;
         }
-        std::vector<int> left = st.pass.gates;
+        std::vector<int> left;
+        for (int u : st.pass.gates)
+            for (int i = units[u].begin; i < units[u].end; ++i) left.push_back(i);
         bool closed = false;
         pb.begin(st.pass.h);
         while (!left.empty()) {
