@@ -16,18 +16,23 @@
 // blocks {00, 11} and {01, 10} of the latter into bit a with control bit b.
 //
 // A pass is one read and write of the state: a CTA takes the tile of 2^T amplitudes of
-// index bits [0,4) and [h, h+T-4), together with the pass's program, and runs its rounds.  In a round a thread holds 16 amplitudes that
-// differ along four vectors v_0..v_3 (a logical bit's place after CNOTs is a sum of
-// place bits) and does, in straight-line code and in place, the tables and
-// the rotation of each vector in turn.  Places at the end of a pass are not logical
-// order in general; the store reads through the map.
+// index bits [0,4) and [h, h+T-4) and runs the pass's rounds.  In a round a thread holds 16
+// amplitudes that differ along four vectors v_0..v_3 (a logical bit's place after CNOTs is
+// a sum of place bits) and does, in straight-line code and in place, the tables and the
+// rotation of each vector in turn.  Places at the end of a pass are not logical order in
+// general; the store reads through the map.
 //
-// Against the op-record rounds (fused_round.cuh), which this replaces for all circuits
-// that have the form above: those kept two arrays of 16 amplitudes per thread (168 registers,
-// 12 warps per SM) and dispatched every op through a switch; FP64 was 52 % of the
-// instructions, and each issue waited 2.5 cycles on table and record loads and 0.9 on
-// instruction fetch.  Here the code of a round is some 6 KB, the amplitudes take 64 registers,
-// and tables come from the constant bank.
+// Bound: 28 qubits, 20 brickwork layers: 17 passes of 9.5 rounds at T = 11.  A round reads
+// and writes the tile in shared memory, whose pipe is 72-80 % busy (39 of 62.5 ms), FP64
+// 40-44 %, issue 53 %, with 16 warps per SM; HBM would take 22 ms.  More amplitudes per
+// thread would need fewer rounds but halve the warps.
+//
+// Against the op-record rounds (fused_round.cuh: 94.8 ms), which remain for circuits
+// without this form or with many controlled rotations (map_plan): those keep two arrays of
+// 16 amplitudes per thread (168 registers, 12 warps per SM) and dispatch every op through a
+// switch; FP64 was 52 % of the instructions, and each issue waited 2.5 cycles on table and
+// record loads and 0.9 on instruction fetch.  Here the code of a round is some 6 KB, the
+// amplitudes take 64 registers, and tables come from the constant bank.
 #pragma nv_diag_suppress 20208  // (long double is the host planner's)
 #include "mapped.h"
 
@@ -188,8 +193,14 @@ struct MapPlaces {
 
 // A table of any kind on the thread's places, one amplitude at a time.
 __device__ __forceinline__ void map_table(const MapPlaces &pl, const MapTable &tb,
-                                          const double2 *data, uint64_t gbase) {
-    if (tb.kind != 1) {
+                                          const double2 *data, uint64_t gbase, uint64_t gwarp) {
+    if (tb.kind == 0) {  // (uniform addresses)
+        const double2 *p = data + tb.data + map_variant(tb, gwarp);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) *pl.at(e) = cmul2(*pl.at(e), p[e]);
+        return;
+    }
+    if (tb.kind == 2) {
         const double2 *p = data + tb.data + map_variant(tb, gbase);
 #pragma unroll
         for (int e = 0; e < 16; ++e) *pl.at(e) = cmul2(*pl.at(e), p[e]);
@@ -350,11 +361,11 @@ __global__ void __launch_bounds__(256, 2)
         case 7: map_line<3, false>(pl, rd, tabs, data, gbase, gwarp); break;
         case 8: map_line<4, false>(pl, rd, tabs, data, gbase, gwarp); break;
         default:
-            for (int k = 0; k < rd.npre; ++k) map_table(pl, tabs[rd.pre + k], data, gbase);
+            for (int k = 0; k < rd.npre; ++k) map_table(pl, tabs[rd.pre + k], data, gbase, gwarp);
             if (rd.nslot) map_any(pl, rd, tabs, data, gbase, gwarp);
             break;
         }
-        for (int k = 0; k < rd.ntail; ++k) map_table(pl, tabs[rd.tail + k], data, gbase);
+        for (int k = 0; k < rd.ntail; ++k) map_table(pl, tabs[rd.tail + k], data, gbase, gwarp);
         __syncthreads();
     }
     // Back in logical order through the map.
@@ -1066,9 +1077,12 @@ public:
         }
         uint32_t in_warp = 0;  // tile bits that differ between threads of a warp
         for (size_t j = 0; j < std::min<size_t>(lanes.size(), 5); ++j) in_warp |= 1u << lanes[j];
-        for (size_t k = old_tabs; k < tabs.size(); ++k)
-            for (int q = 0; q < tabs[k].count && tabs[k].kind == 0; ++q)
-                if (tabs[k].m[q] & spread(in_warp)) tabs[k].kind = 2;
+        auto mark = [&](size_t from) {  // kinds 0 and 2
+            for (size_t k = from; k < tabs.size(); ++k)
+                for (int q = 0; q < tabs[k].count && tabs[k].kind == 0; ++q)
+                    if (tabs[k].m[q] & spread(in_warp)) tabs[k].kind = 2;
+        };
+        mark(old_tabs);
         for (int k = 1; k < rd.nslot; ++k) {
             const MapSlot &d = rd.slot[k];
             if (d.ntab > 1 || (d.ntab && tabs[d.tab].kind != 0)) {
@@ -1103,6 +1117,7 @@ public:
         if (tail) {
             tables(wait.items, true, rd.ntail, rd.tail);
             wait.items.clear();
+            mark((size_t)rd.tail);
         }
         for (int k = 0; k < rd.nslot; ++k) rd.signs |= rd.slot[k].smask != 0;
         if (line) rd.path = rd.nslot + (rd.slot[0].ntab ? 0 : 4);
@@ -1277,6 +1292,10 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     // where its own sweep takes 317)
     for (const PlanStep &st : steps)
         if (!st.fused && shapes[st.gate].type != OP_SWAP) return false;
+    // the last pass takes what still waits (sweeps after it only move amplitudes)
+    size_t last = steps.size();
+    for (size_t si = 0; si < steps.size(); ++si)
+        if (steps[si].fused) last = si;
     out.T = T;
     Waiting wait;
     PassBuilder pb(n, T, wait);
@@ -1318,8 +1337,8 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
             }
             const bool stuck = next.size() == left.size();
             left = std::move(next);
-            // (the circuit's last round takes what still waits, if there is room)
-            closed = left.empty() && si + 1 == steps.size() && pb.bytes() <= kMapProgram / 2;
+            // (in its last round, if there is room)
+            closed = left.empty() && si == last && pb.bytes() <= kMapProgram / 2;
             pb.close_round(closed);
             // a map or program that is full: the pass ends here and goes on as another
             // over the same window
@@ -1328,7 +1347,7 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
                 pb.begin(st.pass.h);
             }
         }
-        if (si + 1 == steps.size() && !closed) {
+        if (si == last && !closed) {
             if (pb.bytes() > kMapProgram) {
                 pb.finish(out);
                 pb.begin(st.pass.h);
@@ -1337,7 +1356,7 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
         }
         pb.finish(out);
     }
-    // a circuit that ends in a sweep of its own, or waits without any pass
+    // (a number from sweeps alone)
     if (!wait.items.empty() || wait.scalar != cd(1.0)) {
         pb.begin(4);
         pb.close_round(true);
