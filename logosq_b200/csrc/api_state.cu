@@ -1244,10 +1244,12 @@ namespace lq {
 // for its stream, and up to some milliseconds for its buffers when no other allocation
 // keeps the driver's memory block mapped: a gradient of a 4-qubit circuit, which makes a
 // handle of its own, took 2.6 ms, nearly all of it there (0.075 ms now).  So a destroyed handle of
-// at most 1 MiB leaves its stream, scratch and buffers, once the device is idle (as
-// cudaFree would have waited for it: others may still read the amplitudes), to the next
-// one on its device.  At most four sets of at most 4 MiB are kept; an allocation that
-// fails frees them.
+// at most 1 MiB leaves its stream, scratch and buffers to the next one on its device.  All of
+// them are used on the handle's own stream, which its destruction waits for; a wait for the
+// whole device would break a graph capture on any other stream.  Only the amplitudes may be
+// known elsewhere (lq_state::lent): they are then given back by cudaFree, which waits for
+// their readers.  At most four sets of at most 4 MiB are kept; a failed allocation of
+// amplitudes frees them.
 // ---------------------------------------------------------------------------
 constexpr size_t kSpares = 4, kSpareBytes = 1 << 20;
 
@@ -1266,6 +1268,9 @@ static std::vector<Spare> &spares() {  // (never destroyed: the driver may be go
     static auto *v = new std::vector<Spare>();
     return *v;
 }
+
+// s's amplitudes may be read on other streams from now on.
+static void lend(const lq_state *s) { const_cast<lq_state *>(s)->lent = true; }
 
 static void free_resources(lq_state *s) {
     if (s->d) cudaFree(s->d);
@@ -1313,19 +1318,19 @@ static bool take_spare(lq_state *s) {
     }
     move_spare(s, x);
     if (x.bytes != s->bytes) {
-        cudaFree(s->d);
+        if (s->d) cudaFree(s->d);
         s->d = nullptr;
     }
     return true;
 }
 
+// The caller has waited for s's stream.
 static bool give_spare(lq_state *s) {
     if (s->bytes > kSpareBytes || !s->d || !s->d_red || !s->d_flag || !s->stream) return false;
-    int device = -1;
-    if (cudaGetDevice(&device) != cudaSuccess || device != s->device ||
-        cudaDeviceSynchronize() != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+    auto room = [] { return spares().size() < kSpares; };
+    {
+        std::lock_guard<std::mutex> lk(g_spare_mu);
+        if (!room()) return false;
     }
     auto trim = [](void *&p, size_t &cap) {
         if (p && cap > kSpareBytes) {
@@ -1336,10 +1341,14 @@ static bool give_spare(lq_state *s) {
     };
     trim(s->d_prog, s->prog_cap);
     trim(s->d_work, s->work_cap);
+    if (s->lent) {
+        cudaFree(s->d);
+        s->d = nullptr;
+    }
     std::lock_guard<std::mutex> lk(g_spare_mu);
-    if (spares().size() >= kSpares) return false;
-    spares().push_back(Spare{device, s->bytes, s->d, s->d_prog, s->d_work, s->prog_cap, s->work_cap,
-                             s->d_red, s->d_flag, s->stream});
+    if (!room()) return false;
+    spares().push_back(Spare{s->device, s->d ? s->bytes : 0, s->d, s->d_prog, s->d_work,
+                             s->prog_cap, s->work_cap, s->d_red, s->d_flag, s->stream});
     return true;
 }
 
@@ -1550,13 +1559,14 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
 
 int lq_state_destroy(lq_state *s) {
     if (!s) return LQ_OK;
-    if (s->stream) cudaStreamSynchronize(s->stream);
+    // (a stream that cannot be waited for is not handed on)
+    const bool idle = s->stream && cudaStreamSynchronize(s->stream) == cudaSuccess;
     if (s->d) {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         g_alloc_in_use -= s->bytes;
     }
     free_plan_cache(s);
-    if (!give_spare(s)) free_resources(s);
+    if (!idle || !give_spare(s)) free_resources(s);
     delete s;
     return LQ_OK;
 }
@@ -1679,6 +1689,7 @@ int lq_state_copy(lq_state *dst, const lq_state *src) {
         return set_error(LQ_ERR_DIMENSION_MISMATCH, "Dimension mismatch: expected 2^%d, got 2^%d",
                          dst->n, src->n);
     LQ_CUDA_TRY(cudaStreamSynchronize(src->stream));
+    lend(src);
     LQ_CUDA_TRY(cudaMemcpyAsync(dst->d, src->d, dst->bytes, cudaMemcpyDeviceToDevice, dst->stream));
     return LQ_OK;
 }
@@ -1694,6 +1705,8 @@ int lq_state_tensor_product(lq_state *out, const lq_state *a, const lq_state *b)
         return set_error(LQ_ERR_UNSUPPORTED, "mixed dtypes");
     LQ_CUDA_TRY(cudaStreamSynchronize(a->stream));
     LQ_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    lend(a);
+    lend(b);
     const uint64_t N = 1ull << out->n;
     if (out->dtype == LQ_C128)
         k_kron<<<grid_for(N, 256), 256, 0, out->stream>>>(
@@ -1729,6 +1742,7 @@ int lq_check_wait_timeout(lq_state *s, unsigned polls) {
 int lq_state_device_ptr(lq_state *s, void **dptr) {
     LQ_TRY(check_state(s));
     if (!dptr) return set_error(LQ_ERR_INVALID_ARG, "null output");
+    lend(s);
     *dptr = s->d;
     return LQ_OK;
 }

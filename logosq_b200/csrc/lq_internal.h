@@ -66,6 +66,7 @@ struct lq_state {
     int device = 0;
     void *d = nullptr;        // 2^n amplitudes
     size_t bytes = 0;
+    bool lent = false;        // work on other streams may read d (its pointer was given out, ...)
     cudaStream_t stream = nullptr;
     double *d_red = nullptr;  // kRedBlocks * 2 * kMaxTermsPerPass doubles
     // Host mirror of the final reduction results.  Plain memory: page-locking 512
