@@ -376,11 +376,14 @@ int lq_batch_num_params(const lq_batch *b, int *out);
 int lq_batch_gradients(lq_batch *b, const double *theta, double shift, double *energy,
                        double *grad);
 /* Tuning of the batch: the largest qubit count kept entirely in shared memory,
- * and the fusion width (tile bits) the autotuner chose on the first
- * lq_batch_gradients call for larger instances (0 before that call). */
+ * and the fusion width (tile bits) of larger instances in the last
+ * lq_batch_gradients call, or the forced one (0 before the first call).  The
+ * reverse sweep takes 11; the shifted circuits take the fastest of 10, 11 and 12,
+ * timed on their first call. */
 int lq_batch_tuning(const lq_batch *b, int *smem_max_qubits, int *tile_bits);
 /* Force the fusion width (tile bits 10, 11 or 12) of the instances larger than
- * 2^12 amplitudes, or 0 to autotune again on the next lq_batch_gradients call.
+ * 2^12 amplitudes, or 0 for 11 in the reverse sweep and a new timing where the
+ * shifted circuits run.
  * No reference counterpart (tuning control of this engine). */
 int lq_batch_set_tile_bits(lq_batch *b, int tile_bits);
 /* Whether the engine of shifted circuits (which runs the circuits that the

@@ -148,7 +148,9 @@ struct lq_batch {
     int grid = 0;
     cudaStream_t stream = nullptr;
     std::vector<lq::BProgram> progs;  // one per candidate fusion width
-    int chosen = -1;                  // index into progs
+    int forced = -1;                  // lq_batch_set_tile_bits; index into progs
+    int chosen = -1;                  // of the shifted circuits: forced, or their autotuner's
+    int used_T = 0;                   // tile width of the last call
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     double shift_captured = 0.0;
@@ -1224,11 +1226,12 @@ int lq_batch_gradients(lq_batch *b, const double *theta, double shift, double *e
     // One reverse sweep per instance where that gives the rule's values (adjoint.cu).
     // Tile width 11 unless the caller forced one: the pair of states fills 64 KB, so
     // three CTAs share an SM and a pass covers seven upper bits.
+    constexpr int kSweepT = 11;
     if (b->sweep && std::isfinite(shift) &&
         std::all_of(theta, theta + b->total_params, [](double x) { return std::isfinite(x); })) {
-        const int want = b->chosen >= 0 ? b->chosen : 1;
-        if (lq_batch::Sweep *sw = ensure_sweep(b, b->progs[want].T)) {
-            b->chosen = want;
+        const int T = b->forced >= 0 ? b->progs[b->forced].T : kSweepT;
+        if (lq_batch::Sweep *sw = ensure_sweep(b, T)) {
+            b->used_T = T;
             return sweep_gradients(b, *sw, theta, shift, energy, grad);
         }
     }
@@ -1259,6 +1262,7 @@ int lq_batch_gradients(lq_batch *b, const double *theta, double shift, double *e
         }
     }
     BProgram &pg = b->progs[b->chosen];
+    b->used_T = pg.T;
     LQ_TRY(fill_coefficients(b, pg, theta, shift, b->coef_h));
     if (!b->exec) {
         // Capture [counter reset, coefficient upload, persistent kernel, energy
@@ -1296,7 +1300,7 @@ int lq_batch_gradients(lq_batch *b, const double *theta, double shift, double *e
 int lq_batch_tuning(const lq_batch *b, int *smem_max_qubits, int *tile_bits) {
     if (!b) return set_error(LQ_ERR_INVALID_ARG, "null batch");
     if (smem_max_qubits) *smem_max_qubits = kSmemStateMax;
-    if (tile_bits) *tile_bits = b->chosen >= 0 ? b->progs[b->chosen].T : 0;
+    if (tile_bits) *tile_bits = b->forced >= 0 ? b->progs[b->forced].T : b->used_T;
     return LQ_OK;
 }
 
@@ -1320,7 +1324,8 @@ int lq_batch_set_tile_bits(lq_batch *b, int tile_bits) {
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
-    b->chosen = pick;  // -1: autotune again on the next lq_batch_gradients call
+    b->forced = b->chosen = pick;  // -1: width 11, and the shifted circuits tune again
+    b->used_T = 0;
     return LQ_OK;
 }
 
