@@ -159,8 +159,11 @@ int lq_version(void);
 int lq_device_count(int *count);
 /* Select the device that later lq_state_create calls on this thread use. */
 int lq_set_device(int device);
-/* Host-side cap on bytes that lq_state_create may allocate (0 = no cap).
- * Lets tests exercise LQ_ERR_OOM without exhausting a shared GPU. */
+/* Host-side cap on bytes of amplitudes that lq_state_create may allocate (0 = no
+ * cap).  Lets tests exercise LQ_ERR_OOM without exhausting a shared GPU.  Gradient
+ * sweeps keep the states they allocate beside the handles within it too: a batch
+ * takes fewer chains at a time, and where not even one fits, the shifted circuits
+ * run. */
 int lq_set_alloc_limit(uint64_t bytes);
 
 /* Launch timing (no reference counterpart; used by the benchmark): when

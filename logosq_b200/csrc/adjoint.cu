@@ -1444,7 +1444,10 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
     // A plain call works in its handle's own program buffer and amplitudes.
     cudaError_t e = cudaSuccess;
     const size_t copies = work ? 1 : 2;
-    if (p.amps > 0) e = cudaMalloc(&p.states, (size_t)p.amps * copies * sizeof(double2));
+    const size_t states = (size_t)p.amps * copies * sizeof(double2);
+    if (states > alloc_room())
+        return set_error(LQ_ERR_OOM, "%zu bytes of states exceed the allocation limit", states);
+    if (states > 0) e = cudaMalloc(&p.states, states);
     if (e == cudaSuccess) {
         if (work) {
             LQ_TRY(ensure_prog(work, off));

@@ -32,6 +32,17 @@ int set_error(int code, const char *fmt, ...) {
 
 void clear_error() { g_last_error.clear(); }
 
+KeepError::KeepError() : text_(g_last_error) {}
+KeepError::~KeepError() {
+    if (on_) g_last_error = std::move(text_);
+}
+
+size_t alloc_room() {
+    std::lock_guard<std::mutex> lk(g_alloc_mu);
+    if (!g_alloc_limit) return (size_t)-1;
+    return g_alloc_limit > g_alloc_in_use ? (size_t)(g_alloc_limit - g_alloc_in_use) : 0;
+}
+
 int check_state(const lq_state *s) {
     if (!s) return set_error(LQ_ERR_INVALID_ARG, "null state handle");
     if (!s->d) return set_error(LQ_ERR_INVALID_ARG, "state handle has no device buffer");

@@ -114,8 +114,8 @@ struct lq_batch {
     std::vector<std::vector<lq_pauli_term>> terms;
     int total_params = 0;
     int maxn = 0;
-    // Reverse-sweep programs (adjoint.cu) by tile width, built on first use; sweep
-    // is false when some instance needs the shifted circuits.
+    // The reverse-sweep program (adjoint.cu) of the tile width used last, built on first
+    // use; sweep is false when some instance has no sweep.
     bool sweep = true;
     struct Sweep {
         int T = 0;
@@ -123,7 +123,11 @@ struct lq_batch {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
     };
-    std::vector<Sweep> sweeps;
+    Sweep sw;
+    // After a failed allocation for it: the free bytes, and those left under the
+    // allocation limit, that a next attempt must exceed.
+    bool sweep_failed = false;
+    size_t sweep_free = 0, sweep_room = 0;
     double *io_h = nullptr;  // pinned: parameters and shift up, energies and gradients down
     // The shifted circuits' device side, made on their first use.
     bool shift_ready = false;
@@ -910,12 +914,14 @@ static void free_shift_engine(lq_batch *b) {
     b->coef_h = b->energy_h = nullptr;
 }
 
+static void drop_sweep(lq_batch *b) {
+    if (b->sw.exec) cudaGraphExecDestroy(b->sw.exec);
+    if (b->sw.graph) cudaGraphDestroy(b->sw.graph);
+    b->sw = lq_batch::Sweep{};
+}
+
 static void free_batch(lq_batch *b) {
-    for (auto &sw : b->sweeps) {
-        if (sw.exec) cudaGraphExecDestroy(sw.exec);
-        if (sw.graph) cudaGraphDestroy(sw.graph);
-    }
-    b->sweeps.clear();
+    drop_sweep(b);
     if (b->io_h) cudaFreeHost(b->io_h);
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -970,36 +976,49 @@ static int ensure_shift_engine(lq_batch *b) {
     return LQ_OK;
 }
 
-// The reverse-sweep program for tile width T, or null with b->sweep cleared when the
-// shifted circuits have to run.
+// The reverse-sweep program for tile width T, or null when the shifted circuits have to
+// run: for good (b->sweep cleared) if some instance has no sweep, for this call if memory
+// is short.  Only one width's program is held at a time.
 static lq_batch::Sweep *ensure_sweep(lq_batch *b, int T) {
-    for (auto &sw : b->sweeps)
-        if (sw.T == T) return &sw;
+    if (b->sw.prog && b->sw.T == T) return &b->sw;
+    const KeepError keep;  // (the call goes on without the sweep)
+    size_t freeb = 0, totalb = 0;
+    const size_t room = alloc_room();
+    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = 0;
+    if (b->sweep_failed && freeb <= b->sweep_free && room <= b->sweep_room) return nullptr;
+    b->sweep_failed = false;
+    drop_sweep(b);
     std::vector<AdjSpec> specs;
     for (int i = 0; i < b->ninst; ++i)
         specs.push_back(AdjSpec{b->n[i], b->ops[i].data(), (int)b->ops[i].size(), b->nparams[i],
                                 b->terms[i].data(), (int)b->terms[i].size(), LQ_Y_REFERENCE});
-    size_t freeb = 0, totalb = 0;
-    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) freeb = 0;
-    lq_batch::Sweep sw;
-    sw.T = T;
-    sw.prog = adj_plan(specs, T, freeb / 2);
-    if (sw.prog && !b->io_h &&
-        cudaMallocHost(&b->io_h, sizeof(double) * (2 * (size_t)b->total_params + 1 + b->ninst)) !=
+    if (b->io_h ||
+        cudaMallocHost(&b->io_h, sizeof(double) * (2 * (size_t)b->total_params + 1 + b->ninst)) ==
             cudaSuccess) {
+        // (smaller budgets: fewer chains at a time, down to one)
+        for (size_t budget : {std::min(freeb / 2, room), std::min(freeb / 8, room), (size_t)0}) {
+            lq_batch::Sweep sw;
+            sw.T = T;
+            sw.prog = adj_plan(specs, T, budget);
+            if (!sw.prog) {
+                b->sweep = false;
+                return nullptr;
+            }
+            const int rc = adj_upload(*sw.prog, nullptr, b->stream);
+            if (rc == LQ_OK && cudaStreamSynchronize(b->stream) == cudaSuccess) {
+                b->sw = std::move(sw);
+                return &b->sw;
+            }
+            if (rc != LQ_ERR_OOM) break;
+        }
+    } else {
         b->io_h = nullptr;
-        sw.prog.reset();
     }
-    if (sw.prog && (adj_upload(*sw.prog, nullptr, b->stream) != LQ_OK ||
-                    cudaStreamSynchronize(b->stream) != cudaSuccess))
-        sw.prog.reset();
-    if (!sw.prog) {
-        cudaGetLastError();
-        b->sweep = false;
-        return nullptr;
-    }
-    b->sweeps.push_back(std::move(sw));
-    return &b->sweeps.back();
+    cudaGetLastError();
+    b->sweep_failed = true;
+    b->sweep_free = freeb;
+    b->sweep_room = room;
+    return nullptr;
 }
 
 static int sweep_gradients(lq_batch *b, lq_batch::Sweep &sw, const double *theta, double shift,

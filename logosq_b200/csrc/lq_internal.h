@@ -19,6 +19,20 @@ namespace lq {
 int set_error(int code, const char *fmt, ...);
 void clear_error();
 
+// Puts the calling thread's last error text back at its end, unless released: around an
+// attempt whose failure the call makes up for.
+class KeepError {
+public:
+    KeepError();
+    ~KeepError();
+    KeepError(const KeepError &) = delete;
+    void release() { on_ = false; }
+
+private:
+    std::string text_;
+    bool on_ = true;
+};
+
 #define LQ_CUDA_TRY(expr)                                                             \
     do {                                                                              \
         cudaError_t _e = (expr);                                                      \
@@ -96,6 +110,8 @@ inline size_t amp_bytes(int dtype) { return dtype == LQ_C64 ? 8 : 16; }
 int check_state(const lq_state *s);
 int check_qubit(const lq_state *s, int q);
 int ensure_prog(lq_state *s, size_t bytes);
+// Bytes of amplitudes that may still be allocated under lq_set_alloc_limit.
+size_t alloc_room();
 
 // gates.cu
 int apply_gate_c128(lq_state *s, const lq_gate *g, const double *theta, int ntheta,

@@ -61,11 +61,13 @@ static int sweep_gradient(lq_state *work, const lq_gate *ops, int nops, const do
     for (int i = 0; i < nparams; ++i)
         if (!std::isfinite(theta[i])) return LQ_OK;
     if (!plain_terms(terms, nterms, work->n)) return LQ_OK;
+    KeepError keep;  // (where the shifted circuits run, the sweep's reason is no error)
     const auto plan = adj_plan({AdjSpec{work->n, ops, nops, nparams, terms, nterms, yconv}}, 11,
                                (size_t)-1);
     if (!plan) return LQ_OK;
     const int rc = adj_upload(*plan, work, work->stream);
     if (rc == LQ_ERR_OOM) return LQ_OK;
+    keep.release();
     LQ_TRY(rc);
     std::vector<double> up(theta, theta + nparams), out(nparams + 1);
     up.push_back(shift);
