@@ -1,5 +1,5 @@
 """GPU: amplitude damping around its size-dependent forms (one target in place, several
-through a second vector), against
+through a second vector that is kept with the handle or allocated for the call), against
 the oracle at the suite's 1e-12."""
 import ctypes as C
 
@@ -39,3 +39,17 @@ def test_one_target_needs_no_second_vector():
     assert before - torch.cuda.mem_get_info()[0] < 32 << 20
     st.close()
 
+
+def test_second_vector_of_a_large_state():
+    n = 24  # 256 MiB: allocated for the call and given back
+    st = State.plus_state(n)
+    call("lq_noise_amplitude_damping", st.handle, 0.2, (C.c_int * 2)(0, n - 1), 2)
+    # plus state: amplitudes by the two bits, (1 + sqrt g) + (1 + sqrt g) and so on
+    g, k = np.sqrt(0.2), np.sqrt(0.8)
+    want = np.array([2 * (1 + g), 1 + g + k, 2 * k])
+    want /= np.sqrt((want[0] ** 2 + 2 * want[1] ** 2 + want[2] ** 2) / 4 * (1 << n))
+    v = st.vector()
+    i = np.arange(1 << n)
+    ones = (i & 1) + (i >> (n - 1))
+    assert np.abs(v - want[ones]).max() < 1e-12
+    st.close()
