@@ -1270,7 +1270,7 @@ static bool adj_plan_one(const AdjSpec &sp, int param_base, int T_large, AdjProg
     for (int dir = 0; dir < 2; ++dir) {
         const auto &go = dir ? back : gops;
         const auto &gr = dir ? back_run : op_run;
-        for (const PlanStep &st : plan_circuit(go, n, T, dir ? 3 : 4)) {
+        for (const PlanStep &st : plan_windows(go, n, T)) {
             if (!st.fused) return false;
             AdjPass ap{};
             ap.h = st.pass.h;

@@ -280,7 +280,7 @@ static int choose_lanes(const int rpos[4], int T, int *lane) {
     // Thread-index bits go to the tile positions outside R.  The first three
     // should be positions whose swizzle images (p mod 3 for p < 6) differ, so
     // that 8 consecutive threads touch 8 distinct 16-byte bank groups.
-    bool inR[kMaxT + 1] = {false};
+    bool inR[kMaxT] = {false};
     for (int k = 0; k < 4; ++k) inR[rpos[k]] = true;
     std::vector<int> free;
     for (int p = 0; p < T; ++p)
@@ -302,16 +302,16 @@ static int choose_lanes(const int rpos[4], int T, int *lane) {
     return (int)order.size();
 }
 
-static void pad_rpos(std::vector<int> &R, int T, int count = 4) {
-    // Fill up to `count` register bits, preferring positions that keep one of
+static void pad_rpos(std::vector<int> &R, int T) {
+    // Fill up to four register bits, preferring positions that keep one of
     // each pair (r, r+3), r < 3, outside R (see choose_lanes).
     auto conflicts = [&](int p) {
         if (p >= 6) return false;
         const int partner = p < 3 ? p + 3 : p - 3;
         return std::find(R.begin(), R.end(), partner) != R.end();
     };
-    for (int pass = 0; pass < 2 && (int)R.size() < count; ++pass) {
-        for (int p = T - 1; p >= 0 && (int)R.size() < count; --p) {
+    for (int pass = 0; pass < 2 && (int)R.size() < 4; ++pass) {
+        for (int p = T - 1; p >= 0 && (int)R.size() < 4; --p) {
             if (std::find(R.begin(), R.end(), p) != R.end()) continue;
             if (pass == 0 && conflicts(p)) continue;
             R.push_back(p);
@@ -709,79 +709,97 @@ static void fold_pairs(std::vector<GateOp> &gops, std::vector<int> &orig, int T)
     }
 }
 
-std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T, int maxr) {
+PlanGate plan_gate(const GateOp &g) {
+    PlanGate p;
+    p.bits = op_bits(g);
+    p.mixed = reg_bits(g);
+    p.fusable = !g.renorm && popc(p.mixed) <= 4;
+    p.barrier = g.renorm;
+    return p;
+}
+
+std::vector<PlanStep> plan_windows(const std::vector<PlanGate> &gates, int n, int T) {
     const int m = T - 4;
     std::vector<PlanStep> steps;
-    const int G = (int)gops.size();
+    const int G = (int)gates.size();
     const uint64_t all = (1ull << n) - 1;
     std::vector<char> done(G, 0);
-    std::vector<uint64_t> bits(G), rbits(G);
-    std::vector<char> fusable(G);
-    for (int i = 0; i < G; ++i) {
-        bits[i] = op_bits(gops[i]);
-        rbits[i] = reg_bits(gops[i]);
-        fusable[i] = !gops[i].renorm && popc(rbits[i]) <= maxr;
-    }
     int remaining = G, first = 0;
+    // The gates that a pass over window W takes, in order (take: mark them done too).
+    auto scan = [&](uint64_t W, std::vector<int> *take) {
+        uint64_t blocked = 0;
+        int cnt = 0;
+        for (int i = first; i < G; ++i) {
+            if (done[i]) continue;
+            const PlanGate &g = gates[i];
+            if (g.fusable && (g.mixed & ~W) == 0 && (g.bits & blocked) == 0) {
+                ++cnt;
+                if (take) {
+                    take->push_back(i);
+                    done[i] = 1;
+                }
+            } else {
+                blocked |= g.barrier ? all : g.bits;
+                if ((blocked & all) == all) break;
+            }
+        }
+        return cnt;
+    };
     while (remaining > 0) {
         while (first < G && done[first]) ++first;
         int best_h = -1, best_cnt = 0;
         for (int h = 4; h + m <= n; ++h) {
-            const uint64_t W = window_mask(h, m);
-            uint64_t blocked = 0;
-            int cnt = 0;
-            for (int i = first; i < G; ++i) {
-                if (done[i]) continue;
-                if (fusable[i] && (rbits[i] & ~W) == 0 && (bits[i] & blocked) == 0) {
-                    ++cnt;
-                } else {
-                    // A renormalising gate is a barrier for every bit.
-                    blocked |= gops[i].renorm ? all : bits[i];
-                    if ((blocked & all) == all) break;
-                }
-            }
+            const int cnt = scan(window_mask(h, m), nullptr);
             if (cnt > best_cnt) {
                 best_cnt = cnt;
                 best_h = h;
             }
         }
+        PlanStep st;
         if (best_cnt == 0) {
-            PlanStep st;
             st.fused = false;
             st.gate = first;
-            steps.push_back(st);
             done[first] = 1;
             --remaining;
-            continue;
+        } else {
+            st.fused = true;
+            st.pass.h = best_h;
+            st.pass.gates.reserve(best_cnt);
+            remaining -= scan(window_mask(best_h, m), &st.pass.gates);
         }
-        PlanStep st;
-        st.fused = true;
-        st.pass.h = best_h;
-        const uint64_t W = window_mask(best_h, m);
-        uint64_t blocked = 0;
-        for (int i = first; i < G; ++i) {
-            if (done[i]) continue;
-            if (fusable[i] && (rbits[i] & ~W) == 0 && (bits[i] & blocked) == 0) {
-                st.pass.gates.push_back(i);
-                done[i] = 1;
-                --remaining;
-            } else {
-                blocked |= gops[i].renorm ? all : bits[i];
-                if ((blocked & all) == all) break;
-            }
-        }
+        steps.push_back(std::move(st));
+    }
+    return steps;
+}
+
+static std::vector<PlanGate> plan_gates(const std::vector<GateOp> &gops) {
+    std::vector<PlanGate> gates;
+    gates.reserve(gops.size());
+    for (const GateOp &g : gops) gates.push_back(plan_gate(g));
+    return gates;
+}
+
+std::vector<PlanStep> plan_windows(const std::vector<GateOp> &gops, int n, int T) {
+    return plan_windows(plan_gates(gops), n, T);
+}
+
+std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T) {
+    const std::vector<PlanGate> gates = plan_gates(gops);
+    std::vector<PlanStep> steps = plan_windows(gates, n, T);
+    for (PlanStep &st : steps) {
+        if (!st.fused) continue;
         // Rounds: greedy, in order; an op joins the round if it is not blocked by
         // an earlier unscheduled op sharing a bit and its register bits fit R.
         const int P = (int)st.pass.gates.size();
         std::vector<char> sched(P, 0);
         std::vector<uint64_t> lreg(P), gall(P);
         for (int k = 0; k < P; ++k) {
-            const int i = st.pass.gates[k];
+            const PlanGate &g = gates[st.pass.gates[k]];
             uint64_t l = 0;
             for (int b = 0; b < n; ++b)
-                if (rbits[i] >> b & 1) l |= 1ull << local_pos(b, best_h);
+                if (g.mixed >> b & 1) l |= 1ull << local_pos(b, st.pass.h);
             lreg[k] = l;
-            gall[k] = bits[i];
+            gall[k] = g.bits;
         }
         int left = P;
         while (left > 0) {
@@ -789,7 +807,7 @@ std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T
             uint64_t R = 0, blk = 0;
             for (int k = 0; k < P; ++k) {
                 if (sched[k]) continue;
-                if ((gall[k] & blk) == 0 && popc(R | lreg[k]) <= maxr) {
+                if ((gall[k] & blk) == 0 && popc(R | lreg[k]) <= 4) {
                     R |= lreg[k];
                     rd.ops.push_back(k);
                     sched[k] = 1;
@@ -801,11 +819,10 @@ std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T
             std::vector<int> Rv;
             for (int p = 0; p < T; ++p)
                 if (R >> p & 1) Rv.push_back(p);
-            pad_rpos(Rv, T, maxr);
-            for (int k = 0; k < 4; ++k) rd.rpos[k] = k < maxr ? Rv[k] : T;
+            pad_rpos(Rv, T);
+            for (int k = 0; k < 4; ++k) rd.rpos[k] = Rv[k];
             st.pass.rounds.push_back(rd);
         }
-        steps.push_back(st);
     }
     return steps;
 }
@@ -817,8 +834,7 @@ void fill_round(FusedRound &fr, const int rpos[4], int T, int h) {
             if (e >> k & 1) off |= 1 << rpos[k];
         fr.eoff[e] = swz(off) << 4;
     }
-    // (position T is the selector of a second state: it is no index bit)
-    for (int k = 0; k < 4; ++k) fr.gpos[k] = rpos[k] < T ? 1ull << global_pos(rpos[k], h) : 0ull;
+    for (int k = 0; k < 4; ++k) fr.gpos[k] = 1ull << global_pos(rpos[k], h);
     fr.nlane = choose_lanes(rpos, T, fr.lane);
 }
 

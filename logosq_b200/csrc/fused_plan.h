@@ -25,10 +25,21 @@ struct PlanStep {  // either a fused pass or a standalone gate
     PlannedPass pass;
 };
 
-// Window [0,4) U [h, h+T-4); returns passes and standalone gates in order.  With
-// maxr = 3 a round picks three tile bits and its fourth register bit is tile
-// position T, the selector of a second state in the same tile (adjoint.cu).
-std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T, int maxr = 4);
+// What the choice of windows reads of a gate.
+struct PlanGate {
+    uint64_t bits = 0;     // index bits that it touches
+    uint64_t mixed = 0;    // those that must lie in the window
+    bool fusable = true;
+    bool barrier = false;  // blocks every bit (a renormalising gate)
+};
+PlanGate plan_gate(const GateOp &g);
+
+// Window [0,4) U [h, h+T-4); returns passes and standalone gates in order, the passes
+// without rounds.
+std::vector<PlanStep> plan_windows(const std::vector<PlanGate> &gates, int n, int T);
+std::vector<PlanStep> plan_windows(const std::vector<GateOp> &gops, int n, int T);
+// The same with the rounds of every pass: four tile bits each (op-record engines).
+std::vector<PlanStep> plan_circuit(const std::vector<GateOp> &gops, int n, int T);
 // Round record (element offsets, register bit masks, thread lanes).
 void fill_round(FusedRound &fr, const int rpos[4], int T, int h);
 // Append the register op of gate g in a round with register positions rpos.

@@ -1287,7 +1287,7 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     if (!map_lower(gops, ops, units)) return false;
     std::vector<GateOp> shapes;
     for (const MapUnit &u : units) shapes.push_back(u.shape);
-    const std::vector<PlanStep> steps = plan_circuit(shapes, n, T);
+    const std::vector<PlanStep> steps = plan_windows(shapes, n, T);
     // (a two-qubit rotation across windows would be three passes here, 983 us on 26 qubits
     // where its own sweep takes 317)
     for (const PlanStep &st : steps)

@@ -764,7 +764,7 @@ int apply_circuit_tc_impl(lq_state *s, const lq_gate *ops, int nops, const doubl
             g = w;
         }
     }
-    std::vector<PlanStep> steps = plan_circuit(planner_ops, n, kTcT);
+    std::vector<PlanStep> steps = plan_windows(planner_ops, n, kTcT);
     std::vector<TcBlock> blocks;
     std::vector<TcPass> passes;
     std::vector<unsigned char> bimg;
