@@ -721,35 +721,43 @@ PlanGate plan_gate(const GateOp &g) {
 std::vector<PlanStep> plan_windows(const std::vector<PlanGate> &gates, int n, int T) {
     const int m = T - 4;
     std::vector<PlanStep> steps;
-    const int G = (int)gates.size();
     const uint64_t all = (1ull << n) - 1;
-    std::vector<char> done(G, 0);
-    int remaining = G, first = 0;
-    // The gates that a pass over window W takes, in order (take: mark them done too).
-    auto scan = [&](uint64_t W, std::vector<int> *take) {
+    // the gates not yet in a step, in order
+    struct Left {
+        uint64_t bits, mixed;  // mixed: all ones where the gate fits no window
+        uint64_t blocks;       // what a gate that stays behind keeps others from
+        int gate;
+        bool taken;
+    };
+    std::vector<Left> left;
+    left.reserve(gates.size());
+    for (const PlanGate &g : gates)
+        left.push_back(Left{g.bits, g.fusable ? g.mixed : ~0ull, g.barrier ? all : g.bits,
+                            (int)left.size(), false});
+    // The number of gates that a pass over window W takes (take: into a step); the count of a
+    // window that cannot have more than `enough` is not finished.
+    auto scan = [&](uint64_t W, std::vector<int> *take, int enough) {
         uint64_t blocked = 0;
-        int cnt = 0;
-        for (int i = first; i < G; ++i) {
-            if (done[i]) continue;
-            const PlanGate &g = gates[i];
-            if (g.fusable && (g.mixed & ~W) == 0 && (g.bits & blocked) == 0) {
+        int cnt = 0, unseen = (int)left.size();
+        for (Left &g : left) {
+            if (cnt + unseen-- <= enough) break;
+            if ((g.mixed & ~W) == 0 && (g.bits & blocked) == 0) {
                 ++cnt;
                 if (take) {
-                    take->push_back(i);
-                    done[i] = 1;
+                    take->push_back(g.gate);
+                    g.taken = true;
                 }
             } else {
-                blocked |= g.barrier ? all : g.bits;
+                blocked |= g.blocks;
                 if ((blocked & all) == all) break;
             }
         }
         return cnt;
     };
-    while (remaining > 0) {
-        while (first < G && done[first]) ++first;
+    while (!left.empty()) {
         int best_h = -1, best_cnt = 0;
         for (int h = 4; h + m <= n; ++h) {
-            const int cnt = scan(window_mask(h, m), nullptr);
+            const int cnt = scan(window_mask(h, m), nullptr, best_cnt);
             if (cnt > best_cnt) {
                 best_cnt = cnt;
                 best_h = h;
@@ -758,16 +766,17 @@ std::vector<PlanStep> plan_windows(const std::vector<PlanGate> &gates, int n, in
         PlanStep st;
         if (best_cnt == 0) {
             st.fused = false;
-            st.gate = first;
-            done[first] = 1;
-            --remaining;
+            st.gate = left[0].gate;
+            left[0].taken = true;
         } else {
             st.fused = true;
             st.pass.h = best_h;
             st.pass.gates.reserve(best_cnt);
-            remaining -= scan(window_mask(best_h, m), &st.pass.gates);
+            scan(window_mask(best_h, m), &st.pass.gates, -1);
         }
         steps.push_back(std::move(st));
+        left.erase(std::remove_if(left.begin(), left.end(), [](const Left &g) { return g.taken; }),
+                   left.end());
     }
     return steps;
 }
@@ -1227,10 +1236,14 @@ struct PlanKeyView {
                (!angles() || memcmp(k.data() + sizeof(hdr) + gates(), theta, angles()) == 0);
     }
     std::vector<unsigned char> copy() const {
-        std::vector<unsigned char> k(sizeof(hdr) + gates() + angles());
-        memcpy(k.data(), hdr, sizeof(hdr));
-        if (gates()) memcpy(k.data() + sizeof(hdr), ops, gates());
-        if (angles()) memcpy(k.data() + sizeof(hdr) + gates(), theta, angles());
+        std::vector<unsigned char> k;
+        k.reserve(sizeof(hdr) + gates() + angles());
+        auto put = [&](const void *p, size_t bytes) {
+            if (bytes) k.insert(k.end(), (const unsigned char *)p, (const unsigned char *)p + bytes);
+        };
+        put(hdr, sizeof(hdr));
+        put(ops, gates());
+        put(theta, angles());
         return k;
     }
 };
@@ -1242,6 +1255,8 @@ struct PlanKeyView {
 // does not renormalise itself it stays where it is.  (A zero vector, or one below the
 // 1e-10 threshold, keeps its norm through unitary gates and is left alone either way.)
 static bool defer_renorm(std::vector<GateOp> &gops) {
+    if (std::none_of(gops.begin(), gops.end(), [](const GateOp &g) { return g.renorm; }))
+        return false;
     int last = -1;  // the gate that owes a division
     for (size_t k = 0; k < gops.size(); ++k) {
         GateOp &g = gops[k];

@@ -37,6 +37,7 @@
 #include "mapped.h"
 
 #include <algorithm>
+#include <array>
 #include <complex>
 #include <cstring>
 #include <map>
@@ -387,40 +388,81 @@ __global__ void __launch_bounds__(256, 2)
 // ---------------------------------------------------------------------------
 // Host: gates -> permutations, diagonals, rotations
 // ---------------------------------------------------------------------------
-enum MapOpKind { MO_PERM, MO_DIAG, MO_ROT };
+enum MapOpKind { MO_PERM, MO_SWAP, MO_DIAG, MO_ROT };
 
+// (Small: a circuit becomes some thousand of them, and with the whole GateOp of 360 bytes in
+// each, copying them was a quarter of the planning.)
 struct MapOp {
     int kind;
-    GateOp g;            // bits (what the window planner reads), and the gate of a PERM
-    // MO_DIAG: factor p[v1 << 1 | v0] of bits b1, b0 (b1 < 0: p[0], p[1] of b0 alone)
-    int b0 = -1, b1 = -1;
-    cd p[4];
-    // MO_ROT on bit t: by t0, or by t0 / t1 for control bit c = 0 / 1
-    int t = -1, c = -1;
+    // MO_PERM: X on t, controlled by c if >= 0.  MO_SWAP: b0 and b1.  MO_DIAG: factor
+    // p[v1 << 1 | v0] of bits b1, b0 (b1 < 0: p[0], p[1] of b0 alone).  MO_ROT: bit t by t0, or
+    // by t0 / t1 for control bit c = 0 / 1.
+    int t = -1, c = -1, b0 = -1, b1 = -1;
+    uint64_t bits = 0;   // index bits that it touches
     double t0 = 0.0, t1 = 0.0;
+    cd p[4];
 };
 
+static uint64_t bit_of(int b) { return b >= 0 ? 1ull << b : 0ull; }
+
 static MapOp map_perm_x(int t, int c) {
-    MapOp o{};
+    MapOp o;
     o.kind = MO_PERM;
-    o.g.type = OP_PERM1;
-    o.g.t = t;
-    if (c >= 0) o.g.nctrl = 1, o.g.ctrl[0] = c;
+    o.t = t;
+    o.c = c;
+    o.bits = bit_of(t) | bit_of(c);
     return o;
 }
 
-static MapOp map_diag(int b1, int b0, cd p00, cd p01, cd p10, cd p11) {
-    MapOp o{};
+static MapOp map_diag(int b1, int b0, const cd &p00, const cd &p01, const cd &p10, const cd &p11) {
+    MapOp o;
     o.kind = MO_DIAG;
-    o.g.type = OP_DIAG;
-    o.g.npat = b1 >= 0 ? 2 : 1;
-    o.g.pat[0] = b0;
-    o.g.pat[1] = b1;
     o.b0 = b0;
     o.b1 = b1;
+    o.bits = bit_of(b0) | bit_of(b1);
     o.p[0] = p00, o.p[1] = p01, o.p[2] = p10, o.p[3] = p11;
     return o;
 }
+
+// Arithmetic on finite numbers of ordinary size: std::complex's operators distinguish
+// infinities and scale against overflow, in library calls that were a fifth of the planning.
+static inline cd mul(const cd &a, const cd &b) {
+    return cd(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real());
+}
+static inline real norm2(const cd &a) { return a.real() * a.real() + a.imag() * a.imag(); }
+static inline real length(const cd &a) { return std::sqrt(norm2(a)); }
+static inline cd inverse(const cd &a) {
+    const real d = 1 / norm2(a);
+    return cd(a.real() * d, -a.imag() * d);
+}
+static inline cd root(const cd &a) {  // the principal square root
+    const real r = length(a), h = std::sqrt((r + std::abs(a.real())) / 2);
+    if (h == 0) return cd(0.0);
+    const real g = a.imag() / (2 * h);
+    if (a.real() >= 0) return cd(h, g);
+    return std::signbit(a.imag()) ? cd(-g, -h) : cd(g, h);
+}
+
+// The last few results of a function of four factors: within a circuit the same gates tend to
+// come again (every bond of a Trotter step).
+template <class R>
+struct Recent {
+    static constexpr int kKept = 4;
+    cd key[kKept][4];
+    R value[kKept];
+    int used = 0, next = 0;
+    const R *find(const cd u[4]) const {
+        for (int k = 0; k < used; ++k)
+            if (std::equal(u, u + 4, key[k])) return &value[k];
+        return nullptr;
+    }
+    void put(const cd u[4], const R &r) {
+        std::copy(u, u + 4, key[next]);
+        value[next] = r;
+        used = std::max(used, next + 1);
+        next = (next + 1) % kKept;
+    }
+};
 
 struct MapEuler {
     cd w, phi, lam;
@@ -431,22 +473,23 @@ struct MapEuler {
 
 // u = w diag(1, phi) [X and sign if turned] scale [[1, -t], [t, 1]] diag(1, lam)
 static bool map_euler(const cd u[4], MapEuler &e) {
-    const real ra = std::abs(u[0]), rb = std::abs(u[1]), rc = std::abs(u[2]), rd = std::abs(u[3]);
+    const real ra = length(u[0]), rb = length(u[1]), rc = length(u[2]), rd = length(u[3]);
     if (!(std::abs(ra * ra + rc * rc - 1.0) <= 1e-12 && std::abs(rb - rc) <= 1e-12 &&
           std::abs(ra - rd) <= 1e-12))
         return false;  // not unitary
     constexpr real tiny = 1e-150;
     e.w = ra > tiny ? u[0] / ra : cd(1.0, 0.0);
     if (rc > tiny && rb > tiny) {
-        e.phi = (u[2] / rc) * std::conj(e.w);
-        e.lam = (-u[1] / rb) * std::conj(e.w);
+        e.phi = mul(u[2] / rc, std::conj(e.w));
+        e.lam = mul(-u[1] / rb, std::conj(e.w));
     } else {
         e.phi = 1.0;
-        e.lam = rd > tiny ? (u[3] / rd) * std::conj(e.w) : cd(1.0, 0.0);
+        e.lam = rd > tiny ? mul(u[3] / rd, std::conj(e.w)) : cd(1.0, 0.0);
     }
-    const cd r[4] = {e.w * ra, -e.w * rc * e.lam, e.w * rc * e.phi, e.w * ra * e.phi * e.lam};
+    const cd r[4] = {e.w * ra, mul(-e.w * rc, e.lam), mul(e.w * rc, e.phi),
+                     mul(mul(e.w * ra, e.phi), e.lam)};
     for (int k = 0; k < 4; ++k)
-        if (!(std::abs(r[k] - u[k]) <= 1e-14)) return false;
+        if (!(length(r[k] - u[k]) <= 1e-14)) return false;
     // [[c, -s], [s, c]] with s > c is [[0, -1], [1, 0]] [[s, c], [-c, s]]
     e.turned = rc > ra;
     e.t = (double)(e.turned ? -ra / rc : rc / ra);
@@ -456,26 +499,35 @@ static bool map_euler(const cd u[4], MapEuler &e) {
 }
 
 // One 2x2 (A on bit t), or A / B for control bit c = 0 / 1.
-static bool map_rotation(const cd A[4], const cd B[4], int t, int c, std::vector<MapOp> &out) {
+static bool map_rotation(const cd A[4], const cd B[4], int t, int c, Recent<MapEuler> &recent,
+                         std::vector<MapOp> &out) {
+    auto euler = [&](const cd u[4], MapEuler &e) {
+        if (const MapEuler *r = recent.find(u)) {
+            e = *r;
+            return true;
+        }
+        if (!map_euler(u, e)) return false;
+        recent.put(u, e);
+        return true;
+    };
     MapEuler a, b;
-    if (!map_euler(A, a)) return false;
+    if (!euler(A, a)) return false;
     if (c < 0) b = a;
-    else if (!map_euler(B, b)) return false;
-    auto diag = [&](cd a0, cd a1, cd b0, cd b1) {  // factors of t = 0 / 1 under A and under B
+    else if (!euler(B, b)) return false;
+    // factors of t = 0 / 1 under A and under B
+    auto diag = [&](const cd &a0, const cd &a1, const cd &b0, const cd &b1) {
         if (c < 0) out.push_back(map_diag(-1, t, a0, a1, 0.0, 0.0));
         else out.push_back(map_diag(c, t, a0, a1, b0, b1));
     };
     diag(1.0, a.lam, 1.0, b.lam);
     if (a.t != 0.0 || b.t != 0.0) {
-        MapOp o{};
+        MapOp o;
         o.kind = MO_ROT;
         o.t = t;
         o.c = a.t == b.t ? -1 : c;  // (RXX, RYY: the two differ in their diagonals only)
+        o.bits = bit_of(t) | bit_of(o.c);
         o.t0 = a.t;
         o.t1 = b.t;
-        o.g.type = OP_M1;
-        o.g.t = t;
-        if (o.c >= 0) o.g.nctrl = 1, o.g.ctrl[0] = c;
         out.push_back(o);
     }
     // the quarter turn: X on t (where it applies), then diag(-1, 1)
@@ -486,12 +538,8 @@ static bool map_rotation(const cd A[4], const cd B[4], int t, int c, std::vector
         if (a.turned != b.turned) out.push_back(map_perm_x(t, c));
     }
     const cd wa = a.w * a.scale, wb = b.w * b.scale;
-    diag(wa * (a.turned ? real(-1) : real(1)), wa * a.phi, wb * (b.turned ? real(-1) : real(1)), wb * b.phi);
+    diag(a.turned ? -wa : wa, mul(wa, a.phi), b.turned ? -wb : wb, mul(wb, b.phi));
     return true;
-}
-
-static inline cd mul(const cd &a, const cd &b) {  // (finite: no case distinctions)
-    return cd(a.real() * b.real() - a.imag() * b.imag(), a.real() * b.imag() + a.imag() * b.real());
 }
 
 static cd coef(const double *m, int k) { return cd(m[2 * k], m[2 * k + 1]); }
@@ -517,13 +565,14 @@ static bool map_single(const GateOp &g, int &bit, cd u[4], bool &diag) {
     return false;
 }
 
-static bool unit(cd z) { return std::abs(std::abs(z) - 1.0) <= 1e-12; }
+static bool unit(const cd &z) { return std::abs(length(z) - 1) <= 1e-12; }
 
 // What the window planner sees: a gate or a run of single-qubit gates, with the map ops
 // that it became.  (Planned op by op, a 2x2 with a quarter turn counted twice, and 60
 // single-qubit gates on 24 qubits took five passes instead of three: 480 us, now 326.)
 struct MapUnit {
-    GateOp shape;
+    PlanGate shape;
+    const GateOp *swap;  // the gate if it is a SWAP
     int begin, end;
 };
 
@@ -541,7 +590,10 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
     };
     std::vector<Run> runs;
     std::vector<Entry> list;
-    std::vector<int> open(64, -1);
+    int open[64];
+    std::fill(open, open + 64, -1);
+    runs.reserve(gops.size());
+    list.reserve(gops.size());
     for (const GateOp &g : gops) {
         if (g.renorm) return false;
         int bit;
@@ -550,8 +602,10 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
         if (map_single(g, bit, u, diag)) {
             if (open[bit] >= 0) {
                 Run &r = runs[open[bit]];
-                const cd p[4] = {u[0] * r.u[0] + u[1] * r.u[2], u[0] * r.u[1] + u[1] * r.u[3],
-                                 u[2] * r.u[0] + u[3] * r.u[2], u[2] * r.u[1] + u[3] * r.u[3]};
+                const cd p[4] = {mul(u[0], r.u[0]) + mul(u[1], r.u[2]),
+                                 mul(u[0], r.u[1]) + mul(u[1], r.u[3]),
+                                 mul(u[2], r.u[0]) + mul(u[3], r.u[2]),
+                                 mul(u[2], r.u[1]) + mul(u[3], r.u[3])};
                 std::copy(p, p + 4, r.u);
                 r.diag = r.diag && diag;
                 r.x = false;
@@ -562,43 +616,45 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
             }
             continue;
         }
-        const uint64_t bits = op_bits(g);
-        for (int b = 0; b < 64; ++b)
-            if (bits >> b & 1) open[b] = -1;
+        for (uint64_t bits = op_bits(g); bits; bits &= bits - 1) open[__builtin_ctzll(bits)] = -1;
         list.push_back(Entry{-1, &g});
     }
+    Recent<MapEuler> recent;
+    out.reserve(3 * list.size());
+    units.reserve(list.size());
     for (const Entry &en : list) {
         if (!units.empty()) units.back().end = (int)out.size();
-        units.push_back(MapUnit{GateOp{}, (int)out.size(), 0});
-        GateOp &shape = units.back().shape;
+        units.push_back(MapUnit{PlanGate{}, nullptr, (int)out.size(), 0});
+        PlanGate &shape = units.back().shape;
         if (en.run >= 0) {
             const Run &r = runs[en.run];
+            shape.bits = bit_of(r.bit);
+            shape.mixed = r.diag ? 0 : shape.bits;
             if (r.x) {
                 out.push_back(map_perm_x(r.bit, -1));
-                shape = out.back().g;
             } else if (r.diag) {
                 if (!unit(r.u[0]) || !unit(r.u[3])) return false;
                 out.push_back(map_diag(-1, r.bit, r.u[0], r.u[3], 0.0, 0.0));
-                shape = out.back().g;
-            } else {
-                if (!map_rotation(r.u, r.u, r.bit, -1, out)) return false;
-                shape.type = OP_M1;
-                shape.t = r.bit;
+            } else if (!map_rotation(r.u, r.u, r.bit, -1, recent, out)) {
+                return false;
             }
             continue;
         }
         const GateOp &g = *en.g;
-        shape = g;
+        shape = plan_gate(g);
         switch (g.type) {
         case OP_PERM1:
             if (g.nctrl != 1) return false;
             out.push_back(map_perm_x(g.t, g.ctrl[0]));
             break;
         case OP_SWAP: {
-            MapOp o{};
-            o.kind = MO_PERM;
-            o.g = g;
+            MapOp o;
+            o.kind = MO_SWAP;
+            o.b0 = g.b0;
+            o.b1 = g.b1;
+            o.bits = bit_of(g.b0) | bit_of(g.b1);
             out.push_back(o);
+            units.back().swap = &g;
             break;
         }
         case OP_DIAG: {
@@ -626,7 +682,7 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
             if (g.nctrl != 1) return false;
             const cd id[4] = {1.0, 0.0, 0.0, 1.0};
             const cd u[4] = {coef(g.m, 0), coef(g.m, 1), coef(g.m, 2), coef(g.m, 3)};
-            if (!map_rotation(id, u, g.t, g.ctrl[0], out)) return false;
+            if (!map_rotation(id, u, g.t, g.ctrl[0], recent, out)) return false;
             break;
         }
         case OP_M2: {
@@ -638,7 +694,7 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
             const cd A[4] = {coef(g.m, 0), coef(g.m, 3), coef(g.m, 12), coef(g.m, 15)};
             const cd B[4] = {coef(g.m, 5), coef(g.m, 6), coef(g.m, 9), coef(g.m, 10)};
             out.push_back(map_perm_x(g.b1, g.b0));
-            if (!map_rotation(A, B, g.b0, g.b1, out)) return false;
+            if (!map_rotation(A, B, g.b0, g.b1, recent, out)) return false;
             out.push_back(map_perm_x(g.b1, g.b0));
             break;
         }
@@ -652,7 +708,7 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
 // ---------------------------------------------------------------------------
 // Host: passes
 // ---------------------------------------------------------------------------
-static inline int par(uint64_t x) { return __builtin_popcountll(x) & 1; }
+static inline int par(uint64_t x) { return __builtin_parityll(x); }
 
 // Waiting diagonal factors z^parity(mask & place), and one number for all amplitudes.
 struct Waiting {
@@ -663,20 +719,38 @@ struct Waiting {
     };
     std::vector<Item> items;
     cd scalar = 1.0;
-    void add(uint64_t mask, cd z, int slot) {
+    bool twice = false;  // a mask may be there for two slots
+    uint64_t seen[4] = {0, 0, 0, 0};  // hashes of the masks (of some that left, too)
+    static unsigned hash(uint64_t mask) { return (unsigned)(mask * 0x9E3779B97F4A7C15ull >> 56); }
+    bool see(uint64_t mask) {
+        const unsigned k = hash(mask);
+        const bool was = seen[k >> 6] >> (k & 63) & 1;
+        seen[k >> 6] |= 1ull << (k & 63);
+        return was;
+    }
+    void clear() {
+        items.clear();
+        std::fill(seen, seen + 4, 0);
+        twice = false;
+    }
+    void add(uint64_t mask, const cd &z, int slot) {
         if (mask == 0 || z == cd(1.0)) return;
-        for (Item &i : items)
-            if (i.mask == mask && i.slot == slot) {
-                i.z *= z;
-                return;
+        if (see(mask))
+            for (Item &i : items) {
+                if (i.mask != mask) continue;
+                if (i.slot == slot) {
+                    i.z = mul(i.z, z);
+                    return;
+                }
+                twice = true;
             }
         items.push_back(Item{mask, z, slot});
     }
     // z^(parity(mask) ^ flip)
     void add1(uint64_t mask, int flip, cd z, int slot) {
         if (flip) {
-            scalar *= z;
-            z = real(1) / z;
+            scalar = mul(scalar, z);
+            z = inverse(z);
         }
         add(mask, z, slot);
     }
@@ -709,21 +783,21 @@ public:
     }
 
     // A permutation whose target lies in the window; false when the map is full.
-    bool permute(const GateOp &g) {
-        if (g.type == OP_SWAP) {
-            const int x = local_pos(g.b0, h), y = local_pos(g.b1, h);
+    bool permute(const MapOp &o) {
+        if (o.kind == MO_SWAP) {
+            const int x = local_pos(o.b0, h), y = local_pos(o.b1, h);
             std::swap(vec[x], vec[y]);
             std::swap(row[x], row[y]);
             std::swap(flip[x], flip[y]);
             return true;
         }
-        const int t = local_pos(g.t, h);
-        if (g.nctrl == 0) {
+        const int t = local_pos(o.t, h);
+        if (o.c < 0) {
             base ^= vec[t];
             flip[t] ^= 1;
             return true;
         }
-        const int c = g.ctrl[0];
+        const int c = o.c;
         if (inside(c)) {
             const int lc = local_pos(c, h);
             vec[lc] ^= vec[t];
@@ -753,19 +827,35 @@ public:
         int f0, f1 = 0;
         const uint64_t m0 = functional(o.b0, f0);
         if (o.b1 < 0) {
-            wait.scalar *= o.p[0];
-            wait.add1(m0, f0, o.p[1] / o.p[0], slot);
+            wait.scalar = mul(wait.scalar, o.p[0]);
+            wait.add1(m0, f0, o.p[1] == o.p[0] ? cd(1.0) : mul(o.p[1], inverse(o.p[0])), slot);
             return;
         }
         // p[v1 v0] = p00 z1^v1 z0^v0 z2^(v1 ^ v0)
         const uint64_t m1 = functional(o.b1, f1);
-        const cd q01 = o.p[1] / o.p[0], q10 = o.p[2] / o.p[0], q11 = o.p[3] / o.p[0];
-        wait.scalar *= o.p[0];
-        const cd z1 = std::sqrt(q10 * q11 / q01);
-        const cd z2 = q10 / z1, z0 = q01 / z2;
-        wait.add1(m1, f1, z1, slot);
-        wait.add1(m0, f0, z0, slot);
-        wait.add1(m0 ^ m1, f0 ^ f1, z2, slot);
+        wait.scalar = mul(wait.scalar, o.p[0]);
+        // (equal factors are compared as such, so that what is 1 is 1 to the bit and left out)
+        if (o.p[1] == o.p[0] && o.p[2] == o.p[0] && o.p[3] == o.p[0]) return;
+        Split z;
+        if (const Split *r = splits.find(o.p)) {
+            z = *r;
+        } else {
+            const cd i0 = inverse(o.p[0]);
+            cd q[4];
+            for (int k = 1; k < 4; ++k) q[k] = o.p[k] == o.p[0] ? cd(1.0) : mul(o.p[k], i0);
+            if (q[1] == q[2]) {
+                z.z0 = z.z1 = root(q[3]);
+                z.z2 = z.z1 == cd(1.0) ? q[2] : mul(q[2], inverse(z.z1));
+            } else {
+                z.z1 = root(mul(mul(q[2], q[3]), inverse(q[1])));
+                z.z2 = mul(q[2], inverse(z.z1));
+                z.z0 = mul(q[1], inverse(z.z2));
+            }
+            splits.put(o.p, z);
+        }
+        wait.add1(m1, f1, z.z1, slot);
+        wait.add1(m0, f0, z.z0, slot);
+        wait.add1(m0 ^ m1, f0 ^ f1, z.z2, slot);
     }
 
     // A round of the given rotations in planning.
@@ -778,17 +868,31 @@ public:
         int bflip;
         std::vector<Waiting::Item> tables;
     };
-    std::vector<Slot> slots;
+    // (their tables keep their memory from round to round)
+    struct Slots {
+        Slot s[4];
+        size_t n = 0;
+        size_t size() const { return n; }
+        bool empty() const { return n == 0; }
+        Slot *begin() { return s; }
+        Slot *end() { return s + n; }
+        const Slot *begin() const { return s; }
+        const Slot *end() const { return s + n; }
+        Slot &operator[](size_t k) { return s[k]; }
+        const Slot &operator[](size_t k) const { return s[k]; }
+    };
+    Slots slots;
 
     bool independent(uint32_t v) const {
-        std::vector<uint32_t> basis;
+        uint32_t basis[4];
+        int nb = 0;
         auto reduce = [&](uint32_t x) {
-            for (uint32_t b : basis) x = std::min(x, x ^ b);
+            for (int k = 0; k < nb; ++k) x = std::min(x, x ^ basis[k]);
             return x;
         };
         for (const Slot &s : slots) {
             const uint32_t x = reduce(s.v);
-            if (x) basis.push_back(x);
+            if (x) basis[nb++] = x;
         }
         return reduce(v) != 0;
     }
@@ -807,17 +911,19 @@ public:
 
     // Whether the round's rotations so far are plain and its factors one table's.
     bool line_so_far() const {
-        std::vector<uint64_t> parts;
-        uint64_t rest = ~0ull;
+        uint64_t parts[kMapParts], rest = ~0ull;
+        int np = 0;
         for (const Slot &s : slots) {
             if (s.ctrl || (&s != &slots[0] && !s.tables.empty())) return false;
             rest &= ~s.bit;
         }
         for (const auto &it : slots[0].tables) {
             const uint64_t p = it.mask & rest;
-            if (p && std::find(parts.begin(), parts.end(), p) == parts.end()) parts.push_back(p);
+            if (!p || std::find(parts, parts + np, p) != parts + np) continue;
+            if (np == kMapParts) return false;
+            parts[np++] = p;
         }
-        return (int)parts.size() <= kMapParts;
+        return true;
     }
 
     // Add the rotation to the round if its vector is free; the factors that it does
@@ -825,14 +931,16 @@ public:
     bool rotate(const MapOp &o) {
         const uint32_t v = vec[local_pos(o.t, h)];
         if (slots.size() == 4 || !independent(v)) return false;
-        Slot s{};
+        const int k = (int)slots.n++;
+        Slot &s = slots[k];
         s.v = v;
         s.t0 = o.t0;
         s.t1 = o.t1;
+        s.ctrl = 0;
+        s.cflip = 0;
         s.bit = functional(o.t, s.bflip);
         if (o.c >= 0) s.ctrl = functional(o.c, s.cflip);
-        slots.push_back(s);
-        const int k = (int)slots.size() - 1;
+        s.tables.clear();
         const uint64_t gv = spread(v);
         // A round that is one straight line so far stays one: a rotation that needs a
         // table of its own after the first rotation opens the next round.  (28-qubit
@@ -841,20 +949,18 @@ public:
         if (k > 0 && o.c < 0 && line_so_far()) {
             for (const auto &it : wait.items) {
                 if (par(it.mask & gv) && earliest(it, k) > 0) {
-                    slots.pop_back();
+                    --slots.n;
                     return false;
                 }
             }
         }
-        std::vector<Waiting::Item> keep;
-        for (const auto &it : wait.items) {
-            if (!par(it.mask & gv)) {
-                keep.push_back(it);
-                continue;
-            }
-            slots[earliest(it, k)].tables.push_back(it);
+        size_t keep = 0;
+        for (size_t q = 0; q < wait.items.size(); ++q) {
+            const Waiting::Item &it = wait.items[q];
+            if (par(it.mask & gv)) slots[earliest(it, k)].tables.push_back(it);
+            else if (keep++ != q) wait.items[keep - 1] = it;
         }
-        wait.items = std::move(keep);
+        wait.items.resize(keep);
         return true;
     }
 
@@ -867,18 +973,23 @@ public:
             return;
         }
         // One round, or as many as their tables make of it
-        std::vector<Slot> all = std::move(slots);
-        for (size_t at = 0, to; at < all.size() || tail; at = to) {
-            to = all.size();
-            for (;;) {
-                slots.assign(all.begin() + at, all.begin() + to);
+        size_t to = emit_round(tail);
+        if (to < slots.size()) {
+            const Slots all = slots;
+            for (size_t at = 0;;) {
+                slots.n = to - at;
+                std::copy(all.begin() + at, all.begin() + to, slots.begin());
                 const size_t stop = at + emit_round(tail && to == all.size());
-                if (stop == to) break;
-                to = stop;
+                if (stop < to) {
+                    to = stop;
+                    continue;
+                }
+                if (to == all.size()) break;
+                at = to;
+                to = all.size();
             }
-            if (to == all.size()) break;
         }
-        slots.clear();
+        slots.n = 0;
         begin_next();
     }
 
@@ -890,24 +1001,25 @@ public:
         MapRound rd{};
         // register vectors: the rotations', then tile bits that leave the threads' bits
         // on different banks
-        std::vector<uint32_t> reg;
-        for (const Slot &s : slots) reg.push_back(s.v);
+        uint32_t reg[4];
         uint32_t piv = 0;  // one pivot bit per vector: thread bases are 0 there
         {
             Reduced red;
-            for (uint32_t v : reg) add_pivot(red, piv, v);
-            while (reg.size() < 4) {
+            Ranks ranks;
+            for (int b = 0; b < T; ++b) ranks.free(banks[b] = bank(b));
+            int nreg = 0;
+            for (const Slot &s : slots) add_pivot(red, ranks, piv, reg[nreg++] = s.v);
+            while (nreg < 4) {
                 int best = -1, best_rank = -1;
                 for (int b = T - 1; b >= 0; --b) {
                     if (piv >> b & 1) continue;
                     // (bits that no rotated bit depends on keep the sign per thread)
-                    int r = bank_rank(piv | 1u << b);
+                    int r = ranks.without(banks[b]);
                     for (const Slot &s : slots)
                         if (!par(s.bit & spread(1u << b))) r += 4;
                     if (r > best_rank) best = b, best_rank = r;
                 }
-                reg.push_back(1u << best);
-                add_pivot(red, piv, 1u << best);
+                add_pivot(red, ranks, piv, reg[nreg++] = 1u << best);
             }
         }
         for (int k = 0; k < 4; ++k) rd.vec[k] = (uint32_t)mswz((int)place(reg[k])) << 4;
@@ -917,23 +1029,29 @@ public:
         uint64_t shared = 0;
         for (const Slot &s : slots)
             for (const auto &it : s.tables) shared |= it.mask & ~off_base;
-        std::vector<int> lanes, rest, last;
+        int lanes[kMaxT], rest[kMaxT], last[kMaxT], nlane = 0, nrest = 0, nlast = 0;
         uint32_t basis[3] = {0, 0, 0};
         for (int b = 0; b < T; ++b) {
             if (piv >> b & 1) continue;
-            if (shared & spread(1u << b)) last.push_back(b);
-            else (bank_add(basis, bank(b)) ? lanes : rest).push_back(b);
+            if (shared & spread(1u << b)) last[nlast++] = b;
+            else if (bank_add(basis, banks[b])) lanes[nlane++] = b;
+            else rest[nrest++] = b;
         }
-        lanes.insert(lanes.end(), rest.begin(), rest.end());
-        if (lanes.size() < 5) {  // too many: some are thread bits all the same
-            for (int b : last)
-                if (bank_add(basis, bank(b))) lanes.insert(lanes.begin(), b);
-            for (int b : last)
-                if (std::find(lanes.begin(), lanes.end(), b) == lanes.end()) lanes.push_back(b);
+        for (int k = 0; k < nrest; ++k) lanes[nlane++] = rest[k];
+        if (nlane < 5) {  // too many: some are thread bits all the same
+            for (int k = 0; k < nlast; ++k) {
+                if (!bank_add(basis, banks[last[k]])) continue;
+                std::copy_backward(lanes, lanes + nlane, lanes + nlane + 1);
+                lanes[0] = last[k];
+                ++nlane;
+            }
+            for (int k = 0; k < nlast; ++k)
+                if (std::find(lanes, lanes + nlane, last[k]) == lanes + nlane)
+                    lanes[nlane++] = last[k];
         } else {
-            lanes.insert(lanes.end(), last.begin(), last.end());
+            for (int k = 0; k < nlast; ++k) lanes[nlane++] = last[k];
         }
-        for (size_t j = 0; j < lanes.size(); ++j) {
+        for (int j = 0; j < nlane; ++j) {
             rd.lane[j] = (uint32_t)mswz((int)place_of[lanes[j]]) << 4;
             rd.lane_bit[j] = 1u << lanes[j];
         }
@@ -948,47 +1066,40 @@ public:
         uint64_t gp[4];
         for (int k = 0; k < 4; ++k) gp[k] = spread(reg[k]);
         auto elements = [&](uint64_t mask) {
+            constexpr uint32_t on[4] = {0xAAAAu, 0xCCCCu, 0xF0F0u, 0xFF00u};  // elements with bit k
             uint32_t w = 0;
-            for (int e = 0; e < 16; ++e) {
-                int p = 0;
-                for (int k = 0; k < 4; ++k)
-                    if (e >> k & 1) p ^= par(mask & gp[k]);
-                w |= (uint32_t)p << e;
-            }
+            for (int k = 0; k < 4; ++k) w ^= on[k] & (0u - (uint32_t)par(mask & gp[k]));
             return w;
         };
         auto thread_part = [&](uint64_t mask) { return mask & ~off_base; };
-        struct Part {
-            uint32_t word;
-            cd z;
-        };
         auto tables = [&](const std::vector<Waiting::Item> &items, bool scalar, int &count,
                           int &first) {
             first = (int)tabs.size();
             count = 0;
-            std::vector<Part> fixed;                                  // no thread part
-            std::vector<std::pair<uint64_t, std::vector<Part>>> groups;  // by thread part
+            parts.clear();
+            groups.clear();
+            bool fixed = false;  // some item has no thread part
             for (const auto &it : items) {
-                const Part p{elements(it.mask), it.z};
                 const uint64_t tp = thread_part(it.mask);
-                if (!tp) {
-                    fixed.push_back(p);
-                    continue;
+                int g = -1;
+                if (tp) {
+                    g = (int)(std::find(groups.begin(), groups.end(), tp) - groups.begin());
+                    if (g == (int)groups.size()) groups.push_back(tp);
                 }
-                auto g = std::find_if(groups.begin(), groups.end(),
-                                      [&](auto &x) { return x.first == tp; });
-                if (g == groups.end()) groups.push_back({tp, {p}});
-                else g->second.push_back(p);
+                fixed = fixed || g < 0;
+                parts.push_back(Part{g, elements(it.mask), it.z});
             }
             cd sc = scalar ? wait.scalar : cd(1.0);
             if (scalar) wait.scalar = 1.0;
             if (groups.size() > kMapParts) {
                 // many thread parts: two factors made by the thread for each pattern over
                 // the elements that has more than one item
+                std::stable_sort(parts.begin(), parts.end(),
+                                 [](const Part &x, const Part &y) { return x.group < y.group; });
                 std::map<uint32_t, std::vector<MapItem>> by_word;
-                for (auto &g : groups)
-                    for (auto &p : g.second)
-                        by_word[p.word].push_back(MapItem{g.first, (double)p.z.real(),
+                for (const Part &p : parts)
+                    if (p.group >= 0)
+                        by_word[p.word].push_back(MapItem{groups[p.group], (double)p.z.real(),
                                                           (double)p.z.imag(), 0.0});
                 for (auto &bw : by_word) {
                     if (bw.second.size() < 2 && bw.first != 0) continue;
@@ -1002,51 +1113,75 @@ public:
                     memcpy(data.data() + o, bw.second.data(), bw.second.size() * sizeof(MapItem));
                     tabs.push_back(tb);
                     ++count;
-                    for (auto &g : groups)
-                        g.second.erase(std::remove_if(g.second.begin(), g.second.end(),
-                                                      [&](const Part &p) {
-                                                          return p.word == bw.first;
-                                                      }),
-                                       g.second.end());
+                    parts.erase(std::remove_if(parts.begin(), parts.end(),
+                                               [&](const Part &p) {
+                                                   return p.group >= 0 && p.word == bw.first;
+                                               }),
+                                parts.end());
                 }
-                groups.erase(std::remove_if(groups.begin(), groups.end(),
-                                            [](auto &g) { return g.second.empty(); }),
-                             groups.end());
+                // the groups that are left, in their order
+                std::vector<uint64_t> kept;
+                int last = -1;
+                for (Part &p : parts) {
+                    if (p.group < 0) continue;
+                    if (p.group != last) {
+                        last = p.group;
+                        kept.push_back(groups[last]);
+                    }
+                    p.group = (int)kept.size() - 1;
+                }
+                groups.swap(kept);
             }
             // tables of up to kMapParts thread parts, the first with what depends on none
-            size_t gi = 0;
+            int gi = 0;
+            const int ng = (int)groups.size();
             bool first_table = true;
-            while (gi < groups.size() || (first_table && (!fixed.empty() || sc != cd(1.0)))) {
-                const int nv = (int)std::min<size_t>(kMapParts, groups.size() - gi);
+            while (gi < ng || (first_table && (fixed || sc != cd(1.0)))) {
+                const int nv = std::min(kMapParts, ng - gi);
                 MapTable tb{};
                 tb.data = (int)(data.size() / 2);
                 tb.count = nv;
-                for (int q = 0; q < nv; ++q) tb.m[q] = groups[gi + q].first;
-                const size_t o = data.size();
-                data.resize(o + (size_t)(1 << nv) * kMapVariant * 2, 0.0);
+                for (int q = 0; q < nv; ++q) tb.m[q] = groups[gi + q];
                 // variants of no part first, then doubled with each part
-                cd f[(1 << kMapParts) * kMapVariant];
-                for (int e = 0; e < 16; ++e) {
-                    f[e] = first_table ? sc : cd(1.0);
-                    if (first_table)
-                        for (const Part &p : fixed)
-                            if (p.word >> e & 1) f[e] = mul(f[e], p.z);
+                real fr[(1 << kMapParts) * kMapVariant], fi[(1 << kMapParts) * kMapVariant];
+                auto times = [&](int k, const cd &z) {
+                    const real x = fr[k], y = fi[k];
+                    fr[k] = x * z.real() - y * z.imag();
+                    fi[k] = x * z.imag() + y * z.real();
+                };
+                for (int e = 0; e < kMapVariant; ++e) {
+                    fr[e] = first_table ? sc.real() : 1;
+                    fi[e] = first_table ? sc.imag() : 0;
                 }
-                for (int q = 0; q < nv; ++q)
-                    for (int e = 0; e < 16; ++e) {
-                        cd z[2] = {1.0, 1.0};
-                        for (const Part &p : groups[gi + q].second) {
-                            cd &w = z[(p.word >> e & 1) ^ 1];
-                            w = mul(w, p.z);
-                        }
-                        for (int v = 0; v < (1 << q); ++v) {
-                            f[((v | 1 << q) * kMapVariant) + e] = mul(f[v * kMapVariant + e], z[1]);
-                            f[v * kMapVariant + e] = mul(f[v * kMapVariant + e], z[0]);
+                if (first_table && fixed)
+                    for (const Part &p : parts)
+                        for (int e = 0; p.group < 0 && e < kMapVariant; ++e)
+                            if (p.word >> e & 1) times(e, p.z);
+                for (int q = 0; q < nv; ++q) {
+                    // a part's factors over the patterns of its items, then on the variants
+                    // (elements where the pattern is 0 have them where the thread part is 1)
+                    const int half = kMapVariant << q;
+                    std::copy(fr, fr + half, fr + half);
+                    std::copy(fi, fi + half, fi + half);
+                    cd z[2][kMapVariant];  // 0: none
+                    for (const Part &p : parts) {
+                        if (p.group != gi + q) continue;
+                        for (int e = 0; e < kMapVariant; ++e) {
+                            cd &w = z[(p.word >> e & 1) ^ 1][e];
+                            w = w == cd(0.0) ? p.z : mul(w, p.z);
                         }
                     }
-                for (int k = 0; k < (1 << nv) * kMapVariant; ++k) {
-                    data[o + 2 * k] = (double)f[k].real();
-                    data[o + 2 * k + 1] = (double)f[k].imag();
+                    for (int v = 0; v < 2; ++v)
+                        for (int e = 0; e < kMapVariant; ++e)
+                            if (z[v][e] != cd(0.0))
+                                for (int k = 0; k < half; k += kMapVariant)
+                                    times(v * half + k + e, z[v][e]);
+                }
+                const size_t o = data.size(), count_f = (size_t)kMapVariant << nv;
+                data.resize(o + 2 * count_f);
+                for (size_t k = 0; k < count_f; ++k) {
+                    data[o + 2 * k] = (double)fr[k];
+                    data[o + 2 * k + 1] = (double)fi[k];
                 }
                 tabs.push_back(tb);
                 ++count;
@@ -1076,7 +1211,7 @@ public:
             tables(s.tables, !s.tables.empty() || !(a > 1e-30 && a < 1e30), d.ntab, d.tab);
         }
         uint32_t in_warp = 0;  // tile bits that differ between threads of a warp
-        for (size_t j = 0; j < std::min<size_t>(lanes.size(), 5); ++j) in_warp |= 1u << lanes[j];
+        for (int j = 0; j < std::min(nlane, 5); ++j) in_warp |= 1u << lanes[j];
         auto mark = [&](size_t from) {  // kinds 0 and 2
             for (size_t k = from; k < tabs.size(); ++k)
                 for (int q = 0; q < tabs[k].count && tabs[k].kind == 0; ++q)
@@ -1116,7 +1251,7 @@ public:
         }
         if (tail) {
             tables(wait.items, true, rd.ntail, rd.tail);
-            wait.items.clear();
+            wait.clear();
             mark((size_t)rd.tail);
         }
         for (int k = 0; k < rd.nslot; ++k) rd.signs |= rd.slot[k].smask != 0;
@@ -1180,22 +1315,39 @@ private:
     // The round's permutations join the map, and the waiting factors are written over
     // the indices that they leave.
     void begin_next() {
-        std::vector<Waiting::Item> old = std::move(wait.items);
-        wait.items.clear();
-        for (const auto &it : old) {
-            uint64_t mk = 0;
-            for (int b = 0; b < n; ++b) {
-                int v;
-                if (inside(b)) {
-                    v = par(it.mask & spread(vec[local_pos(b, h)]));
-                } else {
-                    v = (int)(it.mask >> b & 1);
-                    for (auto &c : cst)
-                        if (c.first == b) v ^= par(it.mask & spread(c.second));
+        // col[j]: what a mask's tile bit j becomes; bit 63 stands for a factor turned round
+        constexpr uint64_t kTurn = 1ull << 63;
+        uint64_t col[kMaxT];
+        for (int j = 0; j < T; ++j) {
+            uint64_t c = base >> j & 1 ? kTurn : 0;
+            for (int b = 0; b < T; ++b)
+                if (vec[b] >> j & 1) c |= 1ull << global_pos(b, h);
+            for (auto &x : cst)
+                if (x.second >> j & 1) c ^= 1ull << x.first;
+            col[j] = c;
+        }
+        const uint64_t in = window_mask(h, m);
+        const bool twice = wait.twice;
+        later.swap(wait.items);
+        wait.clear();
+        for (const auto &it : later) {
+            uint64_t mk = it.mask & ~in;
+            for (uint64_t x = it.mask & in; x; x &= x - 1)
+                mk ^= col[local_pos(__builtin_ctzll(x), h)];
+            const bool turn = mk & kTurn;
+            mk &= ~kTurn;
+            // (the map is one to one: masks meet only if they did before)
+            if (twice) {
+                wait.add1(mk, turn, it.z, 0);
+            } else if (it.z != cd(1.0)) {
+                cd z = it.z;
+                if (turn) {
+                    wait.scalar = mul(wait.scalar, z);
+                    z = inverse(z);
                 }
-                if (v) mk |= 1ull << b;
+                wait.see(mk);
+                wait.items.push_back(Waiting::Item{mk, z, 0});
             }
-            wait.add1(mk, par(it.mask & spread(base)), it.z, 0);
         }
         uint32_t next[kMaxT];
         for (int b = 0; b < T; ++b) next[b] = place(vec[b]);
@@ -1223,28 +1375,46 @@ private:
         }
         return false;
     }
-    int bank_rank(uint32_t taken) const {
-        uint32_t basis[3] = {0, 0, 0};
-        int r = 0;
-        for (int b = 0; b < T; ++b)
-            if (!(taken >> b & 1) && bank_add(basis, bank(b))) ++r;
-        return r;
-    }
+    // How many of the banks' three dimensions the bits not yet taken span.
+    struct Ranks {
+        int count[8] = {0}, present = 0;  // free bits by bank
+        void free(uint32_t v) { present |= 1 << v, ++count[v]; }
+        void take(uint32_t v) {
+            if (--count[v] == 0) present &= ~(1 << v);
+        }
+        int without(uint32_t v) const { return rank(count[v] > 1 ? present : present & ~(1 << v)); }
+        static int rank(int set) {  // of vectors 0-7
+            static const auto table = [] {
+                std::array<unsigned char, 256> t{};
+                for (int s = 0; s < 256; ++s) {
+                    uint32_t basis[3] = {0, 0, 0};
+                    for (uint32_t v = 0; v < 8; ++v) t[s] += (s >> v & 1) && bank_add(basis, v);
+                }
+                return t;
+            }();
+            return table[set];
+        }
+    };
     // Gaussian elimination: a pivot bit for v that no earlier vector has, chosen so that
     // the bits left to the threads keep spanning the banks.
-    using Reduced = std::vector<std::pair<uint32_t, int>>;  // vector, its pivot
-    void add_pivot(Reduced &red, uint32_t &piv, uint32_t v) const {
-        for (const auto &r : red)
-            if (v >> r.second & 1) v ^= r.first;
+    struct Reduced {  // vectors and their pivots
+        uint32_t v[4];
+        int at[4], n = 0;
+    };
+    void add_pivot(Reduced &red, Ranks &ranks, uint32_t &piv, uint32_t v) const {
+        for (int k = 0; k < red.n; ++k)
+            if (v >> red.at[k] & 1) v ^= red.v[k];
         int best = -1, best_rank = -1;
         for (int b = T - 1; b >= 0; --b) {
             if (!(v >> b & 1)) continue;
-            const int rk = bank_rank(piv | 1u << b);
+            const int rk = ranks.without(banks[b]);
             if (rk > best_rank) best = b, best_rank = rk;
         }
-        for (auto &r : red)
-            if (r.first >> best & 1) r.first ^= v;
-        red.push_back({v, best});
+        ranks.take(banks[best]);
+        for (int k = 0; k < red.n; ++k)
+            if (red.v[k] >> best & 1) red.v[k] ^= v;
+        red.v[red.n] = v;
+        red.at[red.n++] = best;
         piv |= 1u << best;
     }
 
@@ -1253,6 +1423,7 @@ private:
     // the map at the round's start: places of the logical tile bits, of index 0, and of
     // outside bits
     uint32_t place_of[kMaxT];
+    uint32_t banks[kMaxT];  // and their banks, while a round is written
     uint32_t place_base = 0;
     std::vector<std::pair<int, uint32_t>> place_cst;
     // the round's permutations so far, over the indices at its start: what each logical
@@ -1262,11 +1433,26 @@ private:
     int flip[kMaxT];
     uint32_t base = 0;
     std::vector<std::pair<int, uint32_t>> cst;
+    std::vector<Waiting::Item> later;  // begin_next's
+    struct Split {                     // diagonal()'s factors of the bits and of their sum
+        cd z0, z1, z2;
+    };
+    Recent<Split> splits;
+    struct Part {                      // a table's factor: emit_round's
+        int group;                     // its thread part, -1: none
+        uint32_t word;                 // its pattern over the elements
+        cd z;
+    };
+    std::vector<Part> parts;
+    std::vector<uint64_t> groups;      // thread parts
     std::vector<MapRound> rounds;
     std::vector<MapTable> tabs;
     std::vector<double> data;
 };
 
+// (Its host time is in every call with new angles: ten Trotter steps of 19 qubits, 730 gates,
+// 0.86 ms, 235 gates of 16-qubit brickwork 0.18; with GateOp records in every op, vectors per
+// round and the complex library's operators 2.25 and 0.48, more than the rounds save there.)
 bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     // A controlled rotation is a whole rotation and a table here, and one record there
     // (40 of CRX and CRY on 26, 18 and 8 qubits: 4.55, 0.091 and 0.061 ms against 3.76, 0.073
@@ -1285,13 +1471,14 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     std::vector<MapOp> ops;
     std::vector<MapUnit> units;
     if (!map_lower(gops, ops, units)) return false;
-    std::vector<GateOp> shapes;
+    std::vector<PlanGate> shapes;
+    shapes.reserve(units.size());
     for (const MapUnit &u : units) shapes.push_back(u.shape);
     const std::vector<PlanStep> steps = plan_windows(shapes, n, T);
     // (a two-qubit rotation across windows would be three passes here, 983 us on 26 qubits
     // where its own sweep takes 317)
     for (const PlanStep &st : steps)
-        if (!st.fused && shapes[st.gate].type != OP_SWAP) return false;
+        if (!st.fused && !units[st.gate].swap) return false;
     // the last pass takes what still waits (sweeps after it only move amplitudes)
     size_t last = steps.size();
     for (size_t si = 0; si < steps.size(); ++si)
@@ -1305,11 +1492,12 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
             // a SWAP across windows: its own sweep; what waits changes bits with it
             MapStep ms{};
             ms.fused = false;
-            ms.gate = shapes[st.gate];
+            ms.gate = *units[st.gate].swap;
             out.steps.push_back(ms);
             for (auto &it : wait.items) {
                 const uint64_t x = it.mask >> ms.gate.b0 & 1, y = it.mask >> ms.gate.b1 & 1;
                 if (x != y) it.mask ^= 1ull << ms.gate.b0 | 1ull << ms.gate.b1;
+                wait.see(it.mask);
             }
             continue;
         }
@@ -1319,24 +1507,23 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
         bool closed = false;
         pb.begin(st.pass.h);
         while (!left.empty()) {
-            std::vector<int> next;
+            size_t keep = 0;
             uint64_t blk = 0;
             for (int i : left) {
                 const MapOp &o = ops[i];
-                const uint64_t b = op_bits(o.g);
                 bool done = false;
-                if (!(b & blk)) {
-                    if (o.kind == MO_PERM) done = pb.permute(o.g);
+                if (!(o.bits & blk)) {
+                    if (o.kind == MO_PERM || o.kind == MO_SWAP) done = pb.permute(o);
                     else if (o.kind == MO_DIAG) pb.diagonal(o, pb.round_slots()), done = true;
                     else done = pb.rotate(o);
                 }
                 if (!done) {
-                    next.push_back(i);
-                    blk |= b;
+                    left[keep++] = i;
+                    blk |= o.bits;
                 }
             }
-            const bool stuck = next.size() == left.size();
-            left = std::move(next);
+            const bool stuck = keep == left.size();
+            left.resize(keep);
             // (in its last round, if there is room)
             closed = left.empty() && si == last && pb.bytes() <= kMapProgram / 2;
             pb.close_round(closed);
