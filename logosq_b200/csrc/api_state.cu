@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <map>
 #include <mutex>
+#include <queue>
 #include <type_traits>
 
 #include "lq_internal.h"
@@ -425,6 +426,7 @@ __global__ void __launch_bounds__(256, 2)
 // ---------------------------------------------------------------------------
 constexpr int kWinT = 12, kWinMinT = 9;
 constexpr int kWinStage = 8192;  // bytes of rounds, groups and terms staged at a time
+constexpr size_t kWinSplit = 16; // terms of a round that are not worth sharing out
 
 struct WinTerm {
     uint64_t z;      // Z bits outside the window
@@ -933,14 +935,20 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
     // term: 0.89 and 0.60 ms; of complex64 a sweep is half of that).  So a window for one
     // group of few terms, or two of complex64, is sweeps instead where the state is large
     // enough for that to count more than the launches (20 qubits, two windows of a group
-    // each: 38 us, two sweeps 46), or it is the only group (16 qubits: 30 us, a window 33);
-    // and a sum of terms without X alone is one folded sweep, as far as that goes (n >= 12).
+    // each: 38 us, two sweeps 46), and a sum of terms without X alone is one folded sweep, as
+    // far as that goes (n >= 12).  A sum of a single group is a sweep unless its many terms on
+    // a large state count more than the window's longer start: 8 qubits 25-29 us for 20 terms
+    // and 60 for 1000 (a window 35-38 and 71-96), 20 qubits 40 us for 20 terms (44), but 67 for
+    // 100 (52-60), 24 qubits 153 for 20 (130).
     constexpr int kSweepQubits = 22;
     constexpr size_t kSweepTerms = 4;
     auto few = [&](const std::vector<size_t> &gs) {
-        bool ok = (n >= kSweepQubits || groups.size() == 1) &&
-                  gs.size() <= (s->dtype == LQ_C64 ? 2 : 1);
-        for (size_t gi : gs) ok = ok && groups[gi].second.size() <= kSweepTerms;
+        const bool only = groups.size() == 1;
+        const size_t most = !only ? kSweepTerms
+                            : n < 19 ? (size_t)kMaxGroupTerms
+                                     : std::max<size_t>(kSweepTerms, 64 >> std::min(n - 19, 6));
+        bool ok = (n >= kSweepQubits || only) && gs.size() <= (s->dtype == LQ_C64 ? 2 : 1);
+        for (size_t gi : gs) ok = ok && groups[gi].second.size() <= most;
         return ok;
     };
     auto to_sweeps = [&](std::vector<size_t> &gs) {
@@ -985,7 +993,7 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         auto local = [&](uint64_t mask) {
             return (uint32_t)(mask & 15u) | (uint32_t)((mask >> h) & ((1ull << m) - 1)) << 4;
         };
-        auto parity = [](uint32_t x) { return (uint32_t)__builtin_popcount(x) & 1u; };
+        auto parity = [](uint32_t x) { return (uint32_t)__builtin_parity(x); };
         // rounds: in order of their masks, a group joins if it lies in the span of the
         // vectors or there are fewer than four
         struct Round {
@@ -1030,15 +1038,117 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
             rounds.push_back(std::move(r));
             left.swap(later);
         }
-        // few tiles: the rounds are shared out among more blocks
-        const int share = std::max(1, 2 * 148 / (tiles * (int)wsets.size()));
-        const size_t parts = std::min<size_t>(rounds.size(), (size_t)share);
+        // every round's program: its terms without X first, then the groups
+        struct Entry {
+            bool z;
+            WinGroup wg;
+            std::vector<WinTerm> terms;
+        };
+        struct RoundTerms {
+            WinRound hd;
+            std::vector<Entry> entries;
+            size_t nterms;
+        };
+        std::vector<RoundTerms> prog;
+        size_t all_terms = 0;
+        for (const Round &r : rounds) {
+            RoundTerms rt{};
+            uint32_t pivots = 0;
+            for (int k = 0; k < 4; ++k) {
+                rt.hd.vec[k] = win_place(r.vec[k]);
+                pivots |= 1u << r.piv[k];
+            }
+            // thread bits: first three whose places lie in different banks
+            std::vector<int> lanes;
+            for (int turn = 0; turn < 2; ++turn)
+                for (int p = 0, seen = 0; p < T; ++p) {
+                    if (pivots >> p & 1u) continue;
+                    const bool first = !(seen >> (p % 3) & 1);
+                    seen |= 1 << (p % 3);
+                    if (first == (turn == 0)) lanes.push_back(p);
+                }
+            for (size_t j = 0; j < lanes.size(); ++j) rt.hd.lane[j] = 1u << lanes[j];
+            for (int zturn = 1; zturn >= 0; --zturn)
+                for (size_t gi : r.groups) {
+                    const uint32_t lx = local(groups[gi].first);
+                    if ((lx == 0) != (zturn == 1)) continue;
+                    Entry en{lx == 0, WinGroup{}, {}};
+                    for (int k = 0; k < 4; ++k) en.wg.d |= (int)((lx >> r.piv[k]) & 1u) << k;
+                    // the pairs (or, without X, the vector itself) whose sign bit j turns
+                    uint32_t turns[4];
+                    for (int j = 0; j < 4; ++j) {
+                        turns[j] = lx == 0 ? 1u << j : 0u;
+                        for (int k = 0; lx != 0 && k < 8; ++k)
+                            turns[j] |= (uint32_t)((win_pair(k, en.wg.d) >> j) & 1) << k;
+                    }
+                    en.terms.reserve(groups[gi].second.size());
+                    for (int t : groups[gi].second) {
+                        const TermCoef c = coef_of(t);
+                        const uint32_t odd = terms[t].ny & 1;
+                        WinTerm wt{c.z & ~inside, odd ? c.cb : c.ca, local(c.z), 0, odd, 0};
+                        for (int j = 0; j < 4; ++j)
+                            wt.mask ^= turns[j] & (0u - parity(wt.lz & r.vec[j]));
+                        en.wg.odd |= (int)odd;
+                        en.terms.push_back(wt);
+                    }
+                    if (lx == 0)
+                        std::stable_sort(en.terms.begin(), en.terms.end(),
+                                         [](const WinTerm &x, const WinTerm &y) { return x.mask < y.mask; });
+                    rt.nterms += en.terms.size();
+                    rt.entries.push_back(std::move(en));
+                }
+            all_terms += rt.nterms;
+            prog.push_back(std::move(rt));
+        }
+        // Few tiles: the rounds are shared out among more blocks, and so are the terms of a
+        // round that has more than its share.  (A block takes 0.16 us for each term of a round,
+        // one after the other: 16 masks of 400 terms on 12 qubits 1010 us in two rounds' blocks,
+        // 260 so.)
+        const size_t share = (size_t)std::max(1, 2 * 148 / (tiles * (int)wsets.size()));
+        const size_t most = share == 1 ? all_terms : std::max<size_t>(kWinSplit, (all_terms + share - 1) / share);
+        struct Slice {
+            size_t entry, begin, end;
+        };
+        std::vector<Slice> slices;
+        struct Job {
+            size_t round, nterms, slice, end, part;
+        };
+        std::vector<Job> jobs;
+        for (size_t ri = 0; ri < prog.size(); ++ri) {
+            auto next = [&] { jobs.push_back(Job{ri, 0, slices.size(), slices.size(), 0}); };
+            next();
+            for (size_t ei = 0; ei < prog[ri].entries.size(); ++ei)
+                for (size_t b = 0, n_e = prog[ri].entries[ei].terms.size(); b < n_e;) {
+                    if (jobs.back().nterms == most) next();
+                    const size_t e = std::min(n_e, b + most - jobs.back().nterms);
+                    slices.push_back(Slice{ei, b, e});
+                    jobs.back().end = slices.size();
+                    jobs.back().nterms += e - b;
+                    b = e;
+                }
+        }
+        // the largest first, each to the part with the fewest terms so far
+        const size_t parts = std::min(jobs.size(), share);
+        std::stable_sort(jobs.begin(), jobs.end(),
+                         [](const Job &x, const Job &y) { return x.nterms > y.nterms; });
+        using Load = std::pair<size_t, size_t>;  // terms, part
+        std::priority_queue<Load, std::vector<Load>, std::greater<Load>> loads;
+        for (size_t k = 0; k < parts; ++k) loads.push({0, k});
+        for (Job &j : jobs) {
+            const Load l = loads.top();
+            loads.pop();
+            j.part = l.second;
+            loads.push({l.first + j.nterms + 1, l.second});
+        }
+        std::stable_sort(jobs.begin(), jobs.end(),
+                         [](const Job &x, const Job &y) { return x.part < y.part; });
+        std::vector<WinRound> cr;
+        std::vector<WinGroup> cg;
+        std::vector<WinTerm> ct;
+        size_t ji = 0;
         for (size_t part = 0; part < parts; ++part) {
             WinDesc wd{h, (int)chunks.size(), 0, nwork};
             nwork += tiles;
-            std::vector<WinRound> cr;
-            std::vector<WinGroup> cg;
-            std::vector<WinTerm> ct;
             auto bytes = [&] {
                 return cr.size() * sizeof(WinRound) + cg.size() * sizeof(WinGroup) +
                        ct.size() * sizeof(WinTerm);
@@ -1056,26 +1166,11 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
                 chunks.push_back(c);
                 cr.clear(), cg.clear(), ct.clear();
             };
-            for (size_t ri = part; ri < rounds.size(); ri += parts) {
-                const Round &r = rounds[ri];
-                WinRound hd{};
-                uint32_t pivots = 0;
-                for (int k = 0; k < 4; ++k) {
-                    hd.vec[k] = win_place(r.vec[k]);
-                    pivots |= 1u << r.piv[k];
-                }
-                // thread bits: first three whose places lie in different banks
-                std::vector<int> lanes;
-                for (int turn = 0; turn < 2; ++turn)
-                    for (int p = 0, seen = 0; p < T; ++p) {
-                        if (pivots >> p & 1u) continue;
-                        const bool first = !(seen >> (p % 3) & 1);
-                        seen |= 1 << (p % 3);
-                        if (first == (turn == 0)) lanes.push_back(p);
-                    }
-                for (size_t j = 0; j < lanes.size(); ++j) hd.lane[j] = 1u << lanes[j];
+            for (; ji < jobs.size() && jobs[ji].part == part; ++ji) {
+                const Job *job = &jobs[ji];
                 auto open = [&](size_t more) {
                     if (!cr.empty() && bytes() + more > (size_t)kWinStage) close();
+                    WinRound hd = prog[job->round].hd;
                     hd.group = (int)cg.size(), hd.ngroups = 0;
                     hd.zterm = (int)ct.size(), hd.nz = 0;
                     cr.push_back(hd);
@@ -1083,47 +1178,28 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
                 // (a piece of a group must fit a stage of its own)
                 constexpr size_t piece = (kWinStage - sizeof(WinRound) - sizeof(WinGroup)) / sizeof(WinTerm);
                 bool opened = false;
-                for (int zturn = 1; zturn >= 0; --zturn)  // a round's terms without X come first
-                    for (size_t gi : r.groups) {
-                        const uint32_t lx = local(groups[gi].first);
-                        if ((lx == 0) != (zturn == 1)) continue;
-                        WinGroup wg{};
-                        for (int k = 0; k < 4; ++k) wg.d |= (int)((lx >> r.piv[k]) & 1u) << k;
-                        std::vector<WinTerm> all;
-                        for (int t : groups[gi].second) {
-                            const TermCoef c = coef_of(t);
-                            const uint32_t odd = terms[t].ny & 1;
-                            WinTerm wt{c.z & ~inside, odd ? c.cb : c.ca, local(c.z), 0, odd, 0};
-                            uint32_t on = 0;
-                            for (int k = 0; k < 4; ++k) on |= parity(wt.lz & r.vec[k]) << k;
-                            if (lx == 0) wt.mask = on;
-                            else
-                                for (int k = 0; k < 8; ++k)
-                                    wt.mask |= parity(on & (uint32_t)win_pair(k, wg.d)) << k;
-                            wg.odd |= (int)odd;
-                            all.push_back(wt);
+                for (size_t si = job->slice; si < job->end; ++si) {
+                    const Slice &sl = slices[si];
+                    const Entry &en = prog[job->round].entries[sl.entry];
+                    for (size_t b = sl.begin; b < sl.end; b += piece) {
+                        const size_t e = std::min(sl.end, b + piece);
+                        const size_t need = (e - b) * sizeof(WinTerm) + sizeof(WinGroup);
+                        if (!opened || bytes() + need > (size_t)kWinStage)
+                            open(need + sizeof(WinRound)), opened = true;
+                        WinRound &rd = cr.back();
+                        if (en.z) {
+                            rd.zterm = (int)ct.size();
+                            rd.nz = (int)(e - b);
+                        } else {
+                            WinGroup wg = en.wg;
+                            wg.term = (int)ct.size();
+                            wg.nterms = (int)(e - b);
+                            cg.push_back(wg);
+                            ++rd.ngroups;
                         }
-                        if (lx == 0)
-                            std::stable_sort(all.begin(), all.end(),
-                                             [](const WinTerm &x, const WinTerm &y) { return x.mask < y.mask; });
-                        for (size_t b = 0; b < all.size(); b += piece) {
-                            const size_t e = std::min(all.size(), b + piece);
-                            const size_t need = (e - b) * sizeof(WinTerm) + sizeof(WinGroup);
-                            if (!opened || bytes() + need > (size_t)kWinStage)
-                                open(need + sizeof(WinRound)), opened = true;
-                            WinRound &rd = cr.back();
-                            if (lx == 0) {
-                                rd.zterm = (int)ct.size();
-                                rd.nz = (int)(e - b);
-                            } else {
-                                wg.term = (int)ct.size();
-                                wg.nterms = (int)(e - b);
-                                cg.push_back(wg);
-                                ++rd.ngroups;
-                            }
-                            ct.insert(ct.end(), all.begin() + b, all.begin() + e);
-                        }
+                        ct.insert(ct.end(), en.terms.begin() + b, en.terms.begin() + e);
                     }
+                }
             }
             close();
             wd.nchunks = (int)chunks.size() - wd.chunk;
@@ -1139,12 +1215,12 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         for (int t : groups[gi].second) packed.push_back(coef_of(t));
     }
     lq_state *ms = const_cast<lq_state *>(s);
-    auto al = [](size_t x) { return (x + 255) / 256 * 256; };
+    auto al = [](size_t x) { return (x + 15) / 16 * 16; };
     const size_t o_win = al(packed.size() * sizeof(TermCoef));
     const size_t o_chk = o_win + al(wins.size() * sizeof(WinDesc));
     const size_t o_pgm = o_chk + al(chunks.size() * sizeof(WinChunk));
     const size_t o_beg = o_pgm + al(program.size());
-    const size_t o_res = o_beg + al(sizeof(pbeg));
+    const size_t o_res = o_beg + (zfold >= 0 ? al(sizeof(pbeg)) : 0);
     const size_t nres = sweeps.size() + (wins.empty() ? 0 : 1);
     LQ_TRY(ensure_prog(ms, o_res + al(nres * sizeof(double)) + 256));
     char *dp = (char *)ms->d_prog;
@@ -1159,7 +1235,7 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
         put(o_win, wins);
         put(o_chk, chunks);
         put(o_pgm, program);
-        memcpy(up.data() + o_beg, pbeg, sizeof(pbeg));
+        if (zfold >= 0) memcpy(up.data() + o_beg, pbeg, sizeof(pbeg));
         LQ_CUDA_TRY(cudaMemcpyAsync(dp, up.data(), o_res, cudaMemcpyHostToDevice, s->stream));
     }
     prof_begin(s->stream, kProfReduce);
