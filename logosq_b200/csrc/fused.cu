@@ -200,8 +200,8 @@ __device__ __forceinline__ void fused_pp_body(const CUtensorMap &tmap, int T, Ti
     }
 }
 
-// 168 registers: six 64-thread CTAs per SM at tile bits 10.  Measured on a
-// 30-qubit brickwork: 481 ms per step at 168 registers (a few spills outside
+// Below tile bits 12, 168 registers: six 64-thread CTAs per SM at tile bits 10.  Measured on
+// a 30-qubit brickwork: 481 ms per step at 168 registers (a few spills outside
 // the hot ops), 540 at 192, 518 at 240 -- resident warps matter more than the
 // last registers.
 #ifndef LQ_PP_MAXNREG
@@ -213,6 +213,17 @@ __global__ void __maxnreg__(LQ_PP_MAXNREG)
                       const FusedRound *__restrict__ rounds, int nrounds,
                       const PassOp *__restrict__ ops, const double *__restrict__ coef,
                       const uint16_t *__restrict__ tbtab, unsigned *__restrict__ flag) {
+    fused_pp_body<MODE>(tmap, T, tc, rounds, nrounds, ops, coef, tbtab, flag);
+}
+
+// Tile bits 12: 256 threads, of which one CTA fits an SM at 168 registers as at 198, so they
+// take what they need (80 gates with Toffolis on 26 qubits: 6.37 ms, 6.84 at 168).
+template <int MODE>
+__global__ void __launch_bounds__(256, 1)
+    k_fused_pp(const __grid_constant__ CUtensorMap tmap, int T, TileCoords tc,
+               const FusedRound *__restrict__ rounds, int nrounds, const PassOp *__restrict__ ops,
+               const double *__restrict__ coef, const uint16_t *__restrict__ tbtab,
+               unsigned *__restrict__ flag) {
     fused_pp_body<MODE>(tmap, T, tc, rounds, nrounds, ops, coef, tbtab, flag);
 }
 
@@ -1010,6 +1021,7 @@ static int set_pp_attrs() {
     const int mx = (int)fused_smem(kMaxT);
 #define LQ_ATTR(K) LQ_CUDA_TRY(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, mx))
     LQ_ATTR(k_fused_pp_narrow<1>);
+    LQ_ATTR(k_fused_pp<1>);
 #undef LQ_ATTR
     done = true;
     return LQ_OK;
@@ -1032,7 +1044,8 @@ static int launch_pass_pp(lq_state *s, int T, int h, const FusedRound *d_rounds,
     K<<<ntiles, blk, smem, s->stream>>>(map, T, tc, d_rounds, nrounds, d_ops, d_coef, d_tb, \
                                         s->d_flag)
     (void)mode;  // one op set (4x4, pair and table ops included); blocks use launch_pass
-    LQ_FUSED_LAUNCH(k_fused_pp_narrow<1>);
+    if (T >= 12) LQ_FUSED_LAUNCH(k_fused_pp<1>);
+    else LQ_FUSED_LAUNCH(k_fused_pp_narrow<1>);
 #undef LQ_FUSED_LAUNCH
     prof_end(s->stream, kProfFused);
     LQ_CUDA_TRY(cudaGetLastError());
