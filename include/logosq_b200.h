@@ -408,7 +408,10 @@ int lq_noise_pauli(lq_state *s, int qubit, int pauli);
 /* AmplitudeDampingNoise::apply (src/noise/mod.rs:108-146): the sum over target
  * qubits of (K0 + K1) psi, K0 = |0><0| + sqrt(1-g)|1><1|, K1 = sqrt(g)|0><1|,
  * then normalised.  More than one target needs a scratch vector of 2^n
- * amplitudes (LQ_ERR_OOM if it cannot be allocated). */
+ * amplitudes (LQ_ERR_OOM if it cannot be allocated).  Scratch of up to 128 MiB,
+ * here and in lq_measure_shots, stays for later calls: 1 MiB with each handle, the
+ * rest, at most 256 MiB, for all handles until the last of them is destroyed or an
+ * allocation fails. */
 int lq_noise_amplitude_damping(lq_state *s, double gamma, const int *qubits, int nqubits);
 /* PhaseDampingNoise::apply (src/noise/mod.rs:173-210): |1> amplitudes of the
  * LAST target qubit scaled by sqrt(1-lambda) (each target rewrites the

@@ -1447,13 +1447,13 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
     const size_t states = (size_t)p.amps * copies * sizeof(double2);
     if (states > alloc_room())
         return set_error(LQ_ERR_OOM, "%zu bytes of states exceed the allocation limit", states);
-    if (states > 0) e = cudaMalloc(&p.states, states);
+    if (states > 0) e = device_malloc(&p.states, states);
     if (e == cudaSuccess) {
         if (work) {
             LQ_TRY(ensure_prog(work, off));
             p.blob = work->d_prog;
         } else {
-            e = cudaMalloc(&p.blob, off);
+            e = device_malloc(&p.blob, off);
             p.own_blob = e == cudaSuccess;
         }
     }

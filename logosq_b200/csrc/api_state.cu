@@ -20,6 +20,7 @@ static thread_local std::string g_last_error;
 static uint64_t g_alloc_limit = 0;
 static std::mutex g_alloc_mu;
 static uint64_t g_alloc_in_use = 0;
+static int64_t g_handles = 0;  // live states
 
 int set_error(int code, const char *fmt, ...) {
     char buf[1024];
@@ -66,47 +67,143 @@ int ensure_prog(lq_state *s, size_t bytes) {
         s->prog_cap = 0;
     }
     size_t cap = std::max<size_t>(bytes, 1 << 16);
-    LQ_CUDA_TRY(cudaMalloc(&s->d_prog, cap));
+    LQ_CUDA_TRY(device_malloc(&s->d_prog, cap));
     s->prog_cap = cap;
     return LQ_OK;
 }
 
-int take_work(lq_state *s, size_t bytes, void **out) {
-    *out = nullptr;
-    if (bytes > kKeptWork) {
-        // (the stream-ordered pool maps the memory piece by piece and afresh each time: damping
-        // two targets of 26 qubits took 14 ms through it, 2.6-3.0 so; a capture has no choice)
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        LQ_CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
-        if (cs == cudaStreamCaptureStatusNone) LQ_CUDA_TRY(cudaMalloc(out, bytes));
-        else LQ_CUDA_TRY(cudaMallocAsync(out, bytes, s->stream));
+// ---------------------------------------------------------------------------
+// Workspaces above kOwnWork, shared by all handles: a call takes one that its own stream used
+// last or whose last use is over, else a new one, else (at most kPoolBytes are there, of at
+// most kKeptWork each) the one unused for longest, and its stream waits for the last use.
+// They stay until the last handle is destroyed or an allocation fails.  (Kept with each
+// handle they were a second copy of every 20- to 22-qubit state that had once been damped or
+// sampled; allocated afresh they cost a call 0.4 to 20 ms.)
+// ---------------------------------------------------------------------------
+constexpr size_t kPoolBytes = 256ull << 20;
+
+struct Workspace {
+    int device;
+    void *p;
+    size_t bytes;
+    cudaEvent_t used;  // recorded after the last use, on
+    cudaStream_t stream;
+};
+
+static std::mutex g_pool_mu;
+static size_t g_pool_bytes = 0;  // of the workspaces of at most kKeptWork, those in use too
+// The free ones, in order of their last use (never destroyed: the driver may be gone by then).
+static std::vector<Workspace> &pool() {
+    static auto *v = new std::vector<Workspace>();
+    return *v;
+}
+
+static void drop_workspace(const Workspace &w) {
+    cudaFree(w.p);  // (waits for its users)
+    cudaEventDestroy(w.used);
+}
+
+static void free_pool() {
+    std::vector<Workspace> all;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        all.swap(pool());
+        for (const Workspace &w : all) g_pool_bytes -= w.bytes;
+    }
+    for (const Workspace &w : all) drop_workspace(w);
+}
+
+static void free_spares(size_t keep);
+
+cudaError_t device_malloc_bytes(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    free_spares(0);
+    free_pool();
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+int Work::take(size_t bytes) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    LQ_CUDA_TRY(cudaStreamIsCapturing(s_->stream, &cs));
+    if (cs != cudaStreamCaptureStatusNone) {  // a graph that outlives the call: its own memory
+        LQ_CUDA_TRY(cudaMallocAsync(&p_, bytes, s_->stream));
+        kind_ = kCaptured;
         return LQ_OK;
     }
-    if (s->work_cap < bytes) {
-        if (s->d_work) {
-            LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
-            LQ_CUDA_TRY(cudaFree(s->d_work));
-            s->d_work = nullptr;
-            s->work_cap = 0;
+    if (bytes <= kOwnWork) {
+        if (s_->work_cap < bytes) {
+            if (s_->d_work) {
+                LQ_CUDA_TRY(cudaStreamSynchronize(s_->stream));
+                LQ_CUDA_TRY(cudaFree(s_->d_work));
+                s_->d_work = nullptr;
+                s_->work_cap = 0;
+            }
+            LQ_CUDA_TRY(device_malloc(&s_->d_work, bytes));
+            s_->work_cap = bytes;
         }
-        LQ_CUDA_TRY(cudaMalloc(&s->d_work, bytes));
-        s->work_cap = bytes;
+        p_ = s_->d_work;
+        return LQ_OK;
     }
-    *out = s->d_work;
+    kind_ = kPooled;
+    bool wait = false;
+    if (bytes <= kKeptWork) {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        auto &v = pool();
+        auto fits = [&](const Workspace &w) { return w.device == s_->device && w.bytes >= bytes; };
+        auto own = [&](const Workspace &w) { return fits(w) && w.stream == s_->stream; };
+        auto idle = [&](const Workspace &w) {
+            if (!fits(w)) return false;
+            const bool over = cudaEventQuery(w.used) == cudaSuccess;
+            if (!over) cudaGetLastError();
+            return over;
+        };
+        auto at = std::find_if(v.begin(), v.end(), own);
+        if (at == v.end()) at = std::find_if(v.begin(), v.end(), idle);
+        if (at == v.end() && g_pool_bytes + bytes > kPoolBytes) {
+            at = std::find_if(v.begin(), v.end(), fits);
+            wait = true;
+        }
+        if (at != v.end()) {
+            p_ = at->p;
+            bytes_ = at->bytes;
+            used_ = at->used;
+            v.erase(at);
+        } else {
+            g_pool_bytes += bytes;
+        }
+    }
+    if (p_) {
+        if (wait) LQ_CUDA_TRY(cudaStreamWaitEvent(s_->stream, used_, 0));
+        return LQ_OK;
+    }
+    bytes_ = bytes;
+    LQ_CUDA_TRY(cudaEventCreateWithFlags(&used_, cudaEventDisableTiming));
+    LQ_CUDA_TRY(device_malloc(&p_, bytes));
     return LQ_OK;
 }
 
-int give_work(lq_state *s, void *p) {
-    if (!p || p == s->d_work) return LQ_OK;
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    LQ_CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
-    if (cs == cudaStreamCaptureStatusNone) {
-        LQ_CUDA_TRY(cudaStreamSynchronize(s->stream));
-        LQ_CUDA_TRY(cudaFree(p));
-    } else {
-        LQ_CUDA_TRY(cudaFreeAsync(p, s->stream));
+Work::~Work() {
+    if (kind_ == kCaptured) cudaFreeAsync(p_, s_->stream);
+    if (kind_ != kPooled) return;
+    const bool counted = bytes_ > 0 && bytes_ <= kKeptWork;
+    if (p_ && counted && cudaEventRecord(used_, s_->stream) == cudaSuccess) {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        if (g_pool_bytes <= kPoolBytes) {
+            pool().push_back(Workspace{s_->device, p_, bytes_, used_, s_->stream});
+            return;
+        }
     }
-    return LQ_OK;
+    if (p_) cudaStreamSynchronize(s_->stream);
+    if (p_) cudaFree(p_);
+    if (used_) cudaEventDestroy(used_);
+    if (counted) {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        g_pool_bytes -= bytes_;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1348,8 +1445,8 @@ namespace lq {
 // them are used on the handle's own stream, which its destruction waits for; a wait for the
 // whole device would break a graph capture on any other stream.  Only the amplitudes may be
 // known elsewhere (lq_state::lent): they are then given back by cudaFree, which waits for
-// their readers.  At most four sets of at most 4 MiB are kept; a failed allocation of
-// amplitudes frees them.
+// their readers.  At most four sets of at most 4 MiB are kept; a failed allocation
+// (device_malloc) frees them.
 // ---------------------------------------------------------------------------
 constexpr size_t kSpares = 4, kSpareBytes = 1 << 20;
 
@@ -1624,17 +1721,10 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
     if (!take_spare(s)) {
         e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
         if (e == cudaSuccess)
-            e = cudaMalloc(&s->d_red, sizeof(double) * kRedBlocks * 2 * kMaxTermsPerPass);
-        if (e == cudaSuccess) e = cudaMalloc(&s->d_flag, sizeof(unsigned) * 4);
+            e = device_malloc(&s->d_red, sizeof(double) * kRedBlocks * 2 * kMaxTermsPerPass);
+        if (e == cudaSuccess) e = device_malloc(&s->d_flag, sizeof(unsigned) * 4);
     }
-    if (e == cudaSuccess && !s->d) {
-        e = cudaMalloc(&s->d, bytes);
-        if (e == cudaErrorMemoryAllocation) {  // (the spares go first)
-            cudaGetLastError();
-            free_spares(0);
-            e = cudaMalloc(&s->d, bytes);
-        }
-    }
+    if (e == cudaSuccess && !s->d) e = device_malloc(&s->d, bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_flag, 0, sizeof(unsigned) * 4, s->stream);
     if (e != cudaSuccess) {
         const int code = e == cudaErrorMemoryAllocation ? LQ_ERR_OOM : LQ_ERR_CUDA;
@@ -1646,6 +1736,7 @@ int lq_state_create(int num_qubits, int dtype, lq_state **out) {
     {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         g_alloc_in_use += bytes;
+        ++g_handles;
     }
     *out = s;
     int rc = lq_state_set_basis(s, 0);
@@ -1661,13 +1752,16 @@ int lq_state_destroy(lq_state *s) {
     if (!s) return LQ_OK;
     // (a stream that cannot be waited for is not handed on)
     const bool idle = s->stream && cudaStreamSynchronize(s->stream) == cudaSuccess;
-    if (s->d) {
+    bool last;
+    {
         std::lock_guard<std::mutex> lk(g_alloc_mu);
         g_alloc_in_use -= s->bytes;
+        last = --g_handles == 0;
     }
     free_plan_cache(s);
     if (!idle || !give_spare(s)) free_resources(s);
     delete s;
+    if (last) free_pool();
     return LQ_OK;
 }
 
@@ -1986,16 +2080,16 @@ static int measure_shots_t(lq_state *s, const A *v, uint64_t n_shots, uint64_t s
     const uint64_t N = 1ull << s->n, nc = (N + kScanChunk - 1) / kScanChunk;
     if (nc > 0x7fffffffull) return set_error(LQ_ERR_UNSUPPORTED, "scan too long");
     cudaStream_t st = s->stream;
-    // The chunk scans are kept where they fit the handle's workspace, or where so many
+    // The chunk scans are kept where they fit a workspace that stays, or where so many
     // shots come that one chunk each would cost more.  Above that a call would allocate
     // half the state's size for some probes (mapping 64 MB fresh and returning it takes
     // 0.4 to 20 ms); a chunk scanned again costs a shot about 4 ns of the whole GPU.
     const bool keep = N * 8 <= kKeptWork / 2 || n_shots > N / 64;
     const uint64_t scratch = scan_scratch(N);
     const uint64_t need = ((keep ? N : 0) + scratch + n_shots) * 8;
-    void *work = nullptr;
-    LQ_TRY(take_work(s, need, &work));
-    double *tot = (double *)work, *local = keep ? tot + scratch + n_shots : nullptr;
+    Work work(s);
+    LQ_TRY(work.take(need));
+    double *tot = (double *)work.get(), *local = keep ? tot + scratch + n_shots : nullptr;
     uint64_t *d_out = (uint64_t *)(tot + scratch);
     double *incl = tot + nc;
     k_scan_chunks<<<(unsigned)nc, 256, 0, st>>>(v, local, tot, N);
@@ -2008,7 +2102,6 @@ static int measure_shots_t(lq_state *s, const A *v, uint64_t n_shots, uint64_t s
             v, tot, incl, N, n_shots, seed, d_out);
     LQ_CUDA_TRY(cudaGetLastError());
     LQ_CUDA_TRY(cudaMemcpyAsync(host_out, d_out, n_shots * 8, cudaMemcpyDeviceToHost, st));
-    LQ_TRY(give_work(s, work));
     LQ_CUDA_TRY(cudaStreamSynchronize(st));
     return LQ_OK;
 }

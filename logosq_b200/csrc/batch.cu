@@ -936,7 +936,7 @@ static int ensure_shift_engine(lq_batch *b) {
     if (b->shift_ready) return LQ_OK;
     auto put = [&](auto *&dst, const auto &v) -> cudaError_t {
         const size_t bytes = sizeof(v[0]) * std::max<size_t>(v.size(), 1);
-        cudaError_t e = cudaMalloc(&dst, bytes);
+        cudaError_t e = device_malloc(&dst, bytes);
         if (e == cudaSuccess && !v.empty())
             e = cudaMemcpy(dst, v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice);
         return e;
@@ -954,13 +954,13 @@ static int ensure_shift_engine(lq_batch *b) {
         if ((e = put(b->ewins, b->h_ewins)) || (e = put(b->groups, b->h_groups)) ||
             (e = put(b->bterms, b->h_bterms)))
             return e;
-        if ((e = cudaMalloc(&b->ckpt, sizeof(double2) * std::max<size_t>(b->ckpt_amps, 1))) ||
-            (e = cudaMalloc(&b->coef_d, sizeof(double) * b->coef_cap)) ||
+        if ((e = device_malloc(&b->ckpt, sizeof(double2) * std::max<size_t>(b->ckpt_amps, 1))) ||
+            (e = device_malloc(&b->coef_d, sizeof(double) * b->coef_cap)) ||
             (e = cudaMallocHost(&b->coef_h, sizeof(double) * b->coef_cap)) ||
-            (e = cudaMalloc(&b->energy_d, sizeof(double) * b->nitems)) ||
+            (e = device_malloc(&b->energy_d, sizeof(double) * b->nitems)) ||
             (e = cudaMallocHost(&b->energy_h, sizeof(double) * b->nitems)) ||
-            (e = cudaMalloc(&b->counter, 2 * sizeof(unsigned))) ||
-            (e = cudaMalloc(&b->scratch, sizeof(double2) * b->slot_amps * b->grid)))
+            (e = device_malloc(&b->counter, 2 * sizeof(unsigned))) ||
+            (e = device_malloc(&b->scratch, sizeof(double2) * b->slot_amps * b->grid)))
             return e;
         return cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)batch_smem());

@@ -332,14 +332,14 @@ static int mlp_reserve(lq_mlp *net, int batch) {
     net->Z.assign(net->dims.size(), nullptr);
     int widest = 0;
     for (size_t l = 0; l < net->dims.size(); ++l) {
-        LQ_CUDA_TRY(cudaMalloc(&net->H[l], sizeof(float) * batch * net->dims[l]));
-        LQ_CUDA_TRY(cudaMalloc(&net->Z[l], sizeof(float) * batch * net->dims[l]));
+        LQ_CUDA_TRY(device_malloc(&net->H[l], sizeof(float) * batch * net->dims[l]));
+        LQ_CUDA_TRY(device_malloc(&net->Z[l], sizeof(float) * batch * net->dims[l]));
         widest = std::max(widest, net->dims[l]);
     }
-    LQ_CUDA_TRY(cudaMalloc(&net->target, sizeof(float) * batch * net->out_dim));
-    LQ_CUDA_TRY(cudaMalloc(&net->mask, sizeof(float) * batch * net->out_dim));
-    LQ_CUDA_TRY(cudaMalloc(&net->dA, sizeof(float) * batch * widest));
-    LQ_CUDA_TRY(cudaMalloc(&net->dB, sizeof(float) * batch * widest));
+    LQ_CUDA_TRY(device_malloc(&net->target, sizeof(float) * batch * net->out_dim));
+    LQ_CUDA_TRY(device_malloc(&net->mask, sizeof(float) * batch * net->out_dim));
+    LQ_CUDA_TRY(device_malloc(&net->dA, sizeof(float) * batch * widest));
+    LQ_CUDA_TRY(device_malloc(&net->dB, sizeof(float) * batch * widest));
     net->cap = batch;
     return LQ_OK;
 }
@@ -432,11 +432,11 @@ int lq_mlp_create(int in_dim, int hidden, int depth, int out_dim, uint64_t seed,
     };
     cudaError_t e;
     if ((e = cudaStreamCreateWithFlags(&net->stream, cudaStreamNonBlocking))) return fail(e);
-    if ((e = cudaMalloc(&net->p, off * 4))) return fail(e);
-    if ((e = cudaMalloc(&net->g, off * 4))) return fail(e);
-    if ((e = cudaMalloc(&net->m, off * 4))) return fail(e);
-    if ((e = cudaMalloc(&net->v, off * 4))) return fail(e);
-    if ((e = cudaMalloc(&net->loss_d, sizeof(double) * kLossBlocks))) return fail(e);
+    if ((e = device_malloc(&net->p, off * 4))) return fail(e);
+    if ((e = device_malloc(&net->g, off * 4))) return fail(e);
+    if ((e = device_malloc(&net->m, off * 4))) return fail(e);
+    if ((e = device_malloc(&net->v, off * 4))) return fail(e);
+    if ((e = device_malloc(&net->loss_d, sizeof(double) * kLossBlocks))) return fail(e);
     if ((e = cudaMemcpy(net->p, init.data(), off * 4, cudaMemcpyHostToDevice))) return fail(e);
     if ((e = cudaMemset(net->m, 0, off * 4)) || (e = cudaMemset(net->v, 0, off * 4)) ||
         (e = cudaMemset(net->g, 0, off * 4)))
@@ -615,11 +615,11 @@ int lq_lanczos_ground_energy(int num_qubits, const lq_pauli_term *terms, int nte
         cudaStreamDestroy(st);
     };
     cudaError_t e;
-    if ((e = cudaMalloc(&V, sizeof(double) * N * (kmax + 1))) ||
-        (e = cudaMalloc(&w, sizeof(double) * N)) ||
-        (e = cudaMalloc(&part, sizeof(double) * kDotBlocks * (kmax + 1))) ||
-        (e = cudaMalloc(&coef, sizeof(double) * (kmax + 1))) ||
-        (e = cudaMalloc(&dterms, sizeof(RealTerm) * rt.size()))) {
+    if ((e = device_malloc(&V, sizeof(double) * N * (kmax + 1))) ||
+        (e = device_malloc(&w, sizeof(double) * N)) ||
+        (e = device_malloc(&part, sizeof(double) * kDotBlocks * (kmax + 1))) ||
+        (e = device_malloc(&coef, sizeof(double) * (kmax + 1))) ||
+        (e = device_malloc(&dterms, sizeof(RealTerm) * rt.size()))) {
         cleanup();
         return set_error(e == cudaErrorMemoryAllocation ? LQ_ERR_OOM : LQ_ERR_CUDA, "%s",
                          cudaGetErrorString(e));

@@ -90,7 +90,7 @@ struct lq_state {
     // Per-handle device buffer for gate programs of fused passes.
     void *d_prog = nullptr;
     size_t prog_cap = 0;
-    // Workspace of calls that need a few temporary arrays (take_work).
+    // Workspace of at most kOwnWork bytes for calls that need temporary arrays (Work).
     void *d_work = nullptr;
     size_t work_cap = 0;
     // Statistics of the last circuit call.
@@ -128,12 +128,34 @@ int gate_matrix(const lq_gate *g, const double *theta, double *m /* 2*64 doubles
 enum GateClass { kClassGeneral = 0, kClassDiagonal = 1, kClassPermutation = 2 };
 int gate_class(int kind);
 
-// Temporary device memory for one call on s's stream.  Up to kKeptWork bytes stay with
-// the handle for its next call (one call at a time: the stream orders their use);
-// more is allocated and returned each time, so a large state never holds a second.
-constexpr size_t kKeptWork = 128ull << 20;
-int take_work(lq_state *s, size_t bytes, void **out);
-int give_work(lq_state *s, void *p);
+// cudaMalloc; if it fails for lack of memory, again after what is kept for later calls
+// (workspaces, spare resources of small handles) has been given back.
+cudaError_t device_malloc_bytes(void **p, size_t bytes);
+template <class T>
+cudaError_t device_malloc(T **p, size_t bytes) {
+    return device_malloc_bytes((void **)p, bytes);
+}
+
+// Temporary device memory for one call on s's stream, given back at the end of its scope.  Up
+// to kOwnWork bytes stay with the handle (one call at a time: the stream orders their use), up
+// to kKeptWork with a pool for all handles; more is allocated and returned each time.
+constexpr size_t kOwnWork = 1ull << 20, kKeptWork = 128ull << 20;
+class Work {
+public:
+    explicit Work(lq_state *s) : s_(s) {}
+    ~Work();
+    Work(const Work &) = delete;
+    int take(size_t bytes);  // once
+    void *get() const { return p_; }
+
+private:
+    enum Kind { kOwn, kPooled, kCaptured };
+    lq_state *s_;
+    void *p_ = nullptr;
+    size_t bytes_ = 0;
+    cudaEvent_t used_ = nullptr;
+    Kind kind_ = kOwn;
+};
 
 // api_state.cu
 int normalize_impl(lq_state *s);

@@ -175,16 +175,16 @@ int lq_noise_amplitude_damping(lq_state *s, double gamma, const int *qubits, int
         LQ_CUDA_TRY(cudaGetLastError());
         return scale_by_partials(s, nullptr, grid);
     }
-    void *out = nullptr;
-    LQ_TRY(take_work(s, N * sizeof(double2), &out));
+    Work work(s);
+    LQ_TRY(work.take(N * sizeof(double2)));
+    void *out = work.get();
     const int grid = red_grid(N, 256);
     prof_begin(s->stream, kProfGate);
     k_damp_norm<<<grid, 256, 0, s->stream>>>((const double2 *)s->d, (double2 *)out, N, d,
                                             s->d_red);
     prof_end(s->stream, kProfGate);
     LQ_CUDA_TRY(cudaGetLastError());
-    LQ_TRY(scale_by_partials(s, out, grid));
-    return give_work(s, out);
+    return scale_by_partials(s, out, grid);
 }
 
 int lq_noise_phase_damping(lq_state *s, double lambda, const int *qubits, int nqubits) {
