@@ -1441,7 +1441,10 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
     const size_t o_epart = take((size_t)p.nepart * sizeof(double));
     const size_t o_theta = take(((size_t)p.nparams + 1) * sizeof(double));
     const size_t o_out = take(((size_t)p.ninst + p.nparams) * sizeof(double));
-    // A plain call works in its handle's own program buffer and amplitudes.
+    // A plain call works in its handle's own program buffer and amplitudes.  (The partial sums
+    // of a large state, 24 bytes per tile and run of gates, would stay there for the handle's
+    // life, 0.3 GB after a gradient of 28 qubits and 84 runs: they are given back.)
+    constexpr size_t kHandleProgram = 32ull << 20;
     cudaError_t e = cudaSuccess;
     const size_t copies = work ? 1 : 2;
     const size_t states = (size_t)p.amps * copies * sizeof(double2);
@@ -1449,7 +1452,7 @@ int adj_upload(AdjProgram &p, lq_state *work, cudaStream_t st) {
         return set_error(LQ_ERR_OOM, "%zu bytes of states exceed the allocation limit", states);
     if (states > 0) e = device_malloc(&p.states, states);
     if (e == cudaSuccess) {
-        if (work) {
+        if (work && off <= kHandleProgram) {
             LQ_TRY(ensure_prog(work, off));
             p.blob = work->d_prog;
         } else {
