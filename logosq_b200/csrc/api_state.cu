@@ -88,6 +88,7 @@ struct Workspace {
     size_t bytes;
     cudaEvent_t used;  // recorded after the last use, on
     cudaStream_t stream;
+    bool idle;         // its last use is known to be over
 };
 
 static std::mutex g_pool_mu;
@@ -156,7 +157,7 @@ int Work::take(size_t bytes) {
         auto fits = [&](const Workspace &w) { return w.device == s_->device && w.bytes >= bytes; };
         auto own = [&](const Workspace &w) { return fits(w) && w.stream == s_->stream; };
         auto idle = [&](const Workspace &w) {
-            if (!fits(w)) return false;
+            if (!fits(w) || w.idle) return fits(w);
             const bool over = cudaEventQuery(w.used) == cudaSuccess;
             if (!over) cudaGetLastError();
             return over;
@@ -165,7 +166,7 @@ int Work::take(size_t bytes) {
         if (at == v.end()) at = std::find_if(v.begin(), v.end(), idle);
         if (at == v.end() && g_pool_bytes + bytes > kPoolBytes) {
             at = std::find_if(v.begin(), v.end(), fits);
-            wait = true;
+            wait = true;  // (none that fits is idle)
         }
         if (at != v.end()) {
             p_ = at->p;
@@ -190,10 +191,10 @@ Work::~Work() {
     if (kind_ == kCaptured) cudaFreeAsync(p_, s_->stream);
     if (kind_ != kPooled) return;
     const bool counted = bytes_ > 0 && bytes_ <= kKeptWork;
-    if (p_ && counted && cudaEventRecord(used_, s_->stream) == cudaSuccess) {
+    if (p_ && counted && (idle_ || cudaEventRecord(used_, s_->stream) == cudaSuccess)) {
         std::lock_guard<std::mutex> lk(g_pool_mu);
         if (g_pool_bytes <= kPoolBytes) {
-            pool().push_back(Workspace{s_->device, p_, bytes_, used_, s_->stream});
+            pool().push_back(Workspace{s_->device, p_, bytes_, used_, s_->stream, idle_});
             return;
         }
     }
@@ -2103,6 +2104,7 @@ static int measure_shots_t(lq_state *s, const A *v, uint64_t n_shots, uint64_t s
     LQ_CUDA_TRY(cudaGetLastError());
     LQ_CUDA_TRY(cudaMemcpyAsync(host_out, d_out, n_shots * 8, cudaMemcpyDeviceToHost, st));
     LQ_CUDA_TRY(cudaStreamSynchronize(st));
+    work.waited();
     return LQ_OK;
 }
 

@@ -147,6 +147,7 @@ public:
     Work(const Work &) = delete;
     int take(size_t bytes);  // once
     void *get() const { return p_; }
+    void waited() { idle_ = true; }  // the caller has waited for its last use
 
 private:
     enum Kind { kOwn, kPooled, kCaptured };
@@ -155,6 +156,7 @@ private:
     size_t bytes_ = 0;
     cudaEvent_t used_ = nullptr;
     Kind kind_ = kOwn;
+    bool idle_ = false;
 };
 
 // api_state.cu
