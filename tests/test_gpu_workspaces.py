@@ -95,3 +95,31 @@ def test_samples_between_dampings():
         assert np.array_equal(sample(), first)
     a.close()
     b.close()
+
+
+GROWING = """
+import ctypes as C, torch, numpy as np
+from logosq_b200 import State
+from logosq_b200._lib import call
+def free():
+    return torch.cuda.mem_get_info()[0] >> 20
+st = State.plus_state(23)
+call("lq_state_synchronize", st.handle)
+before = free()
+low = []
+for k in range(40):
+    out = np.empty(100 + 3000 * k, np.uint64)
+    call("lq_measure_shots", st.handle, len(out), k, out.ctypes.data_as(C.POINTER(C.c_uint64)))
+    low.append(before - free())
+print(max(low), low[-1] - low[-2], low[-1])
+"""
+
+
+def test_workspaces_of_growing_sizes():
+    """Samples of 23 qubits want 64 MiB and a little more each time: they share a buffer, and
+    a call that finds only smaller ones takes their place."""
+    out = subprocess.run([sys.executable, "-c", GROWING], capture_output=True, text=True,
+                         check=True)
+    most, last, kept = map(int, out.stdout.split())
+    assert most <= 256 + 64
+    assert last == 0 and kept > 0  # nothing allocated for the last call alone
