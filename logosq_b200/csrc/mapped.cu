@@ -571,14 +571,14 @@ static bool unit(const cd &z) { return std::abs(length(z) - 1) <= 1e-12; }
 // that it became.  (Planned op by op, a 2x2 with a quarter turn counted twice, and 60
 // single-qubit gates on 24 qubits took five passes instead of three: 480 us, now 326.)
 struct MapUnit {
-    PlanGate shape;
     const GateOp *swap;  // the gate if it is a SWAP
     int begin, end;
 };
 
-// The circuit as map ops; runs of single-qubit gates on a bit become one 2x2 first.
-static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
-                      std::vector<MapUnit> &units) {
+// The circuit as map ops, and its passes; runs of single-qubit gates on a bit become one 2x2
+// first.
+static bool map_lower(const std::vector<GateOp> &gops, int n, int T, std::vector<MapOp> &out,
+                      std::vector<MapUnit> &units, std::vector<PlanStep> &steps) {
     struct Run {
         int bit;
         cd u[4];
@@ -619,17 +619,34 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
         for (uint64_t bits = op_bits(g); bits; bits &= bits - 1) open[__builtin_ctzll(bits)] = -1;
         list.push_back(Entry{-1, &g});
     }
+    units.reserve(list.size());
+    std::vector<PlanGate> shapes;
+    shapes.reserve(list.size());
+    for (const Entry &en : list) {
+        PlanGate p;
+        if (en.run >= 0) {
+            p.bits = bit_of(runs[en.run].bit);
+            p.mixed = runs[en.run].diag ? 0 : p.bits;
+        } else {
+            p = plan_gate(*en.g);
+        }
+        shapes.push_back(p);
+        units.push_back(MapUnit{en.run < 0 && en.g->type == OP_SWAP ? en.g : nullptr, 0, 0});
+    }
+    steps = plan_windows(shapes, n, T);
+    // (a two-qubit rotation across windows would be three passes here, 983 us on 26 qubits
+    // where its own sweep takes 317; seen before the gates are taken apart, which costs more
+    // than the windows)
+    for (const PlanStep &st : steps)
+        if (!st.fused && !units[st.gate].swap) return false;
     Recent<MapEuler> recent;
     out.reserve(3 * list.size());
-    units.reserve(list.size());
-    for (const Entry &en : list) {
-        if (!units.empty()) units.back().end = (int)out.size();
-        units.push_back(MapUnit{PlanGate{}, nullptr, (int)out.size(), 0});
-        PlanGate &shape = units.back().shape;
+    for (size_t k = 0; k < list.size(); ++k) {
+        const Entry &en = list[k];
+        if (k > 0) units[k - 1].end = (int)out.size();
+        units[k].begin = (int)out.size();
         if (en.run >= 0) {
             const Run &r = runs[en.run];
-            shape.bits = bit_of(r.bit);
-            shape.mixed = r.diag ? 0 : shape.bits;
             if (r.x) {
                 out.push_back(map_perm_x(r.bit, -1));
             } else if (r.diag) {
@@ -641,7 +658,6 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
             continue;
         }
         const GateOp &g = *en.g;
-        shape = plan_gate(g);
         switch (g.type) {
         case OP_PERM1:
             if (g.nctrl != 1) return false;
@@ -654,7 +670,6 @@ static bool map_lower(const std::vector<GateOp> &gops, std::vector<MapOp> &out,
             o.b1 = g.b1;
             o.bits = bit_of(g.b0) | bit_of(g.b1);
             out.push_back(o);
-            units.back().swap = &g;
             break;
         }
         case OP_DIAG: {
@@ -1470,15 +1485,8 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
     if (n < 20 && 3 * (controlled + blocks) > 2 * gops.size()) return false;
     std::vector<MapOp> ops;
     std::vector<MapUnit> units;
-    if (!map_lower(gops, ops, units)) return false;
-    std::vector<PlanGate> shapes;
-    shapes.reserve(units.size());
-    for (const MapUnit &u : units) shapes.push_back(u.shape);
-    const std::vector<PlanStep> steps = plan_windows(shapes, n, T);
-    // (a two-qubit rotation across windows would be three passes here, 983 us on 26 qubits
-    // where its own sweep takes 317)
-    for (const PlanStep &st : steps)
-        if (!st.fused && !units[st.gate].swap) return false;
+    std::vector<PlanStep> steps;
+    if (!map_lower(gops, n, T, ops, units, steps)) return false;
     // the last pass takes what still waits (sweeps after it only move amplitudes)
     size_t last = steps.size();
     for (size_t si = 0; si < steps.size(); ++si)
