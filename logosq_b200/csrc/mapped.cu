@@ -1469,20 +1469,25 @@ private:
 // 0.86 ms, 235 gates of 16-qubit brickwork 0.18; with GateOp records in every op, vectors per
 // round and the complex library's operators 2.25 and 0.48, more than the rounds save there.)
 bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
-    // A controlled rotation is a whole rotation and a table here, and one record there
-    // (40 of CRX and CRY on 26, 18 and 8 qubits: 4.55, 0.091 and 0.061 ms against 3.76, 0.073
-    // and 0.034; a third of them among single-qubit gates 2.62 against 2.15 on 26): more than
-    // a fifth of them go there.  RXX and RYY are two such rotations in one, and better here
-    // except in small states without much besides (40 on 26, 18 and 11 qubits: 3.9, 0.050 and
-    // 0.059 ms against 4.3, 0.058 and 0.044; three Trotter steps, half of whose gates are
-    // diagonal: 12.1, 0.144 and 0.069 against 19.4, 0.193 and 0.095).
+    // A controlled rotation is a whole rotation and a table here, and one record there; RXX and
+    // RYY are two such rotations in one.  Whether the rest of the circuit makes up for them
+    // depends on the size (times of 60 to 200 gates submitted again, here against there).
+    // Up to 10 qubits, a few dozen threads, next to none: controlled rotations a tenth of the
+    // gates 85 us against 68, four Trotter steps, half of whose gates are RXX and RYY, 150
+    // against 118 on 6 qubits and 228 against 231 on 10.  Up to 19 qubits a sixth of controlled
+    // rotations (15 %, 16 qubits: 119 against 140; 20 % with new angles 325 against 293) and
+    // half of RXX and RYY (Trotter steps of 11 to 19 qubits: 203 against 280, 340 against 395,
+    // 481 against 638; 60 % with new angles 556 against 392).  Above, a fifth and any number (26
+    // qubits: 40 CRX and CRY alone 4.55 ms against 3.76; 40 RXX and RYY alone 3.9 against 4.3).
     size_t controlled = 0, blocks = 0;
     for (const GateOp &g : gops) {
         controlled += g.type == OP_M1 && g.nctrl > 0;
         blocks += g.type == OP_M2;
     }
-    if (5 * controlled > gops.size()) return false;
-    if (n < 20 && 3 * (controlled + blocks) > 2 * gops.size()) return false;
+    if (n <= 10 ? 12 * (controlled + blocks) > gops.size()
+                : n < 20 ? 6 * controlled > gops.size() || 2 * (controlled + blocks) > gops.size()
+                         : 5 * controlled > gops.size())
+        return false;
     std::vector<MapOp> ops;
     std::vector<MapUnit> units;
     std::vector<PlanStep> steps;
