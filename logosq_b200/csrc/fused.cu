@@ -1321,6 +1321,13 @@ static int launch_cached(lq_state *s, const PlanCache &pc) {
     return LQ_OK;
 }
 
+static int is_capturing(lq_state *s, bool *out) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    LQ_CUDA_TRY(cudaStreamIsCapturing(s->stream, &cs));
+    *out = cs != cudaStreamCaptureStatusNone;
+    return LQ_OK;
+}
+
 int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *theta,
                        int ntheta, int mode) {
     const int n = s->n;
@@ -1330,10 +1337,15 @@ int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *
     const bool can_fuse = mode == LQ_EXEC_FUSED && s->dtype == LQ_C128 && n >= 5;
     const PlanKeyView key{{n, std::min(fusion_width(), n), nops, ntheta, real_fold_mode()},
                           ops, theta};
+    const PlanCache *known = nullptr;  // the records in the handle's buffer, for a capture
     if (can_fuse) {
         const PlanCache *pc = static_cast<const PlanCache *>(s->plan_cache);
-        if (pc && (pc->mapped || s->prog_valid) && key.equals(pc->key))
-            return launch_cached(s, *pc);
+        if (pc && (pc->mapped || s->prog_valid) && key.equals(pc->key)) {
+            bool captured = false;
+            if (!pc->mapped) LQ_TRY(is_capturing(s, &captured));
+            if (!captured) return launch_cached(s, *pc);
+            known = pc;
+        }
     }
     std::vector<GateOp> gops(nops);
     for (int i = 0; i < nops; ++i) LQ_TRY(make_gate_op(&ops[i], theta, n, &gops[i]));
@@ -1350,8 +1362,21 @@ int apply_circuit_impl(lq_state *s, const lq_gate *ops, int nops, const double *
     pc->T = T;
     pc->normalize = defer_renorm(gops);
     // Mapped rounds where every gate has that form (mapped.cu), else op records.
+    // A capturing stream takes the mapped rounds wherever there are any: their program is
+    // part of the launch, that of the records lies in the handle's buffer, which cannot be
+    // filled then and which the handle's next circuit overwrites.
     MapProgram mp;
-    if (map_plan(gops, n, T, mp)) {
+    bool mapped = map_plan(gops, n, T, mp);
+    if (!mapped) {
+        bool captured;
+        LQ_TRY(is_capturing(s, &captured));
+        if (captured) {
+            mp = MapProgram{};
+            mapped = map_plan(gops, n, T, mp, true);
+        }
+    }
+    if (!mapped && known) return launch_cached(s, *known);
+    if (mapped) {
         pc->mapped = true;
         pc->map = std::move(mp);
         free_plan_cache(s);

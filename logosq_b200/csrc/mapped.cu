@@ -1468,7 +1468,7 @@ private:
 // (Its host time is in every call with new angles: ten Trotter steps of 19 qubits, 730 gates,
 // 0.86 ms, 235 gates of 16-qubit brickwork 0.18; with GateOp records in every op, vectors per
 // round and the complex library's operators 2.25 and 0.48, more than the rounds save there.)
-bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
+bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out, bool always) {
     // A controlled rotation is a whole rotation and a table here, and one record there; RXX and
     // RYY are two such rotations in one.  Whether the rest of the circuit makes up for them
     // depends on the size (times of 60 to 200 gates submitted again, here against there).
@@ -1484,9 +1484,10 @@ bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out) {
         controlled += g.type == OP_M1 && g.nctrl > 0;
         blocks += g.type == OP_M2;
     }
-    if (n <= 10 ? 12 * (controlled + blocks) > gops.size()
-                : n < 20 ? 6 * controlled > gops.size() || 2 * (controlled + blocks) > gops.size()
-                         : 5 * controlled > gops.size())
+    if (!always &&
+        (n <= 10  ? 12 * (controlled + blocks) > gops.size()
+         : n < 20 ? 6 * controlled > gops.size() || 2 * (controlled + blocks) > gops.size()
+                  : 5 * controlled > gops.size()))
         return false;
     std::vector<MapOp> ops;
     std::vector<MapUnit> units;

@@ -29,8 +29,9 @@ struct MapProgram {
 };
 
 // Plan gops (canonical ops in order, none renormalising) for n qubits and tile bits
-// T.  False when some gate has no mapped form; host work only.
-bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out);
+// T.  False when some gate has no mapped form or, unless `always`, the op records are the
+// faster engine for such a circuit; host work only.
+bool map_plan(const std::vector<GateOp> &gops, int n, int T, MapProgram &out, bool always = false);
 // Launch one pass of the program (its blob stays on the host).
 int map_launch(lq_state *s, int T, const MapLaunch &pass, const unsigned char *blob);
 
