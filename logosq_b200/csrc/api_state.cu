@@ -1048,14 +1048,15 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
     // group of few terms, or two of complex64, is sweeps instead where the state is large
     // enough for that to count more than the launches (20 qubits, two windows of a group
     // each: 38 us, two sweeps 46), and a sum of terms without X alone is one folded sweep, as
-    // far as that goes (n >= 12).  A sum of a single group is a sweep unless its many terms on
-    // a large state count more than the window's longer start: 8 qubits 25-29 us for 20 terms
-    // and 60 for 1000 (a window 35-38 and 71-96), 20 qubits 40 us for 20 terms (44), but 67 for
-    // 100 (52-60), 24 qubits 153 for 20 (130).
+    // far as that goes (n >= 12).  A single group that fits a window (alone, or beside others
+    // that fit none) is a sweep unless its many terms on a large state count more than the
+    // window's longer start: 8 qubits 25-29 us for 20 terms and 60 for 1000 (a window 35-38
+    // and 71-96), 20 qubits 40 us for 20 terms (44), but 67 for 100 (52-60), 24 qubits 153 for
+    // 20 (130); 18 qubits, ten random terms of which one fits 94 us (106).
     constexpr int kSweepQubits = 22;
     constexpr size_t kSweepTerms = 4;
+    const bool only = needs.size() + anywhere.size() == 1;
     auto few = [&](const std::vector<size_t> &gs) {
-        const bool only = groups.size() == 1;
         const size_t most = !only ? kSweepTerms
                             : n < 19 ? (size_t)kMaxGroupTerms
                                      : std::max<size_t>(kSweepTerms, 64 >> std::min(n - 19, 6));

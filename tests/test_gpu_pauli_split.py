@@ -57,6 +57,16 @@ def test_one_mask(n, count, x):
     check(n, [(float(r.normal()), x, int(r.integers(0, 1 << n))) for _ in range(count)])
 
 
+@pytest.mark.parametrize("x", [0, 3, 1 << 6])
+@pytest.mark.parametrize("n,count", [(13, 1), (13, 300), (18, 40), (19, 64), (19, 65)])
+def test_one_mask_that_fits_beside_masks_that_do_not(n, count, x):
+    r = np.random.default_rng(n + count)
+    wide = [(float(r.normal()), 1 << 4 | 1 << (n - 1) | k, int(r.integers(0, 1 << n)))
+            for k in range(3)]
+    check(n, wide[:2] + [(float(r.normal()), x, int(r.integers(0, 1 << n)))
+                         for _ in range(count)] + wide[2:])
+
+
 @pytest.mark.parametrize("n", [13, 14])
 def test_masks_of_a_window_are_not_slower_than_masks_that_fit_none(n):
     """16 masks of 400 terms: 0.26 ms in a window's rounds (1.0 ms with a round's terms in one
