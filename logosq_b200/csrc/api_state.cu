@@ -1163,9 +1163,11 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
             size_t nterms;
         };
         std::vector<RoundTerms> prog;
+        prog.reserve(rounds.size());
         size_t all_terms = 0;
         for (const Round &r : rounds) {
             RoundTerms rt{};
+            rt.entries.reserve(r.groups.size());
             uint32_t pivots = 0;
             for (int k = 0; k < 4; ++k) {
                 rt.hd.vec[k] = win_place(r.vec[k]);
@@ -1240,21 +1242,23 @@ int expectation_impl(const lq_state *s, const lq_pauli_term *terms, int nterms, 
                     b = e;
                 }
         }
-        // the largest first, each to the part with the fewest terms so far
         const size_t parts = std::min(jobs.size(), share);
-        std::stable_sort(jobs.begin(), jobs.end(),
-                         [](const Job &x, const Job &y) { return x.nterms > y.nterms; });
-        using Load = std::pair<size_t, size_t>;  // terms, part
-        std::priority_queue<Load, std::vector<Load>, std::greater<Load>> loads;
-        for (size_t k = 0; k < parts; ++k) loads.push({0, k});
-        for (Job &j : jobs) {
-            const Load l = loads.top();
-            loads.pop();
-            j.part = l.second;
-            loads.push({l.first + j.nterms + 1, l.second});
+        if (parts > 1) {
+            // the largest first, each to the part with the fewest terms so far
+            std::stable_sort(jobs.begin(), jobs.end(),
+                             [](const Job &x, const Job &y) { return x.nterms > y.nterms; });
+            using Load = std::pair<size_t, size_t>;  // terms, part
+            std::priority_queue<Load, std::vector<Load>, std::greater<Load>> loads;
+            for (size_t k = 0; k < parts; ++k) loads.push({0, k});
+            for (Job &j : jobs) {
+                const Load l = loads.top();
+                loads.pop();
+                j.part = l.second;
+                loads.push({l.first + j.nterms + 1, l.second});
+            }
+            std::stable_sort(jobs.begin(), jobs.end(),
+                             [](const Job &x, const Job &y) { return x.part < y.part; });
         }
-        std::stable_sort(jobs.begin(), jobs.end(),
-                         [](const Job &x, const Job &y) { return x.part < y.part; });
         std::vector<WinRound> cr;
         std::vector<WinGroup> cg;
         std::vector<WinTerm> ct;
